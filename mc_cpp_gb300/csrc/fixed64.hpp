@@ -1,0 +1,39 @@
+// Pair terms of the FP64 path in 64-bit integer arithmetic: the constants a box needs, and the host
+// code that forms them.  The device side is fixed64.cuh.
+#pragma once
+#include <cstdint>
+
+#include "dev_types.hpp"
+
+namespace mcg {
+
+// Constants of one box.  Lengths are in units of the effective box Leff: max(L) / 2^sh, where the
+// wrapped 64-bit displacement of a pair within reach, shifted left by sh, still fits 63 bits; or
+// 2 max(L) with displacements halved, for pairs at any distance.
+struct Fix64Geom {
+    int sh;                  // left shift of the stored positions, hence of every displacement
+    int iso;                 // equal box lengths and displacements not halved
+    int up;                  // displacement = high half of (difference x ratio) << up: 2, or 1 when halved
+    int64_t ratio[3];        // L[k] / max(L) in units of 2^-62
+    uint64_t c2;             // (rc / Leff)^2 in units of 2^-64
+    int sD;                  // (c2 - u) << sD fits 64 bits for every u above ron^2 (1 - 2^-8)
+    uint64_t rD;             // 2^126 / ((rc^2 - ron^2) / Leff^2 << sD): v = (rc^2 - u) / (rc^2 - ron^2)
+    float Ls[3], Ll[3];      // L / 2^32 as float-float: FP32 displacement from the high words
+    float in2, out2;         // FP32 r^2 below in2 lies inside ron, above out2 beyond rc (A^2)
+    double leff;
+};
+
+// Geometry of the pairs within rc (1 + 1e-4), switched from ron (may be 0), in a box at least 2 rc wide:
+// shifted when it is at least twice the reach wide, halved otherwise.
+Fix64Geom fix64_geom(const double L[3], double rc, double ron);
+// Geometry of any pair of a box, without a cutoff: halved (iso: equal box lengths).
+Fix64Geom fix64_geom_full(const double L[3]);
+
+// One pair of parameter classes: el += qq / r, vd += (c12 / r^6 - c6) / r^6 with lengths in Leff
+// (qq = qi qj / Leff, c6 = ei ej (si + sj)^6 / Leff^6, c12 = c6 (si + sj)^6 / Leff^6).
+struct alignas(32) Fix64Pair {
+    double qq, c6, c12, pad;
+};
+Fix64Pair fix64_pair(double qi, double ei, double si, double qj, double ej, double sj, double leff);
+
+}  // namespace mcg

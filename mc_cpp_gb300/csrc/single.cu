@@ -6,6 +6,8 @@
 //   es14[n]      double2 (eps14, sig14)
 //   fx[n]        uint4 (fx, fy, fz, parameter class)  fixed-point mirror for the mixed kernels
 //   cls_of[n], cls[ncls]  parameter class of each atom and the classes' (q hi, q lo, eps, sig)
+//   x64[n]       ulonglong4 (x, y, z as box fractions in 2^-64, class), FP64 switched periodic systems
+//   pair64[ncls^2]   the class pairs' parameter products (fixed64.hpp)
 //   esf[n]       float2 (eps, sig)
 //   nbr[n*cap]   int   Verlet rows: partners j > i from the front, j < i from the back
 //   nup[n], nlo[n]
@@ -16,7 +18,9 @@
 // Kernels (all launched on the handle's stream):
 //   k_cell_assign / k_cell_scan / k_cell_scatter / k_cell_sort / k_build_rows   Verlet build
 //   k_energy_list<P>   switch energy over the half list (warp per row)        FField_MDBAS.cpp:336-424
+//   k_energy_list64    the same in FP64 for periodic boxes, on 64-bit integer pair terms
 //   k_energy_all<P>    full energy over all pairs (triangular tile grid)      FField_MDBAS.cpp:194-265
+//   k_energy_all64     the same in FP64 for periodic boxes, on 64-bit integer pair terms
 //   k_energy_14<P>     1-4 pairs                                               FField_MDBAS.cpp:267-318,426-488
 //   k_bonded           bonds, Urey-Bradley, angles, dihedrals, impropers       FField_MDBAS.cpp:490-786
 //   k_finalize         fixed-order reduction of the partials into ener[10]
@@ -34,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.hpp"
+#include "fixed64.cuh"
 #include "pair_math.cuh"
 #include "single.hpp"
 
@@ -50,6 +55,9 @@ constexpr int NB_THREADS = 256;
 constexpr int MAX_MOVED = 1024;
 constexpr int SORT_MAX = 2048;       // cells larger than this are sorted by one thread
 constexpr int CLS_MAX = 1024;        // parameter classes the mixed pair kernel keeps in shared memory
+// parameter classes whose pairs the FP64 kernel's table holds: 512 KB of products at 128, which stay in
+// L2 with a few rows of the matrix in L1; a system of more classes forms them per pair (9 FP64 operations)
+constexpr int CLS64_MAX = 128;
 
 enum { PREC_F64 = 0, PREC_MIX = 1 };
 
@@ -336,6 +344,9 @@ struct AtomsDev {
     const float2* esf14;
     const float2* qf;     // charge as float-float (hi, lo)
     float Ls[3], Lsl[3];  // box / 2^32 as float-float (mixed displacement scale)
+    ulonglong4_32a* x64;  // 64-bit box fractions and parameter class (null: no 64-bit mirror)
+    const Fix64Pair* pair64;   // products of the class pairs (null: formed per pair)
+    int ncls64;
 };
 
 template <int P>
@@ -399,6 +410,125 @@ __global__ void __launch_bounds__(NB_THREADS) k_energy_list(AtomsDev A, int n, P
             else { fe.add((float)el); fv.add((float)vd); }
         }
         if (P == PREC_MIX) { sel += fe.value(); svd += fv.value(); }
+    }
+    block_reduce2(sel, svd, part + 2 * blockIdx.x);
+}
+
+// The pair's parameter products with lengths in Leff: from the table of class pairs, or formed here
+// for a system of more than CLS64_MAX distinct parameter sets.
+template <bool TABLE>
+__device__ __forceinline__ void pair64_params(const AtomsDev& A, double ileff, int i, int j, int ci, int cj, double& qq,
+                                              double& c6, double& c12) {
+    if (TABLE) {
+        const double4_32a p = reinterpret_cast<const double4_32a*>(A.pair64)[ci * A.ncls64 + cj];
+        qq = p.x; c6 = p.y; c12 = p.z;
+    } else {
+        const double2 a = A.es[i], b = A.es[j];
+        const double s = (a.y + b.y) * ileff, s2 = s * s, s6 = s2 * s2 * s2;
+        qq = A.pq[i].w * A.pq[j].w * ileff;
+        c6 = a.x * b.x * s6;
+        c12 = c6 * s6;
+    }
+}
+
+// FP64 switch energy over the half list for periodic boxes.  Bound by the integer and FP64 pipes
+// (64-76 cycles of a scheduler per FP64 warp instruction, about 22 per 64-bit product), so:
+//  - a warp per row places its entries by the FP32 distance of the fixed-point mirrors: beyond
+//    rc (37% of a 14 A list at 12 A) they are dropped, the others go, with their row's atom, to one
+//    of two rings in shared memory, inside ron (no switch factor) or not;
+//  - a ring with 32 pairs is evaluated by all lanes at once, so no lane is idle at a row's end or at
+//    the cutoff, and the switch is formed only for the pairs that need it;
+//  - a pair's distance and powers are 64-bit integers (fixed64.cuh), with 3 FP64 operations.
+// The FP32 placement has a margin of 1e-4 in r^2; a pair placed within rc that lies beyond takes a
+// switch factor of exactly 0, and one placed outside ron a factor of 1 to 2^-58.
+// The rings are drained at one place in the code, after a chunk of E64_U entries per lane: with the
+// evaluation inlined behind every entry the kernel stalled on instruction fetch (0.69 against 0.61 ms on
+// the 100,002-atom water box).  That box takes 0.53 ms, 69 G pairs/s (4.2 ms with the pair terms in
+// FP64); ncu at 12,288 atoms: FP64 pipe 45%, ALU 45%, the rest latency of the gathers.  Three entries
+// per lane in flight against two: 0.527 and 0.532 ms; five or six CTAs per SM instead of four: 0.520 and
+// 0.513 ms there, but 0.073 against 0.070 ms at 12,288 atoms.
+constexpr int E64_U = 3;
+constexpr int E64_RING = 128;   // up to 31 pending pairs and 32 E64_U new ones
+
+template <bool ISO, bool TABLE>
+__global__ void __launch_bounds__(NB_THREADS) k_energy_list64(AtomsDev A, Fix64Geom G, PbcDev pbc, CutDev cut, int n,
+                                                              const int* __restrict__ nbr, const int* __restrict__ nup,
+                                                              int cap, double* part) {
+    __shared__ int2 s_ring[NB_THREADS / 32][2][E64_RING];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const double ileff = 1.0 / G.leff;
+    int2* ring = s_ring[wib][0];              // inside ron, then the switched pairs at + E64_RING
+    double sel = 0.0, svd = 0.0;
+    int head0 = 0, tail0 = 0, head1 = 0, tail1 = 0;   // ring positions, warp-uniform
+    int i = warp, k0 = 0, m = i < n ? nup[i] : 0;
+    uint4 fi = i < n ? A.fx[i] : make_uint4(0, 0, 0, 0);
+    for (;;) {
+        const bool last = i >= n;
+        if (!last) {
+            const int* row = nbr + (size_t)i * cap;
+            int j[E64_U];
+            float r2[E64_U];
+#pragma unroll
+            for (int u = 0; u < E64_U; u++) {
+                const int k = k0 + u * 32 + lane;
+                j[u] = k < m ? row[k] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < E64_U; u++) {
+                const uint4 fj = j[u] >= 0 ? A.fx[j[u]] : fi;
+                const float dx = fixed_delta(fi.x, fj.x, G.Ls[0], G.Ll[0]), dy = fixed_delta(fi.y, fj.y, G.Ls[1], G.Ll[1]),
+                            dz = fixed_delta(fi.z, fj.z, G.Ls[2], G.Ll[2]);
+                r2[u] = j[u] >= 0 ? fmaf(dx, dx, fmaf(dy, dy, dz * dz)) : 3.0e38f;
+            }
+#pragma unroll
+            for (int u = 0; u < E64_U; u++) {
+                const bool in = r2[u] < G.in2, sw = !in && r2[u] <= G.out2;
+                const unsigned bi = __ballot_sync(0xffffffffu, in), bs = __ballot_sync(0xffffffffu, sw);
+                if (in) ring[(head0 + __popc(bi & below)) & (E64_RING - 1)] = make_int2(i, j[u]);
+                if (sw) ring[E64_RING + ((head1 + __popc(bs & below)) & (E64_RING - 1))] = make_int2(i, j[u]);
+                head0 += __popc(bi);
+                head1 += __popc(bs);
+            }
+            k0 += 32 * E64_U;
+            if (k0 >= m) {
+                i += nwarps;
+                k0 = 0;
+                if (i < n) { m = nup[i]; fi = A.fx[i]; }
+            }
+            __syncwarp();
+        }
+        // full rings, and what is left of them after the last row
+        const int least = last ? 1 : 32;
+        for (;;) {
+            const bool sw = head0 - tail0 < least;
+            if (sw && head1 - tail1 < least) break;
+            const int at = sw ? E64_RING + ((tail1 + lane) & (E64_RING - 1)) : (tail0 + lane) & (E64_RING - 1);
+            if (lane < (sw ? head1 - tail1 : head0 - tail0)) {
+                const int2 p = ring[at];
+                const ulonglong4_32a a = A.x64[p.x], b = A.x64[p.y];
+                const Fix64Dist u = fix64_dist2<ISO>(G, a, b);
+                double ys, w, ws;
+                if (fix64_terms(G, u, sw, ys, w, ws)) {
+                    double qq, c6, c12;
+                    pair64_params<TABLE>(A, ileff, p.x, p.y, (int)a.w, (int)b.w, qq, c6, c12);
+                    sel = fma(qq, ys, sel);
+                    svd = fma(fma(c12, w, -c6), ws, svd);
+                } else {
+                    double el, vd;
+                    const uint4 f0 = make_uint4(0, 0, 0, 0);
+                    pair_energy<PREC_F64>(A, pbc, cut, false, A.pq[p.x], f0, p.x, A.pq[p.y], f0, p.y, true, el, vd);
+                    sel += el;
+                    svd += vd;
+                }
+            }
+            if (sw) tail1 = min(tail1 + 32, head1);
+            else tail0 = min(tail0 + 32, head0);
+        }
+        if (last) break;
+        __syncwarp();
     }
     block_reduce2(sel, svd, part + 2 * blockIdx.x);
 }
@@ -611,6 +741,69 @@ __global__ void __launch_bounds__(TILE) k_energy_all(AtomsDev A, int n, PbcDev p
             else { fe.add((float)el); fv.add((float)vd); }
         }
         if (P == PREC_MIX) { sel = fe.value(); svd = fv.value(); }
+    }
+    block_reduce2(sel, svd, part + 2 * blockIdx.x);
+}
+
+// FP64 full energy for periodic boxes, on 64-bit integer pair terms (fixed64.cuh): three FP64
+// operations a pair, about 230 cycles of a scheduler's FP64 pipe per warp, beside some 150 integer
+// and FP32 ones.  A unit of work is A64_I rows (a thread each) against A64_J columns staged in shared
+// memory; units are numbered over the upper triangle row tile by row tile and dealt to the CTAs in
+// turn.  Short columns, because a thread's walk along them is serial: a box of 1,536 atoms has 312
+// units (12 x 13 / 2 = 78 with square tiles, for 152 SMs), and a CTA's partial sum covers all its units.
+// 12,288 atoms (75 M pairs): the whole energy call takes 0.58 ms, 3.78 ms with the pair terms in FP64.
+constexpr int A64_I = 128, A64_J = 32;
+
+template <bool ISO, bool TABLE>
+__global__ void __launch_bounds__(A64_I) k_energy_all64(AtomsDev A, Fix64Geom G, PbcDev pbc, CutDev cut, int n,
+                                                        const int* __restrict__ fxs, const int* __restrict__ fxd,
+                                                        int units, double* part) {
+    __shared__ ulonglong4_32a sx[A64_J];
+    const double ileff = 1.0 / G.leff;
+    const int c0 = (n + A64_J - 1) / A64_J;      // columns chunks of row tile 0; each next tile has A64_I / A64_J fewer
+    constexpr int STEP = A64_I / A64_J;
+    double sel = 0.0, svd = 0.0;
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        // row tile I: the last with I c0 - STEP I (I - 1) / 2 <= unit
+        auto first = [&](int I) { return (long long)I * c0 - (long long)STEP * I * (I - 1) / 2; };
+        const float b = c0 + 0.5f * STEP;
+        int I = (int)((b - sqrtf(fmaxf(b * b - 2.0f * STEP * unit, 0.0f))) / STEP);
+        while (I > 0 && first(I) > unit) I--;
+        while (first(I + 1) <= unit) I++;
+        const int jb = I * A64_I + (int)(unit - first(I)) * A64_J, je = min(n, jb + A64_J);
+        const int i = I * A64_I + threadIdx.x;
+        __syncthreads();
+        if (threadIdx.x < A64_J && jb + threadIdx.x < n) sx[threadIdx.x] = A.x64[jb + threadIdx.x];
+        __syncthreads();
+        if (i >= n) continue;
+        const ulonglong4_32a a = A.x64[i];
+        int cur = fxs[i];
+        const int xe = fxs[i + 1], j0 = max(jb, i + 1);
+        while (cur < xe && fxd[cur] < j0) cur++;
+        int next = cur < xe ? fxd[cur] : n;      // the reference's sorted-row cursor (FField_MDBAS.cpp:227-234)
+        for (int j = jb; j < je; j++) {
+            if (j <= i) continue;
+            if (j == next) {
+                cur++;
+                next = cur < xe ? fxd[cur] : n;
+                continue;
+            }
+            const ulonglong4_32a bj = sx[j - jb];
+            const Fix64Dist u = fix64_dist2<ISO, true>(G, a, bj);
+            double ys, w, ws;
+            if (fix64_terms(G, u, false, ys, w, ws)) {
+                double qq, c6, c12;
+                pair64_params<TABLE>(A, ileff, i, j, (int)a.w, (int)bj.w, qq, c6, c12);
+                sel = fma(qq, ys, sel);
+                svd = fma(fma(c12, w, -c6), ws, svd);
+            } else {
+                double el, vd;
+                const uint4 f0 = make_uint4(0, 0, 0, 0);
+                pair_energy<PREC_F64>(A, pbc, cut, false, A.pq[i], f0, i, A.pq[j], f0, j, false, el, vd);
+                sel += el;
+                svd += vd;
+            }
+        }
     }
     block_reduce2(sel, svd, part + 2 * blockIdx.x);
 }
@@ -981,25 +1174,29 @@ __global__ void __launch_bounds__(256) k_delta_e(AtomsDev A, int n, PbcDev pbc, 
     }
 }
 
-template <int P>
-__global__ void k_commit(int m, const int* idx, const double* xyz, double4_32a* pq, uint4* fx, PbcDev pbc,
-                         const __grid_constant__ MoveInline inl) {
+__device__ __forceinline__ void store_x64(ulonglong4_32a* x64, const double4_32a& p, const PbcDev& pbc, int sh, unsigned cls) {
+    *x64 = make_ulonglong4_32a(to_fixed64(p.x, pbc.L[0], pbc.rL[0], sh), to_fixed64(p.y, pbc.L[1], pbc.rL[1], sh),
+                               to_fixed64(p.z, pbc.L[2], pbc.rL[2], sh), cls);
+}
+
+// A thread per coordinate: a coordinate's mirrors are some 25 dependent FP64 operations, at 64 cycles each.
+__global__ void k_commit(int m, const int* idx, const double* xyz, double4_32a* pq, uint4* fx, ulonglong4_32a* x64,
+                         int sh, PbcDev pbc, const __grid_constant__ MoveInline inl) {
     if (inl.m > 0) { idx = inl.idx; xyz = inl.xyz; }
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, k = t / 3, c = t - 3 * k;
     if (k >= m) return;
-    int a = idx[k];
-    double4_32a p = pq[a];
-    p.x = xyz[3 * k]; p.y = xyz[3 * k + 1]; p.z = xyz[3 * k + 2];
-    pq[a] = p;
+    const int a = idx[k];
+    const double v = xyz[t];
+    reinterpret_cast<double*>(pq + a)[c] = v;
     if (pbc.type != 0) {
-        uint4 f = fx[a];
-        f.x = to_fixed(p.x, pbc.rL[0]); f.y = to_fixed(p.y, pbc.rL[1]); f.z = to_fixed(p.z, pbc.rL[2]);
-        fx[a] = f;
+        reinterpret_cast<uint32_t*>(fx + a)[c] = to_fixed(v, pbc.rL[c]);
+        if (x64) reinterpret_cast<unsigned long long*>(x64 + a)[c] = to_fixed64(v, pbc.L[c], pbc.rL[c], sh);
     }
 }
 
-// Fixed-point mirror of every atom from the FP64 masters; w carries the atom's parameter class.
-__global__ void k_fix_all(int n, const double4_32a* __restrict__ pq, const int* __restrict__ cls_of, uint4* fx, PbcDev pbc) {
+// Fixed-point mirrors of every atom from the FP64 masters; w carries the atom's parameter class.
+__global__ void k_fix_all(int n, const double4_32a* __restrict__ pq, const int* __restrict__ cls_of, uint4* fx,
+                          ulonglong4_32a* x64, int sh, PbcDev pbc) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double4_32a p = pq[i];
@@ -1008,6 +1205,7 @@ __global__ void k_fix_all(int n, const double4_32a* __restrict__ pq, const int* 
     else { f.x = f.y = f.z = 0; }
     f.w = (unsigned)cls_of[i];
     fx[i] = f;
+    if (x64) store_x64(x64 + i, p, pbc, sh, f.w);
 }
 
 // ==========================================================================================
@@ -1035,7 +1233,7 @@ void SingleEngine::release() {
     void* ptrs[] = {d_pq, d_es, d_es14, d_fx, d_esf, d_esf14, d_qf, d_prmf, d_frozen, d_xs, d_xd, d_fxs, d_fxd, d_p14, d_c14s,
                     d_c14d, d_bonds, d_ubs, d_angles, d_dihes, d_imprs, d_nbr, d_nup, d_nlo, d_cell_of,
                     d_cell_count, d_cell_start, d_cell_fill, d_cell_atoms, d_part, d_ticket, d_maxrow,
-                    d_stage, d_prn, d_pnup, d_pkept, d_cls_of, d_cls};
+                    d_stage, d_prn, d_pnup, d_pkept, d_cls_of, d_cls, d_x64, d_pair64};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (cudaEvent_t& e : ev_prune) if (e) { cudaEventDestroy(e); e = nullptr; }
     if (h_stage) cudaFreeHost(h_stage);
@@ -1074,10 +1272,31 @@ int SingleEngine::init(const HostSystem& h) {
         prmf[i] = make_float4(qf[i].x, qf[i].y, esf[i].x, esf[i].y);
     }
     // parameter classes: the distinct (q hi, q lo, eps, sig) of the mixed pair kernel, in first-seen
-    // order; more than CLS_MAX classes leave the table empty (the kernel gathers per atom)
+    // order; more than CLS_MAX (CLS64_MAX) classes leave the table empty (the kernel gathers per atom)
     std::vector<int> cls_of(n, 0);
     std::vector<float4> cls;
-    {
+    std::vector<Fix64Pair> pair64;
+    if (uses_fix64()) {   // FP64: the distinct (q, eps, sig) and the products of every pair of them
+        fix64 = hs.cut == MCG_CUT_SWITCH ? fix64_geom(hs.L, hs.rc, hs.ron) : fix64_geom_full(hs.L);
+        std::map<std::array<double, 3>, int> seen;
+        std::vector<std::array<double, 3>> par;
+        for (int i = 0; i < n && (int)par.size() <= CLS64_MAX; i++) {
+            const std::array<double, 3> key{hs.q[i], hs.eps[i], hs.sig[i]};
+            auto it = seen.find(key);
+            if (it == seen.end()) {
+                it = seen.emplace(key, (int)par.size()).first;
+                par.push_back(key);
+            }
+            cls_of[i] = it->second;
+        }
+        if ((int)par.size() <= CLS64_MAX) {
+            ncls64 = (int)par.size();
+            for (const auto& a : par)
+                for (const auto& b : par) pair64.push_back(fix64_pair(a[0], a[1], a[2], b[0], b[1], b[2], fix64.leff));
+        } else {
+            std::fill(cls_of.begin(), cls_of.end(), 0);
+        }
+    } else {
         std::map<std::array<uint32_t, 4>, int> seen;
         for (int i = 0; i < n && (int)cls.size() <= CLS_MAX; i++) {
             std::array<uint32_t, 4> key;
@@ -1105,6 +1324,7 @@ int SingleEngine::init(const HostSystem& h) {
         (rc = dupload(&d_fxd, hs.fexclData, stream)))
         return rc;
     if ((rc = dalloc(&d_fx, n))) return rc;
+    if (uses_fix64() && ((rc = dalloc(&d_x64, n)) || (ncls64 > 0 && (rc = dupload(&d_pair64, pair64, stream))))) return rc;
     if (uses_pair_variants() && ncls > 0) {   // groups of the group-pair kernels (residue runs of <= 4 atoms)
         if ((rc = grp.setup(hs.resid))) return rc;
         grp_setup = true;
@@ -1154,7 +1374,7 @@ int SingleEngine::init(const HostSystem& h) {
     CK(cudaHostAlloc((void**)&h_map, 32 * sizeof(double), cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer((void**)&d_map, h_map, 0));
     if ((rc = dalloc((char**)&d_stage, stage_bytes))) return rc;
-    k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, pbc);
+    k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
     CK(cudaGetLastError());
     host_x = hs.x; host_y = hs.y; host_z = hs.z;
     if (hs.cut == MCG_CUT_SWITCH) {
@@ -1168,6 +1388,17 @@ int SingleEngine::init(const HostSystem& h) {
 // periodic boxes).
 int SingleEngine::launch_nonbonded(double* nbp) {
     AtomsDev A = atoms();
+    if (uses_fix64()) {
+        const int blocks = std::min(NB_BLOCKS, (n + NB_THREADS / 32 - 1) / (NB_THREADS / 32));
+#define MCG_LIST64(ISO_, TAB_)                                                                                        \
+    k_energy_list64<ISO_, TAB_><<<blocks, NB_THREADS, 0, stream>>>(A, fix64, pbc, cut, n, d_nbr, d_nup, cap, nbp)
+        if (fix64.iso && ncls64) MCG_LIST64(true, true);
+        else if (fix64.iso) MCG_LIST64(true, false);
+        else if (ncls64) MCG_LIST64(false, true);
+        else MCG_LIST64(false, false);
+#undef MCG_LIST64
+        return blocks;
+    }
     if (hs.prec == MCG_PREC_FP64)
         k_energy_list<PREC_F64><<<NB_BLOCKS, NB_THREADS, 0, stream>>>(A, n, pbc, cut, d_nbr, d_nup, cap, nbp);
     else if (pbc.type != 0)
@@ -1530,6 +1761,7 @@ int SingleEngine::time_nonbonded_flushed(int reps, float* ms) {
 
 AtomsDev SingleEngine::atoms() const {
     AtomsDev A;
+    A.x64 = d_x64; A.pair64 = d_pair64; A.ncls64 = ncls64;
     A.pq = d_pq; A.es = d_es; A.es14 = d_es14; A.fx = d_fx; A.esf = d_esf; A.esf14 = d_esf14; A.qf = d_qf;
     for (int k = 0; k < 3; k++) {
         const double ls = hs.L[k] / 4294967296.0;
@@ -1636,7 +1868,18 @@ int SingleEngine::energy(double ener[10]) {
         nnb = launch_nonbonded(nbp);
     } else {
         nnb = ntile * (ntile + 1) / 2;
-        if (hs.prec == MCG_PREC_FP64)
+        if (uses_fix64()) {
+            const long long tiles = (n + A64_I - 1) / A64_I, c0 = (n + A64_J - 1) / A64_J;
+            const int units = (int)(tiles * c0 - (A64_I / A64_J) * tiles * (tiles - 1) / 2);
+            nnb = std::min(units, 152 * 8);
+#define MCG_ALL64(ISO_, TAB_)                                                                                         \
+    k_energy_all64<ISO_, TAB_><<<nnb, A64_I, 0, stream>>>(A, fix64, pbc, cut, n, d_fxs, d_fxd, units, nbp)
+            if (fix64.iso && ncls64) MCG_ALL64(true, true);
+            else if (fix64.iso) MCG_ALL64(true, false);
+            else if (ncls64) MCG_ALL64(false, true);
+            else MCG_ALL64(false, false);
+#undef MCG_ALL64
+        } else if (hs.prec == MCG_PREC_FP64)
             k_energy_all<PREC_F64><<<nnb, TILE, 0, stream>>>(A, n, pbc, cut, d_fxs, d_fxd, ntile, nbp);
         else
             k_energy_all<PREC_MIX><<<nnb, TILE, 0, stream>>>(A, n, pbc, cut, d_fxs, d_fxd, ntile, nbp);
@@ -1675,7 +1918,7 @@ int SingleEngine::set_coords(const double* x, const double* y, const double* z) 
     if (!prune_dirty)
         for (int i = 0; i < n && !prune_dirty; i++) note_moved(i);
     CK(cudaMemcpyAsync(d_pq, pq.data(), sizeof(double4_32a) * n, cudaMemcpyHostToDevice, stream));
-    k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, pbc);
+    k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream));
     return MCG_OK;
@@ -2150,6 +2393,10 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
     ReplayState* d_st = nullptr;
     int rc = MCG_OK;
     auto done = [&](int r) {
+        // the run keeps pq and fx current; the 64-bit mirror, which it does not read, follows here
+        k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
+        launches++;
+        if (cudaStreamSynchronize(stream) != cudaSuccess && r == MCG_OK) r = fail(MCG_ECUDA, "device run: mirrors");
         if (d_first) cudaFree(d_first);
         if (d_ranges) cudaFree(d_ranges);
         if (d_words) cudaFree(d_words);
@@ -2227,7 +2474,7 @@ int SingleEngine::commit() {
         memcpy(inl.idx, pending_idx.data(), 4 * (size_t)pending_m);
         memcpy(inl.xyz, pending_xyz.data(), 24 * (size_t)pending_m);
     }
-    k_commit<0><<<(pending_m + 127) / 128, 128, 0, stream>>>(pending_m, didx, dxyz, d_pq, d_fx, pbc, inl);
+    k_commit<<<(3 * pending_m + 127) / 128, 128, 0, stream>>>(pending_m, didx, dxyz, d_pq, d_fx, d_x64, fix64.sh, pbc, inl);
     CK(cudaGetLastError());
     for (int k = 0; k < pending_m; k++) {
         int a = pending_idx[k];

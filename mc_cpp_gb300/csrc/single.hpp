@@ -10,6 +10,7 @@
 #include "groups.hpp"
 #include "dev_types.hpp"
 #include "engine.hpp"
+#include "fixed64.hpp"
 
 namespace mcg {
 
@@ -108,6 +109,13 @@ private:
     int* d_cls_of = nullptr;      // parameter class of each atom (also in the mirror's w)
     float4* d_cls = nullptr;      // the classes' (q hi, q lo, eps, sig); ncls = 0: per-atom gathers
     int ncls = 0;
+    // FP64 energies in periodic boxes run on 64-bit integer pair terms (k_energy_list<PREC_F64> and
+    // k_energy_all<PREC_F64> are left with systems without a box, whose coordinates have no fixed range)
+    bool uses_fix64() const { return hs.prec == MCG_PREC_FP64 && hs.pbc != MCG_PBC_NONE; }
+    Fix64Geom fix64{};
+    ulonglong4_32a* d_x64 = nullptr;
+    Fix64Pair* d_pair64 = nullptr;   // ncls64 x ncls64; ncls64 = 0: products formed per pair
+    int ncls64 = 0;
     uint8_t* d_frozen = nullptr;
     int *d_xs = nullptr, *d_xd = nullptr, *d_fxs = nullptr, *d_fxd = nullptr;
     int2* d_p14 = nullptr;

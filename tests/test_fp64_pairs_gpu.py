@@ -6,6 +6,8 @@ terms' magnitudes bounds both for the sizes here.  Only totals are visible, so t
 taken from the oracle's energies of the attractive and repulsive parts, |elec| + |vdw| of the same
 system with all charges made positive.
 """
+from decimal import Decimal, localcontext
+
 import numpy as np
 import pytest
 
@@ -64,3 +66,113 @@ def test_minimum_image_at_its_switch_points(boxes, offset):
     s.set_coords(xyz)
     got = FFieldCUDA(s, "fp64", moves=False).getE10()
     _check(s, got, np.array(orc.Oracle(s, moves=False).energy()))
+
+
+def _near(s, seed, jitter=0.3):
+    """A configuration with pairs on both sides of the cutoffs: the lattice shaken up."""
+    rng = np.random.default_rng(seed)
+    s.set_coords(s.coords() + rng.uniform(-jitter, jitter, (s.natom, 3)))
+    return s
+
+
+# 2 atoms (one pair, mostly empty rings), sizes around a block's rows and a ring's 32 pairs, and
+# parameter sets on both sides of the class table's limit of 128
+@pytest.mark.parametrize("n", [2, 9, 32, 33, 127, 128, 129, 500, 1531])
+@pytest.mark.parametrize("box", ["cubic", "orbic"])
+def test_switched_energy(n, box):
+    s = _near(_charged_argon(n, 11), 12)
+    if n < 200:          # boxes of at least the cutoff, so that small systems have pairs at all ranges
+        s.box = (25.0, 25.0, 25.0)
+        s.set_coords(s.coords() * (25.0 / max(np.ptp(s.coords()), 1.0)) * 0.9)
+    if box == "orbic":
+        s.pbc_type = "orbic"
+        s.box = (s.box[0], s.box[1] * 1.25, s.box[2] * 1.0625)
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    _check(s, got, np.array(orc.Oracle(s, moves=False).energy()))
+
+
+# a unit of the full energy is 128 rows by 32 columns; 129 parameter sets leave the class table
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 127, 128, 129, 160, 161, 257, 1000])
+@pytest.mark.parametrize("box", ["cubic", "orbic"])
+def test_full_energy(n, box):
+    s = _near(_charged_argon(n, 31, cut_mode="full"), 32)
+    if box == "orbic":
+        s.pbc_type = "orbic"
+        s.box = (s.box[0], s.box[1] * 1.5, s.box[2] * 1.0625)
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    _check(s, got, np.array(orc.Oracle(s, moves=False).energy()))
+
+
+def test_full_energy_with_exclusions():
+    s = systems.water_box(173, seed=9)
+    s.cut_mode = "full"
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    _check(s, got, np.array(orc.Oracle(s, moves=False).energy()))
+
+
+# boxes on both sides of twice the pairs' reach (the smallest accepted holds the cutoff sphere exactly)
+@pytest.mark.parametrize("L", [24.0, 24.002, 24.003, 25.0])
+@pytest.mark.parametrize("box", ["cubic", "orbic"])
+def test_switched_energy_smallest_boxes(L, box):
+    s = _near(_charged_argon(64, 41), 42)
+    s.set_coords(s.coords() * (L / s.box[0]))
+    s.box = (L, L, L)
+    if box == "orbic":
+        s.pbc_type = "orbic"
+        s.box = (L, L * 1.25, L * 1.0625)
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    _check(s, got, np.array(orc.Oracle(s, moves=False).energy()))
+
+
+@pytest.mark.parametrize("ron", [0.0, 5.0, 11.9])
+def test_switched_energy_other_switches(ron):
+    s = _near(_charged_argon(600, 3, cuton=ron), 4)
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    _check(s, got, np.array(orc.Oracle(s, moves=False).energy()))
+
+
+def _exact_pair(s):
+    """(elec, vdw) of atoms 0 and 1 in 60 digits: near the cutoffs the FP64 switch is ill-conditioned."""
+    with localcontext() as c:
+        c.prec = 60
+        D = Decimal
+        u = D(0)
+        for k, v in enumerate((s.x, s.y, s.z)):
+            d, L = D(float(v[1])) - D(float(v[0])), D(float(s.box[k]))
+            u += (d - L * (d / L).to_integral_value()) ** 2
+        rc2, ron2 = D(s.cutoff) ** 2, D(s.cuton) ** 2
+        f = D(0) if u > rc2 else (D(1) if u <= ron2 else (rc2 - u) ** 2 * (rc2 + 2 * u - 3 * ron2) / (rc2 - ron2) ** 3)
+        e = [D(float(np.sqrt(v * 418.4))) for v in s.eps[:2]]
+        x6 = ((D(float(s.sig[0])) + D(float(s.sig[1]))) ** 2 / u) ** 3
+        elec = D(float(332.0716 * 418.4)) * D(float(s.q[0])) * D(float(s.q[1])) / u.sqrt() * f
+        return np.array([float(elec), float(4 * e[0] * e[1] * (x6 * x6 - x6) * f)])
+
+
+# closer than the 64-bit form's limit (some 2e-3 A), at it, above it; on the cutoffs
+@pytest.mark.parametrize("r", [1e-5, 1e-3, 2e-3, 4e-3, 0.5, 9.9995, 10.0, 10.0005, 11.9995, 12.0, 12.0005])
+def test_one_pair(r):
+    s = _charged_argon(3, 7)
+    s.box = (40.0, 40.0, 40.0)
+    s.set_coords(np.array([[-19.9, 3.0, -2.0], [-19.9 - r * 0.6, 3.0 + r * 0.8, -2.0], [1.0, -12.0, 17.5]]))
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    want = _exact_pair(s)
+    # one term: its displacement carries the coordinates' rounding (2^-49 A) on either side
+    rel = 40 * 2.0 ** -53 + 14 * 2.0 ** -48 / r
+    assert np.all(np.isfinite(got)) and np.all(np.abs(got[3:5] - want) <= rel * _scale(s) + 1e-30), (got, want)
+
+
+def test_moves_keep_the_mirror_current():
+    s = _near(_charged_argon(700, 21), 22, 0.1)
+    ff = FFieldCUDA(s, "fp64", moves=False)
+    xyz = s.coords()
+    rng = np.random.default_rng(1)
+    for _ in range(5):
+        idx = rng.choice(s.natom, 3, replace=False)
+        new = xyz[idx] + rng.uniform(-0.2, 0.2, (3, 3))
+        ff.delta_e(idx, new)
+        ff.commit()
+        xyz[idx] = new
+    got = ff.getE10()
+    s.set_coords(xyz)
+    o = orc.Oracle(s, moves=False)
+    _check(s, got, np.array(o.energy()))
