@@ -45,6 +45,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.hpp"
+#include "fixed64.cuh"
 #include "mcg.h"
 #include "pair_math.cuh"
 
@@ -1023,45 +1024,142 @@ __device__ __forceinline__ double master_to_f64(unsigned long long v, double L) 
     return (double)(long long)v * (L * (1.0 / TWO64));
 }
 
-// ---- fresh FP64 energy of every chain (reference arithmetic, all pairs, cutoff + switch)
-constexpr int ETILE = 128;
-__global__ void k_batch_energy64(const ChainDev* __restrict__ chains, const int* __restrict__ tile_chain,
-                                 const int* __restrict__ tile_first, const ulonglong4_32a* __restrict__ M,
-                                 const double* __restrict__ prm, CutDev cut, double* part) {
-    const int t = blockIdx.x;
-    const int c = tile_chain[t];
-    const ChainDev& C = chains[c];
-    const int n = C.nres * C.apr;
-    const int i = tile_first[t] + threadIdx.x;
-    double s = 0.0;
-    if (i < n) {
-        PbcDev pbc;
-        pbc.type = 2;
-        for (int k = 0; k < 3; k++) { pbc.L[k] = C.L[k]; pbc.rL[k] = C.rL[k]; }
-        const ulonglong4_32a ma = M[C.atom0 + i];
-        const double ax = master_to_f64(ma.x, C.L[0]), ay = master_to_f64(ma.y, C.L[1]), az = master_to_f64(ma.z, C.L[2]);
-        const int ri = i / C.apr;
-        const double* pa = prm + 3 * (size_t)(C.atom0 + i);
-        for (int j = i + 1; j < n; j++) {
-            if (j / C.apr == ri) continue;  // intra-residue pairs are excluded
-            const ulonglong4_32a mb = M[C.atom0 + j];
-            const double r2 = ref64_dist2(ax, ay, az, master_to_f64(mb.x, C.L[0]), master_to_f64(mb.y, C.L[1]),
-                                          master_to_f64(mb.z, C.L[2]), pbc);
-            if (r2 > cut.c2) continue;
-            const double* pb = prm + 3 * (size_t)(C.atom0 + j);
-            double el, vd;
-            ref64_pair(r2, pa[0], pb[0], pa[1], pb[1], pa[2], pb[2], true, cut, el, vd);
-            s += CHGCHARMM * KCALTOIU * el + 4.0 * vd;
+// ---- fresh FP64 energy of every chain (all pairs, cutoff + switch), on 64-bit integer pair terms
+// (fixed64.cuh; the masters are box fractions already).  Two kernels:
+//  - k_batch_extent: each chain's largest distance from a residue's first atom to its other atoms, from
+//    the mirrors, so that residues whose first atoms are farther than rc + 2 extents share no pair;
+//  - k_batch_energy64: a CTA per E64_RES residues of a chain, a warp per residue r.  Its lanes test
+//    the first atoms of all residues q > r by FP32 distance; the residue pairs within reach go to a ring,
+//    32 of them at a time are split into atom pairs, placed by FP32 distance again, and the atom pairs
+//    within rc go to two rings (inside ron, or switched), each evaluated with all 32 lanes busy.
+// Nothing depends on the neighbour lists.  The tests are FP32 and cheap: a chain of 8,192 residues takes
+// about 2,600 warp instructions of them per residue, beside some 11,000 for its pair terms.
+// 64 water chains of 512 to 8,192 molecules: 3.5 ms, 308 ms with a thread per atom over all later atoms
+// in FP64.
+constexpr int E64_RING = 64;      // up to 31 pending entries and 32 new ones
+constexpr int E64_RES = 32;       // residues of a CTA (8 when that leaves SMs without one)
+
+__global__ void __launch_bounds__(256) k_batch_extent(const ChainDev* __restrict__ chains, const uint4* __restrict__ F,
+                                                      int* ext2) {
+    const ChainDev& C = chains[blockIdx.x];
+    float d2 = 0.0f;
+    for (int r = blockIdx.y * blockDim.x + threadIdx.x; r < C.nres; r += gridDim.y * blockDim.x) {
+        const uint4 a = F[C.atom0 + r * C.apr];
+        for (int k = 1; k < C.apr; k++) {
+            const uint4 b = F[C.atom0 + r * C.apr + k];
+            const float dx = fdelta(a.x, b.x, C.Ls[0], C.Lsl[0]), dy = fdelta(a.y, b.y, C.Ls[1], C.Lsl[1]),
+                        dz = fdelta(a.z, b.z, C.Ls[2], C.Lsl[2]);
+            d2 = fmaxf(d2, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
         }
     }
+    for (int o = 16; o > 0; o >>= 1) d2 = fmaxf(d2, __shfl_xor_sync(0xffffffffu, d2, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(&ext2[blockIdx.x], __float_as_int(d2));   // non-negative floats order as their bits
+}
+
+__global__ void __launch_bounds__(256) k_batch_energy64(const ChainDev* __restrict__ chains, const Fix64Geom* __restrict__ geom,
+                                                        const Fix64Pair* __restrict__ table, const int* __restrict__ ext2,
+                                                        const int* __restrict__ tile_chain, const int* __restrict__ tile_first,
+                                                        int tile_res, const ulonglong4_32a* __restrict__ M,
+                                                        const uint4* __restrict__ F, double* part) {
+    __shared__ int2 s_ring[8][3][E64_RING];
+    __shared__ Fix64Geom G;
+    const int c = tile_chain[blockIdx.x];
+    const ChainDev& C = chains[c];
+    const int nres = C.nres, apr = C.apr, lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    if (threadIdx.x == 0) G = geom[c];
+    __syncthreads();
+    const Fix64Pair* tab = table + (size_t)c * MAX_APR * MAX_APR;
+    const uint4* Fc = F + C.atom0;
+    const ulonglong4_32a* Mc = M + C.atom0;
+    int2* res_ring = s_ring[wib][0];
+    int2* ring = s_ring[wib][1];               // inside ron, then the switched pairs at + E64_RING
+    const float reach = sqrtf(G.out2) + 2.0f * sqrtf(__int_as_float(ext2[c])) + 1e-3f;
+    const float reach2 = reach * reach;
+    const int last_res = min(tile_first[blockIdx.x] + tile_res, nres);
+    double sel = 0.0, svd = 0.0;
+    int rhead = 0, rtail = 0, head0 = 0, tail0 = 0, head1 = 0, tail1 = 0;
+    int r = tile_first[blockIdx.x] + wib, q0 = r + 1;
+    auto dist2 = [&](const uint4& a, const uint4& b) {
+        const float dx = fdelta(a.x, b.x, G.Ls[0], G.Ll[0]), dy = fdelta(a.y, b.y, G.Ls[1], G.Ll[1]),
+                    dz = fdelta(a.z, b.z, G.Ls[2], G.Ll[2]);
+        return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    };
+    for (;;) {
+        const bool last = r >= last_res;
+        if (!last) {
+            const int q = q0 + lane;
+            const bool near = q < nres && dist2(Fc[r * apr], Fc[min(q, nres - 1) * apr]) <= reach2;
+            const unsigned b = __ballot_sync(0xffffffffu, near);
+            if (near) res_ring[(rhead + __popc(b & below)) & (E64_RING - 1)] = make_int2(r * apr, q * apr);
+            rhead += __popc(b);
+            q0 += 32;
+            if (q0 >= nres) { r += 8; q0 = r + 1; }
+            __syncwarp();
+            if (rhead - rtail < 32) continue;
+        }
+        // 32 residue pairs (at the end: what is left), then, at the end, what is left of the atom pairs
+        const bool flush = last && rhead - rtail <= 32;
+        const bool have = lane < rhead - rtail;
+        const int2 rp = have ? res_ring[(rtail + lane) & (E64_RING - 1)] : make_int2(0, 0);
+        rtail = min(rtail + 32, rhead);
+        int ka = 0, kb = 0;
+        for (int s = 0; s < apr * apr + (flush ? 1 : 0); s++) {
+            const bool rest = s == apr * apr;
+            if (!rest) {
+                const int i = rp.x + ka, j = rp.y + kb;
+                const float r2 = have ? dist2(Fc[i], Fc[j]) : 3.0e38f;
+                const bool in = r2 < G.in2, sw = !in && r2 <= G.out2;
+                const unsigned bi = __ballot_sync(0xffffffffu, in), bs = __ballot_sync(0xffffffffu, sw);
+                if (in) ring[(head0 + __popc(bi & below)) & (E64_RING - 1)] = make_int2(i << 3 | ka, j << 3 | kb);
+                if (sw) ring[E64_RING + ((head1 + __popc(bs & below)) & (E64_RING - 1))] = make_int2(i << 3 | ka, j << 3 | kb);
+                head0 += __popc(bi);
+                head1 += __popc(bs);
+                if (++kb == apr) { kb = 0; ka++; }
+                __syncwarp();
+            }
+            const int least = rest ? 1 : 32;
+            for (;;) {
+                const bool sw = head0 - tail0 < least;
+                if (sw && head1 - tail1 < least) break;
+                const int at = sw ? E64_RING + ((tail1 + lane) & (E64_RING - 1)) : (tail0 + lane) & (E64_RING - 1);
+                if (lane < (sw ? head1 - tail1 : head0 - tail0)) {
+                    const int2 p = ring[at];
+                    const int i = p.x >> 3, j = p.y >> 3;
+                    const ulonglong4_32a a = Mc[i], b = Mc[j];
+                    const double4_32a t = reinterpret_cast<const double4_32a*>(tab)[(p.x & 7) * MAX_APR + (p.y & 7)];
+                    const unsigned long long dx = b.x - a.x << G.sh, dy = b.y - a.y << G.sh, dz = b.z - a.z << G.sh;
+                    const Fix64Dist u = G.iso ? fix64_dist2<true>(G, dx, dy, dz) : fix64_dist2<false>(G, dx, dy, dz);
+                    double ys, w, ws;
+                    if (fix64_terms(G, u, sw, ys, w, ws)) {
+                        sel = fma(t.x, ys, sel);
+                        svd = fma(fma(t.z, w, -t.y), ws, svd);
+                    } else {
+                        // closer than the 64-bit form reaches: the same products on an FP64 distance
+                        const double ex = (double)(long long)(b.x - a.x) * (C.L[0] * (1.0 / TWO64)),
+                                     ey = (double)(long long)(b.y - a.y) * (C.L[1] * (1.0 / TWO64)),
+                                     ez = (double)(long long)(b.z - a.z) * (C.L[2] * (1.0 / TWO64));
+                        const double y = rsqrt64(ex * ex + ey * ey + ez * ez) * G.leff, y2 = y * y, y6 = y2 * y2 * y2;
+                        sel = fma(t.x, y, sel);
+                        svd = fma(fma(t.z, y6, -t.y), y6, svd);
+                    }
+                }
+                if (sw) tail1 = min(tail1 + 32, head1);
+                else tail0 = min(tail0 + 32, head0);
+            }
+            __syncwarp();
+        }
+        if (flush) break;
+    }
+    double s = CHGCHARMM * KCALTOIU * sel + 4.0 * svd;
     s = warp_sum(s);
-    __shared__ double sh[ETILE / 32];
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __shared__ double sh[8];
+    if (lane == 0) sh[wib] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
         double v = 0.0;
-        for (int w = 0; w < ETILE / 32; w++) v += sh[w];
-        part[t] = v;
+        for (int w = 0; w < 8; w++) v += sh[w];
+        part[blockIdx.x] = v;
     }
 }
 
@@ -1334,12 +1432,16 @@ struct mcg_batch {
     uint4* d_gpos = nullptr;      // first-atom positions in cell order, w = residue (list builds)
     int *d_item_chain = nullptr, *d_chain_item0 = nullptr, *d_build = nullptr;
     int nitems = 0;               // list-build work items (home cells, or 32-residue chunks) of all chains
-    double* d_prm = nullptr;
+    // FP64 energies: each chain's 64-bit geometry, slot-pair products and extent, tiles of tile_res residues
+    Fix64Geom* d_geom64 = nullptr;
+    Fix64Pair* d_pair64 = nullptr;
+    int* d_ext2 = nullptr;
+    int tile_res = 0;
+    std::vector<int> tile_chain;
     int* d_tile_chain = nullptr;
     int* d_tile_first = nullptr;
     double* d_part = nullptr;
     int ntiles = 0;
-    CutDev cut64{};
     cudaGraphExec_t graph = nullptr;
     cudaGraphExec_t tgraph = nullptr;   // the same sweep with event records around its two phases
     cudaEvent_t tev[3] = {nullptr, nullptr, nullptr};
@@ -1370,7 +1472,7 @@ struct mcg_batch {
         if (stream2) cudaStreamDestroy(stream2);
         if (d_cl_order) cudaFree(d_cl_order);
         if (d_cl_start) cudaFree(d_cl_start);
-        void* p[] = {d_chains, d_state, d_order, d_M, d_F, d_FB, d_LST, d_NL, d_gorder, d_gcell, d_prm, d_tile_chain,
+        void* p[] = {d_chains, d_state, d_order, d_M, d_F, d_FB, d_LST, d_NL, d_gorder, d_gcell, d_geom64, d_pair64, d_ext2, d_tile_chain,
                      d_tile_first, d_part, d_xyz, d_gstarts, d_res_chain, d_eres, d_cta_start, d_gpos, d_item_chain,
                      d_chain_item0, d_build, d_log, d_changed};
         for (void* q : p) if (q) cudaFree(q);
@@ -1648,7 +1750,8 @@ int mcg_batch_create(const mcg_system_desc* descs, int nchains, const mcg_batch_
     const double rc = d0.cutoff, ron = d0.cuton, skin = d0.dcut > 0 ? d0.dcut : 2.0;
     std::vector<ulonglong4_32a> M;
     std::vector<uint4> F;
-    std::vector<double> prm;
+    std::vector<Fix64Geom> geom64(nchains);
+    std::vector<Fix64Pair> pair64((size_t)nchains * MAX_APR * MAX_APR);
     double rext = 0.0;       // largest distance from a residue's first atom to its other atoms
     double span_max = 0.0;   // largest intra-residue distance
     int apr_all = -1;
@@ -1719,12 +1822,16 @@ int mcg_batch_create(const mcg_system_desc* descs, int nchains, const mcg_batch_
                 C.tab[a][b][2] = (float)(s * s);
                 C.tablo[a][b][1] = (float)(s * s - (double)(float)(s * s));
             }
+        geom64[c] = fix64_geom(hs.L, rc, ron);
+        for (int a = 0; a < apr; a++)
+            for (int b = 0; b < apr; b++)
+                pair64[((size_t)c * MAX_APR + a) * MAX_APR + b] =
+                    fix64_pair(hs.q[a], hs.eps[a], hs.sig[a], hs.q[b], hs.eps[b], hs.sig[b], geom64[c].leff);
         for (int i = 0; i < hs.n; i++) {
             ulonglong4_32a m;
             m.x = host_master(hs.x[i], hs.rL[0]); m.y = host_master(hs.y[i], hs.rL[1]); m.z = host_master(hs.z[i], hs.rL[2]); m.w = 0;
             M.push_back(m);
             F.push_back(make_uint4((uint32_t)(m.x >> 32), (uint32_t)(m.y >> 32), (uint32_t)(m.z >> 32), (uint32_t)(i % apr)));
-            prm.push_back(hs.q[i]); prm.push_back(hs.eps[i]); prm.push_back(hs.sig[i]);
         }
         for (int r = 0; r < nres; r++)
             for (int k = 0; k < apr; k++)
@@ -1841,7 +1948,8 @@ int mcg_batch_create(const mcg_system_desc* descs, int nchains, const mcg_batch_
     if ((r = balloc(&B->d_chains, nchains)) || (r = balloc(&B->d_state, nchains)) ||
         (r = balloc(&B->d_M, atom0)) || (r = balloc(&B->d_F, atom0)) || (r = balloc(&B->d_FB, atom0)) ||
         (r = balloc(&B->d_LST, (size_t)res0 * G.cap)) || (r = balloc(&B->d_NL, res0)) || (r = balloc(&B->d_gorder, res0)) ||
-        (r = balloc(&B->d_gcell, res0)) || (r = balloc(&B->d_prm, prm.size())) ||
+        (r = balloc(&B->d_gcell, res0)) || (r = balloc(&B->d_geom64, nchains)) || (r = balloc(&B->d_pair64, pair64.size())) ||
+        (r = balloc(&B->d_ext2, nchains)) ||
         (r = balloc(&B->d_gstarts, (size_t)nchains * (MAX_CELLS + 1))) || (r = balloc(&B->d_res_chain, res0)) ||
         (r = balloc(&B->d_gpos, res0)))
         return r;
@@ -1854,13 +1962,14 @@ int mcg_batch_create(const mcg_system_desc* descs, int nchains, const mcg_batch_
     BK(cudaMemcpyAsync(B->d_chains, B->chains.data(), sizeof(ChainDev) * nchains, cudaMemcpyHostToDevice, B->stream));
     BK(cudaMemcpyAsync(B->d_M, M.data(), sizeof(ulonglong4_32a) * atom0, cudaMemcpyHostToDevice, B->stream));
     BK(cudaMemcpyAsync(B->d_F, F.data(), sizeof(uint4) * atom0, cudaMemcpyHostToDevice, B->stream));
-    BK(cudaMemcpyAsync(B->d_prm, prm.data(), sizeof(double) * prm.size(), cudaMemcpyHostToDevice, B->stream));
+    BK(cudaMemcpyAsync(B->d_geom64, geom64.data(), sizeof(Fix64Geom) * nchains, cudaMemcpyHostToDevice, B->stream));
+    BK(cudaMemcpyAsync(B->d_pair64, pair64.data(), sizeof(Fix64Pair) * pair64.size(), cudaMemcpyHostToDevice, B->stream));
     BK(cudaMemsetAsync(B->d_state, 0, sizeof(ChainState) * nchains, B->stream));
-    std::vector<int> tc, tf;
-    for (int c = 0; c < nchains; c++) {
-        int n = B->chains[c].nres * B->chains[c].apr;
-        for (int f = 0; f < n; f += ETILE) { tc.push_back(c); tf.push_back(f); }
-    }
+    std::vector<int>& tc = B->tile_chain;
+    std::vector<int> tf;
+    B->tile_res = res0 >= (int64_t)4 * B->nsm * E64_RES ? E64_RES : 8;   // four CTAs of the larger tiles per SM, or the smaller
+    for (int c = 0; c < nchains; c++)
+        for (int f = 0; f < B->chains[c].nres; f += B->tile_res) { tc.push_back(c); tf.push_back(f); }
     B->ntiles = (int)tc.size();
     if ((r = balloc(&B->d_tile_chain, tc.size())) || (r = balloc(&B->d_tile_first, tf.size())) || (r = balloc(&B->d_part, tc.size())))
         return r;
@@ -1880,9 +1989,6 @@ int mcg_batch_create(const mcg_system_desc* descs, int nchains, const mcg_batch_
         BK(cudaMemcpy(B->d_chain_item0, i0.data(), sizeof(int) * nchains, cudaMemcpyHostToDevice));
     }
     BK(cudaMemcpyAsync(B->d_tile_first, tf.data(), sizeof(int) * tf.size(), cudaMemcpyHostToDevice, B->stream));
-    B->cut64.mode = 1;
-    B->cut64.c2 = rc * rc; B->cut64.n2 = ron * ron;
-    { double dd = B->cut64.c2 - B->cut64.n2; B->cut64.sw2 = 1. / (dd * dd * dd); }
     if ((r = B->launch_build())) return r;
     std::vector<double> e(nchains);
     r = mcg_batch_energy_fp64(B.get(), e.data());
@@ -2210,17 +2316,17 @@ int mcg_batch_stats(mcg_batch* b, int64_t* trials, int64_t* accepted, double* et
 
 int mcg_batch_energy_fp64(mcg_batch* b, double* e) {
     if (!b || !e) return fail(MCG_EINVAL, "null argument");
-    k_batch_energy64<<<b->ntiles, ETILE, 0, b->stream>>>(b->d_chains, b->d_tile_chain, b->d_tile_first, b->d_M, b->d_prm,
-                                                         b->cut64, b->d_part);
+    BK(cudaMemsetAsync(b->d_ext2, 0, sizeof(int) * b->nchains, b->stream));
+    k_batch_extent<<<dim3(b->nchains, 8), 256, 0, b->stream>>>(b->d_chains, b->d_F, b->d_ext2);
+    k_batch_energy64<<<b->ntiles, 256, 0, b->stream>>>(b->d_chains, b->d_geom64, b->d_pair64, b->d_ext2, b->d_tile_chain,
+                                                       b->d_tile_first, b->tile_res, b->d_M, b->d_F, b->d_part);
     BK(cudaGetLastError());
     std::vector<double> part(b->ntiles);
-    std::vector<int> tc(b->ntiles);
     BK(cudaMemcpyAsync(part.data(), b->d_part, sizeof(double) * b->ntiles, cudaMemcpyDeviceToHost, b->stream));
-    BK(cudaMemcpyAsync(tc.data(), b->d_tile_chain, sizeof(int) * b->ntiles, cudaMemcpyDeviceToHost, b->stream));
     BK(cudaStreamSynchronize(b->stream));
     for (int c = 0; c < b->nchains; c++) e[c] = 0.0;
-    for (int t = 0; t < b->ntiles; t++) e[tc[t]] += part[t];
-    b->launches += 1;
+    for (int t = 0; t < b->ntiles; t++) e[b->tile_chain[t]] += part[t];
+    b->launches += 2;
     return MCG_OK;
 }
 

@@ -13,7 +13,7 @@ import pytest
 
 import oracle as orc
 from mc_cpp_gb300 import build, native, systems
-from mc_cpp_gb300.engine import FFieldCUDA
+from mc_cpp_gb300.engine import BatchChains, FFieldCUDA
 
 pytestmark = pytest.mark.gpu
 REL = 1e-13
@@ -176,3 +176,36 @@ def test_moves_keep_the_mirror_current():
     s.set_coords(xyz)
     o = orc.Oracle(s, moves=False)
     _check(s, got, np.array(o.energy()))
+
+
+def _check_chains(B, chains):
+    e = B.energy_fp64()
+    for k, s in enumerate(chains):
+        t = s.copy()
+        t.set_coords(B.coords(k))
+        want = np.array(orc.Oracle(t, moves=False).energy())
+        assert abs(e[k] - (want[3] + want[4])) <= REL * _scale(t), (k, e[k], want)
+
+
+# tiles of 8 or 32 residues (the larger from 19,456 residues in all), residue sizes 1 and 3 and both
+@pytest.mark.parametrize("sizes", [[("water", 513)], [("argon", 331), ("argon", 513)], [("water", 512), ("argon", 640), ("water", 519)],
+                                   [("water", 6500), ("water", 6489), ("water", 6511)]])
+def test_batch_energy(sizes):
+    chains = [systems.water_box(n, seed=n) if kind == "water" else systems.argon_random(n, 0.0213, n) for kind, n in sizes]
+    if len(chains) == 2:
+        chains[1].pbc_type = "orbic"
+        chains[1].box = (chains[1].box[0], chains[1].box[1] * 1.25, chains[1].box[2] * 1.0625)
+    B = BatchChains(chains, seed=3)
+    _check_chains(B, chains)
+    B.sweep(1)
+    _check_chains(B, chains)
+
+
+def test_batch_energy_of_residues_wider_than_at_creation():
+    chains = [systems.water_box(600, seed=1)]
+    B = BatchChains(chains, seed=3)
+    xyz = chains[0].coords()
+    xyz[4] += [4.0, -5.0, 6.0]
+    xyz[901] += [-9.0, 0.0, 2.0]
+    B.set_coords(0, xyz)
+    _check_chains(B, chains)
