@@ -93,29 +93,39 @@ __global__ void k_cell_assign(const double4_32a* __restrict__ pq, int n, PbcDev 
     atomicAdd(&cell_count[cell], 1);
 }
 
-// Exclusive scan of cell counts by one block (cells are few: one per (rc+skin)^3 of volume).
-__global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int* cell_start, int* cell_fill) {
-    __shared__ int sh[1024];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < ncell; base += 1024) {
-        int i = base + threadIdx.x;
-        int v = i < ncell ? cell_count[i] : 0;
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            int t = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += t;
-            __syncthreads();
+// Exclusive scans by one block (cells are few) of the cell counts and of the cells' row-build tasks
+// (runs of at most `run` home atoms), carried together in the halves of a 64-bit sum.
+__global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int run, int* cell_start, int* cell_fill,
+                            int* task_start) {
+    __shared__ unsigned long long sw[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (int base = 0; base < ncell; base += blockDim.x) {
+        const int i = base + threadIdx.x;
+        const unsigned v = i < ncell ? (unsigned)cell_count[i] : 0u;
+        const unsigned long long own = (unsigned long long)((v + run - 1) / run) << 32 | v;
+        unsigned long long s = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += up;
         }
-        if (i < ncell) { cell_start[i] = carry + sh[threadIdx.x] - v; cell_fill[i] = 0; }
+        if (lane == 31) sw[w] = s;
         __syncthreads();
-        if (threadIdx.x == 1023) carry += sh[1023];
+        if (w == 0) {
+            unsigned long long t = sw[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long up = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= o) t += up;
+            }
+            sw[lane] = t;
+        }
+        __syncthreads();
+        const unsigned long long at = carry + (w ? sw[w - 1] : 0ull) + s - own;
+        if (i < ncell) { cell_start[i] = (int)(unsigned)at; cell_fill[i] = 0; task_start[i] = (int)(at >> 32); }
+        carry += sw[31];
         __syncthreads();
     }
-    if (threadIdx.x == 0) cell_start[ncell] = carry;
+    if (threadIdx.x == 0) { cell_start[ncell] = (int)(unsigned)carry; task_start[ncell] = (int)(carry >> 32); }
 }
 
 __global__ void k_cell_scatter(const int* __restrict__ cell_of, int n, const int* __restrict__ cell_start,
@@ -127,13 +137,18 @@ __global__ void k_cell_scatter(const int* __restrict__ cell_of, int n, const int
     cell_atoms[cell_start[c] + slot] = i;
 }
 
-// Sort each cell's atoms ascending so rows come out in a deterministic order.
-__global__ void k_cell_sort(const int* __restrict__ cell_start, int ncell, int* cell_atoms) {
+// Sort each cell's atoms ascending so rows come out in a deterministic order, and write the cell's
+// share of the candidates in cell order (fixed-point position, atom index), of the home atoms grouped by
+// the octant of the cell they lie in (places in cell order), and of the row build's tasks: runs of at
+// most `run` of these.  The grouping only decides which rows are built together.
+__global__ void k_cell_sort(const int* __restrict__ cell_start, const int* __restrict__ task_start, int ncell, int run,
+                            const uint4* __restrict__ fx, Grid g, int* cell_atoms, uint4* cell_pos, int* home, int2* tasks) {
     __shared__ int sh[SORT_MAX];
+    __shared__ uint8_t oct[SORT_MAX];
     int c = blockIdx.x;
     if (c >= ncell) return;
     int b = cell_start[c], e = cell_start[c + 1], m = e - b;
-    if (m <= 1) return;
+    for (int k = threadIdx.x; k * run < m; k += blockDim.x) tasks[task_start[c] + k] = make_int2(c, b + k * run);
     if (m > SORT_MAX) {
         if (threadIdx.x == 0)
             for (int i = b + 1; i < e; i++) {
@@ -141,25 +156,49 @@ __global__ void k_cell_sort(const int* __restrict__ cell_start, int ncell, int* 
                 while (k >= b && cell_atoms[k] > v) { cell_atoms[k + 1] = cell_atoms[k]; k--; }
                 cell_atoms[k + 1] = v;
             }
-        return;
-    }
-    int m2 = 1;
-    while (m2 < m) m2 <<= 1;
-    for (int i = threadIdx.x; i < m2; i += blockDim.x) sh[i] = i < m ? cell_atoms[b + i] : 0x7fffffff;
-    __syncthreads();
-    for (int k = 2; k <= m2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < m2; i += blockDim.x) {
-                int l = i ^ j;
-                if (l > i) {
-                    bool up = (i & k) == 0;
-                    int a = sh[i], bb = sh[l];
-                    if ((a > bb) == up) { sh[i] = bb; sh[l] = a; }
+        __syncthreads();
+    } else if (m > 1) {
+        int m2 = 1;
+        while (m2 < m) m2 <<= 1;
+        for (int i = threadIdx.x; i < m2; i += blockDim.x) sh[i] = i < m ? cell_atoms[b + i] : 0x7fffffff;
+        __syncthreads();
+        for (int k = 2; k <= m2; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int i = threadIdx.x; i < m2; i += blockDim.x) {
+                    int l = i ^ j;
+                    if (l > i) {
+                        bool up = (i & k) == 0;
+                        int a = sh[i], bb = sh[l];
+                        if ((a > bb) == up) { sh[i] = bb; sh[l] = a; }
+                    }
                 }
+                __syncthreads();
             }
-            __syncthreads();
+        for (int i = threadIdx.x; i < m; i += blockDim.x) cell_atoms[b + i] = sh[i];
+        __syncthreads();
+    }
+    for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
+        const int a = cell_atoms[i];
+        uint4 p = fx[a];
+        p.w = (unsigned)a;
+        cell_pos[i] = p;
+        if (m <= SORT_MAX) {   // the half of the cell along each axis, from the box fraction
+            const unsigned hx = (unsigned)((unsigned long long)p.x * (2 * g.nc[0]) >> 32) & 1u,
+                           hy = (unsigned)((unsigned long long)p.y * (2 * g.nc[1]) >> 32) & 1u,
+                           hz = (unsigned)((unsigned long long)p.z * (2 * g.nc[2]) >> 32) & 1u;
+            oct[i - b] = (uint8_t)(hz << 2 | hy << 1 | (hx ^ hy));   // neighbouring octants share a face
+        } else {
+            home[i] = i;
         }
-    for (int i = threadIdx.x; i < m; i += blockDim.x) cell_atoms[b + i] = sh[i];
+    }
+    if (m > SORT_MAX) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const int o = oct[i];
+        int r = 0;
+        for (int k = 0; k < m; k++) r += oct[k] < o || (oct[k] == o && k < i);
+        home[b + r] = b + i;
+    }
 }
 
 struct ListParams {
@@ -168,9 +207,11 @@ struct ListParams {
     int maxspan;
     // periodic boxes: FP32 prefilter on the fixed-point mirrors.  A pair whose FP32 r^2 lies below
     // lo2 is inside, above hi2 outside; only the band between takes the reference's FP64 test.
-    float Ls[3], Ll[3];
+    // (A^2, or units of (L 2^-32)^2 when the box lengths are equal)
+    float Ls[3];
     float lo2, hi2;
     float reach2;   // rows of cells farther than this (squared, with a margin) are not scanned
+    int any_frozen;
 };
 
 __device__ __forceinline__ bool stored_excluded(int lo, int hi, const int* __restrict__ xs,
@@ -181,134 +222,139 @@ __device__ __forceinline__ bool stored_excluded(int lo, int hi, const int* __res
     return false;
 }
 
-// One warp per atom i; lanes walk the candidates of the stencil cells 32 at a time.  In periodic
-// boxes each candidate is first placed by its FP32 distance from the exact fixed-point mirrors
-// (error ~2e-7 of (rc + skin)^2); the reference's FP64 distance decides only the pairs within 1e-4
-// of the list radius, so the rows are the reference's sets at a fraction of the FP64 work (GB300's
-// FP64 rate is 1/64 of FP32).
-__global__ void __launch_bounds__(256) k_build_rows(const double4_32a* __restrict__ pq, const uint4* __restrict__ fx,
-                                                    const uint8_t* __restrict__ frozen,
-                                                    int n, PbcDev pbc, Grid g, ListParams lp,
-                                                    const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                                                    const int* __restrict__ cell_atoms, const int* __restrict__ xs,
-                                                    const int* __restrict__ xd, int* nbr, int* nup, int* nlo,
-                                                    int* max_row) {
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const bool periodic = pbc.type != 0;
-    for (int i = warp; i < n; i += nwarps) {
-        double4_32a pi = pq[i];
-        const uint4 xi = periodic ? fx[i] : make_uint4(0, 0, 0, 0);
-        bool fi = frozen[i] != 0;
-        const int c = cell_of[i];
+// A warp per task: up to A home atoms of one cell share the walk over the stencil's candidates, which
+// lie in cell order (coalesced 16-byte loads, no index gather), 32 at a time.  The stencil's rows of
+// cells become ranges of the candidates, dropped or trimmed where no home atom reaches; the ranges are
+// walked as one sequence (a lane finds its range by advancing through their prefix sums), so short
+// ranges leave no lane idle, and the next 32 candidates load while these are tested.  A row lists its
+// partners in the candidates' order, whatever the grouping.  In periodic boxes a pair is first placed by its
+// FP32 distance from the exact fixed-point mirrors (error ~2e-7 of (rc + skin)^2); the reference's FP64
+// distance decides only the pairs within 1e-4 of the list radius, so the rows are the reference's sets.
+// Before the home atoms' tests the candidates pass one against the sphere around all of them, and the
+// survivors (1,750 of 3,200 for four atoms of one octant of a water cell, 1,150 end in a row) are
+// gathered in a ring, 32 at a time.  Bound by issue.  (One atom per warp with an index gather in front
+// of every candidate took 1.48 ms on the 100,002-atom water box and 188 us at 12,288 atoms; this form
+// takes 0.70 ms and 123 us.)
+constexpr int ROW_WARPS = 4;
+constexpr int ROW_RING = 64;   // up to 31 pending candidates and 32 new ones
+
+// The pairs the FP32 test does not decide: in the band around the list radius, close in index (the atom
+// itself, or perhaps excluded), or with frozen atoms about.
+__device__ __noinline__ bool row_pair(const double4_32a* __restrict__ pq, const uint8_t* __restrict__ frozen, const PbcDev& pbc,
+                                      const ListParams& lp, const int* __restrict__ xs, const int* __restrict__ xd, int i, int j,
+                                      bool exact) {
+    if (j == i) return false;
+    if (exact) {
+        const double4_32a pi = pq[i], pj = pq[j];
+        if (!(ref64_dist2(pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, pbc) <= lp.cutnb2)) return false;
+    }
+    if (lp.any_frozen && frozen[i] && frozen[j]) return false;
+    return !stored_excluded(min(i, j), max(i, j), xs, xd, lp.maxspan);
+}
+
+// a predicated store: the branch around an ordinary one costs more than the store
+__device__ __forceinline__ void store_if(int* p, int v, bool pred) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q st.global.s32 [%0], %1;\n}" ::"l"(p), "r"(v), "r"((int)pred) : "memory");
+}
+
+template <int A, bool PERIODIC, bool ISO>
+__global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a* __restrict__ pq, const uint4* __restrict__ cell_pos,
+                                                               const uint8_t* __restrict__ frozen, PbcDev pbc, Grid g,
+                                                               ListParams lp, const int* __restrict__ cell_start,
+                                                               const int* __restrict__ task_start, int ncell,
+                                                               const int* __restrict__ home, const int2* __restrict__ tasks,
+                                                               const int* __restrict__ xs,
+                                                               const int* __restrict__ xd, int* nbr, int* nup, int* nlo,
+                                                               int* max_row) {
+    __shared__ int2 s_range[ROW_WARPS][66];
+    __shared__ uint4 s_ring[ROW_WARPS][ROW_RING];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    int2* range = s_range[wib];
+    uint4* ring = s_ring[wib];
+    const int ntask = task_start[ncell];
+    const int span = lp.any_frozen ? 0x3fffffff : lp.maxspan;   // frozen atoms: every pair is looked at
+    int longest = 0;
+    for (int task = blockIdx.x * ROW_WARPS + wib; task < ntask; task += gridDim.x * ROW_WARPS) {
+        const int2 tk = tasks[task];
+        const int c = tk.x, m = min(A, cell_start[c + 1] - tk.y);
         const int ctr[3] = {c % g.nc[0], (c / g.nc[0]) % g.nc[1], c / (g.nc[0] * g.nc[1])};
-        // per axis: the offsets scanned, and the atom's place inside its cell (in cell widths) for
-        // the distance from the atom to a cell d away along that axis.  FP32 throughout (FP64 here,
-        // warp-uniform but at GB300's FP64 rate, had cost more than the candidate tests): pos is
-        // off by ~1e-6 cell widths, inside the margin of lp.reach2.
+        // the home atoms: candidate entries tk.y .. tk.y + m; a missing one repeats the first and is not stored
+        uint32_t hx[A][3];
+        int hi[A], up[A], back[A];
+        int* row[A];
+#pragma unroll
+        for (int k = 0; k < A; k++) {
+            const uint4 p = cell_pos[home[tk.y + (k < m ? k : 0)]];
+            hx[k][0] = p.x; hx[k][1] = p.y; hx[k][2] = p.z;
+            hi[k] = (int)p.w;
+            up[k] = 0;
+            back[k] = lp.cap - 1;
+            row[k] = nbr + (size_t)p.w * lp.cap;
+        }
+        // per axis: the offsets scanned, and the home atoms' extent inside the cell (in cell widths) for
+        // the distance from them to a cell d away along that axis.  FP32 throughout (FP64 here, at
+        // GB300's FP64 rate, had cost more than the candidate tests): off by ~1e-6 cell widths, inside
+        // the margin of lp.reach2.
         int dlo[3], dhi[3];
         bool whole[3];
-        float pos[3];
-        const uint32_t fi3[3] = {xi.x, xi.y, xi.z};
-        const double ci[3] = {pi.x, pi.y, pi.z};
-        for (int k = 0; k < 3; k++) {
-            float p;
-            if (g.periodic) {   // the mirror holds the box fraction in units of 2^-32
-                p = (float)fi3[k] * 2.3283064365386963e-10f * (float)g.nc[k] - (float)ctr[k];
-                if (p < -0.5f * g.nc[k]) p += (float)g.nc[k];       // fraction just below 1, stored as 0
-                else if (p > 0.5f * g.nc[k]) p -= (float)g.nc[k];
-            } else {
-                p = (float)((ci[k] - g.lo[k]) * g.inv[k]) * (float)g.nc[k] - (float)ctr[k];
+        float pmin[3], pmax[3], ball2 = 0.f;
+        uint32_t ball[3] = {0, 0, 0};
+        {
+            const uint4 q = cell_pos[home[tk.y + min(lane, m - 1)]];
+            const uint32_t q3[3] = {q.x, q.y, q.z};
+            double d3[3] = {0, 0, 0};
+            if (!PERIODIC) { const double4_32a d = pq[q.w]; d3[0] = d.x; d3[1] = d.y; d3[2] = d.z; }
+            for (int k = 0; k < 3; k++) {
+                float p;
+                if (PERIODIC) {   // the mirror holds the box fraction in units of 2^-32
+                    p = (float)q3[k] * 2.3283064365386963e-10f * (float)g.nc[k] - (float)ctr[k];
+                    if (p < -0.5f * g.nc[k]) p += (float)g.nc[k];       // fraction just below 1, stored as 0
+                    else if (p > 0.5f * g.nc[k]) p -= (float)g.nc[k];
+                } else {
+                    p = (float)((d3[k] - g.lo[k]) * g.inv[k]) * (float)g.nc[k] - (float)ctr[k];
+                }
+                p = fminf(fmaxf(p, 0.f), 1.f);       // non-negative floats order as their bits
+                pmin[k] = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(p)));
+                pmax[k] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(p)));
+                whole[k] = PERIODIC && g.nc[k] < 5;
+                if (whole[k]) { dlo[k] = -ctr[k]; dhi[k] = g.nc[k] - 1 - ctr[k]; }
+                else if (PERIODIC) { dlo[k] = -2; dhi[k] = 2; }
+                else { dlo[k] = max(-2, -ctr[k]); dhi[k] = min(2, g.nc[k] - 1 - ctr[k]); }
             }
-            pos[k] = fminf(fmaxf(p, 0.f), 1.f);
-            whole[k] = g.periodic && g.nc[k] < 5;
-            if (whole[k]) { dlo[k] = -ctr[k]; dhi[k] = g.nc[k] - 1 - ctr[k]; }
-            else if (g.periodic) { dlo[k] = -2; dhi[k] = 2; }
-            else { dlo[k] = max(-2, -ctr[k]); dhi[k] = min(2, g.nc[k] - 1 - ctr[k]); }
+            if (PERIODIC) {   // the sphere around the home atoms: the middle of their extent, and its radius
+                float far2 = 0.f;
+                for (int k = 0; k < 3; k++) {
+                    const int d = (int)(q3[k] - hx[0][k]);
+                    const int mn = __reduce_min_sync(0xffffffffu, d), mx = __reduce_max_sync(0xffffffffu, d);
+                    const int mid = mn + (int)((unsigned)(mx - mn) >> 1);
+                    ball[k] = hx[0][k] + (uint32_t)mid;
+                    const float e = (float)(d - mid) * lp.Ls[k];
+                    far2 = fmaf(e, e, far2);
+                }
+                far2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(far2)));
+                const float reach = sqrtf(lp.reach2) + sqrtf(far2);
+                ball2 = reach * reach;
+            }
         }
         auto gap2 = [&](int k, int d) -> float {   // squared lower bound on |displacement| along axis k
             if (whole[k] || d == 0) return 0.f;
-            const float w = (d > 0 ? (float)(d - 1) + (1.f - pos[k]) : (float)(-d - 1) + pos[k]) * g.csf[k];
+            const float w = (d > 0 ? (float)(d - 1) + (1.f - pmax[k]) : (float)(-d - 1) + pmin[k]) * g.csf[k];
             return w * w;
         };
-        int up = 0, lo = 0;
-        int* row = nbr + (size_t)i * lp.cap;
-        // candidates b .. e-1 of cell_atoms, four batches of 32 in flight per warp (the index load
-        // and the gather behind it are the latency); rows keep the candidates' order
-        auto scan = [&](int b, int e) {
-            constexpr int U = 4;
-            for (int base = b; base < e; base += 32 * U) {
-                int jj[U];
-                uint4 xj[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int t = base + 32 * u + lane;
-                    jj[u] = t < e ? cell_atoms[t] : -1;
-                }
-                if (periodic) {
-#pragma unroll
-                    for (int u = 0; u < U; u++) xj[u] = jj[u] >= 0 ? fx[jj[u]] : make_uint4(0, 0, 0, 0);
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (base + 32 * u >= e) break;   // warp-uniform
-                    const int j = jj[u];
-                    bool ok_up = false, ok_lo = false;
-                    if (j >= 0 && j != i) {
-                        bool in;
-                        float r2f = 0.0f;
-                        if (periodic) {
-                            const float dx = fixed_delta(xi.x, xj[u].x, lp.Ls[0], lp.Ll[0]);
-                            const float dy = fixed_delta(xi.y, xj[u].y, lp.Ls[1], lp.Ll[1]);
-                            const float dz = fixed_delta(xi.z, xj[u].z, lp.Ls[2], lp.Ll[2]);
-                            r2f = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        }
-                        if (periodic && r2f < lp.lo2) in = true;
-                        else if (periodic && r2f > lp.hi2) in = false;
-                        else {
-                            double4_32a pj = pq[j];
-                            in = ref64_dist2(pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, pbc) <= lp.cutnb2;
-                        }
-                        if (in && !(fi && frozen[j])) {
-                            int a = min(i, j), bb = max(i, j);
-                            if (!stored_excluded(a, bb, xs, xd, lp.maxspan)) {
-                                ok_up = j > i;
-                                ok_lo = j < i;
-                            }
-                        }
-                    }
-                    unsigned bu = __ballot_sync(0xffffffffu, ok_up);
-                    unsigned bl = __ballot_sync(0xffffffffu, ok_lo);
-                    unsigned lt = (1u << lane) - 1u;
-                    if (ok_up) {
-                        int p = up + __popc(bu & lt);
-                        if (p + lo < lp.cap) row[p] = j;
-                    }
-                    if (ok_lo) {
-                        int p = lo + __popc(bl & lt);
-                        if (up + p < lp.cap) row[lp.cap - 1 - p] = j;
-                    }
-                    up += __popc(bu);
-                    lo += __popc(bl);
-                }
-            }
-        };
-        // the stencil's rows of cells along x (at most 5 x 5), one per lane: rows and end cells out
-        // of reach are dropped, and each row becomes one or two contiguous ranges of cell_atoms
+        // the stencil's rows of cells along x (at most 5 x 5), one per lane, z outer and y inner: each
+        // becomes one or two ranges of candidates, the wrapped part of a row first
         const int ny = dhi[1] - dlo[1] + 1, nrow = ny * (dhi[2] - dlo[2] + 1);
         int rb0 = 0, re0 = 0, rb1 = 0, re1 = 0;
-        bool keep = false;
         if (lane < nrow) {
             const int dy = dlo[1] + lane % ny, dz = dlo[2] + lane / ny;
             const float left = lp.reach2 - gap2(2, dz) - gap2(1, dy);
             if (left >= 0.f) {
-                keep = true;
                 int x0 = dlo[0], x1 = dhi[0];
                 while (x0 < 0 && gap2(0, x0) > left) x0++;
                 while (x1 > 0 && gap2(0, x1) > left) x1--;
                 int y = ctr[1] + dy, z = ctr[2] + dz;
-                if (g.periodic) { y = (y + g.nc[1]) % g.nc[1]; z = (z + g.nc[2]) % g.nc[2]; }
+                if (PERIODIC) { y = (y + g.nc[1]) % g.nc[1]; z = (z + g.nc[2]) % g.nc[2]; }
                 const int rowc = (z * g.nc[1] + y) * g.nc[0];
                 int a0 = ctr[0] + x0, a1 = ctr[0] + x1;   // both wrap only on a whole axis, which has none
                 if (a0 < 0) { rb1 = cell_start[rowc + a0 + g.nc[0]]; re1 = cell_start[rowc + g.nc[0]]; a0 = 0; }
@@ -317,20 +363,116 @@ __global__ void __launch_bounds__(256) k_build_rows(const double4_32a* __restric
                 re0 = cell_start[rowc + a1 + 1];
             }
         }
-        // rows in lane order (z outer, y inner), the wrapped part of a row first
-        for (unsigned km = __ballot_sync(0xffffffffu, keep); km; km &= km - 1) {
-            const int r = __ffs(km) - 1;
-            const int b1 = __shfl_sync(0xffffffffu, rb1, r), e1 = __shfl_sync(0xffffffffu, re1, r);
-            const int b0 = __shfl_sync(0xffffffffu, rb0, r), e0 = __shfl_sync(0xffffffffu, re0, r);
-            if (e1 > b1) scan(b1, e1);
-            scan(b0, e0);
+        // the non-empty ranges in order; a walk over them takes 32 candidates at a time, the end of one
+        // range together with the beginning of the next
+        const unsigned b1 = __ballot_sync(0xffffffffu, re1 > rb1), b0 = __ballot_sync(0xffffffffu, re0 > rb0);
+        const int nrange = __popc(b1) + __popc(b0);
+        __syncwarp();
+        if (re1 > rb1) range[__popc(b1 & below) + __popc(b0 & below)] = make_int2(rb1, re1);
+        if (re0 > rb0) range[__popc(b1 & (below << 1 | 1u)) + __popc(b0 & below)] = make_int2(rb0, re0);
+        if (lane < 2) range[nrange + lane] = make_int2(0, 0);
+        __syncwarp();
+        int rg = 0;
+        int2 cur = range[0], nxt = range[1];
+        auto fetch = [&]() -> uint4 {
+            const int rem = cur.y - cur.x;                       // at least 1 until the walk's end
+            const int at = lane < rem ? cur.x + lane : nxt.x + lane - rem;
+            const bool have = lane < rem || at < nxt.y;
+            if (rem > 32) {
+                cur.x += 32;
+            } else {
+                cur = make_int2(min(nxt.x + 32 - rem, nxt.y), nxt.y);
+                rg++;
+                nxt = rg + 1 < nrange ? range[rg + 1] : make_int2(0, 0);
+                if (cur.x == cur.y && rg < nrange) {             // the next range was used up whole
+                    cur = nxt;
+                    rg++;
+                    nxt = rg + 1 < nrange ? range[rg + 1] : make_int2(0, 0);
+                }
+            }
+            return have ? cell_pos[at] : make_uint4(0, 0, 0, 0xffffffffu);
+        };
+        bool more = rg < nrange;
+        uint4 next = fetch();
+        int head = 0, tail = 0;            // candidates within reach of the home atoms, pending in the ring
+        while (more || head != tail) {
+            if (more) {
+                const uint4 cd = next;
+                more = rg < nrange;
+                if (more) next = fetch();
+                bool near = cd.w != 0xffffffffu;
+                if (PERIODIC) {
+                    const float dx = __int2float_rn((int)(cd.x - ball[0])) * lp.Ls[0], dy = __int2float_rn((int)(cd.y - ball[1])) * lp.Ls[1],
+                                dz = __int2float_rn((int)(cd.z - ball[2])) * lp.Ls[2];
+                    near = near && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= ball2;
+                }
+                const unsigned b = __ballot_sync(0xffffffffu, near);
+                if (near) ring[(head + __popc(b & below)) & (ROW_RING - 1)] = cd;
+                head += __popc(b);
+                __syncwarp();
+                if (more && head - tail < 32) continue;
+            }
+            uint4 cd = make_uint4(0, 0, 0, 0xffffffffu);
+            if (lane < head - tail) cd = ring[(tail + lane) & (ROW_RING - 1)];
+            tail = min(tail + 32, head);
+            __syncwarp();
+            const int j = (int)cd.w;      // -1 past the end
+            // bit k: the candidate is in home atom k's row; close to it in index; in the band (one branch
+            // for all that have to be looked at)
+            unsigned in = 0, look = 0, band = 0;
+            if (PERIODIC) {
+                const float lo2 = j >= 0 ? lp.lo2 : -1.0f, hi2 = j >= 0 ? lp.hi2 : -1.0f;
+#pragma unroll
+                for (int k = 0; k < A; k++) {
+                    const float ux = __int2float_rn((int)(cd.x - hx[k][0])), uy = __int2float_rn((int)(cd.y - hx[k][1])),
+                                uz = __int2float_rn((int)(cd.z - hx[k][2]));
+                    float r2;
+                    if (ISO) {
+                        r2 = fmaf(ux, ux, fmaf(uy, uy, uz * uz));   // in units of (L 2^-32)^2, as lo2 and hi2
+                    } else {
+                        const float dx = ux * lp.Ls[0], dy = uy * lp.Ls[1], dz = uz * lp.Ls[2];
+                        r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    }
+                    if (r2 <= hi2) {
+                        in |= 1u << k;
+                        if (!(r2 < lo2)) band |= 1u << k;
+                        if ((unsigned)(j - hi[k] + span) <= 2u * (unsigned)span) look |= 1u << k;
+                    }
+                }
+            } else if (j >= 0) {
+                in = band = (1u << A) - 1u;
+            }
+            if (look | band) {
+                for (unsigned l = look | band; l; l &= l - 1) {
+                    const int k = __ffs(l) - 1;
+                    int i = hi[0];
+#pragma unroll
+                    for (int q = 1; q < A; q++) if (k == q) i = hi[q];
+                    if (!row_pair(pq, frozen, pbc, lp, xs, xd, i, j, band >> k & 1u)) in &= ~(1u << k);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < A; k++) {
+                const bool mine = in >> k & 1u, above = j > hi[k];
+                const unsigned b = __ballot_sync(0xffffffffu, mine), bu = __ballot_sync(0xffffffffu, mine && above);
+                const int rank = __popc((above ? bu : b ^ bu) & below), at = up[k] + rank;
+                // the front of the row grows up, its back down; a row that would pass its capacity is not stored
+                const int off = above ? at : back[k] - rank;
+                store_if(row[k] + off, j, mine && at <= back[k]);
+                up[k] += __popc(bu);
+                back[k] -= __popc(b ^ bu);
+            }
         }
-        if (lane == 0) {
-            nup[i] = up;
-            nlo[i] = lo;
-            atomicMax(max_row, up + lo);
-        }
+#pragma unroll
+        for (int k = 0; k < A; k++)
+            if (k < m) {
+                const int lo = lp.cap - 1 - back[k];
+                if (lane == 0) { nup[hi[k]] = up[k]; nlo[hi[k]] = lo; }
+                longest = max(longest, up[k] + lo);
+            }
     }
+    if (lane == 0 && longest > 0) atomicMax(max_row, longest);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1232,7 +1374,7 @@ SingleEngine::~SingleEngine() { release(); }
 void SingleEngine::release() {
     void* ptrs[] = {d_pq, d_es, d_es14, d_fx, d_esf, d_esf14, d_qf, d_prmf, d_frozen, d_xs, d_xd, d_fxs, d_fxd, d_p14, d_c14s,
                     d_c14d, d_bonds, d_ubs, d_angles, d_dihes, d_imprs, d_nbr, d_nup, d_nlo, d_cell_of,
-                    d_cell_count, d_cell_start, d_cell_fill, d_cell_atoms, d_part, d_ticket, d_maxrow,
+                    d_cell_count, d_cell_start, d_cell_fill, d_task_start, d_tasks, d_cell_atoms, d_cell_pos, d_home, d_part, d_ticket, d_maxrow,
                     d_stage, d_prn, d_pnup, d_pkept, d_cls_of, d_cls, d_x64, d_pair64};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (cudaEvent_t& e : ev_prune) if (e) { cudaEventDestroy(e); e = nullptr; }
@@ -1246,6 +1388,7 @@ void SingleEngine::release() {
 int SingleEngine::init(const HostSystem& h) {
     hs = h;
     n = hs.n;
+    any_frozen = std::any_of(hs.frozen.begin(), hs.frozen.end(), [](uint8_t f) { return f != 0; });
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     pbc.type = hs.pbc;
     for (int k = 0; k < 3; k++) { pbc.L[k] = hs.L[k]; pbc.rL[k] = hs.rL[k]; }
@@ -1797,15 +1940,24 @@ int SingleEngine::build_list() {
         for (int k = 0; k < 3; k++) g.nc[k] = std::max(1, g.nc[k] / 2);
     for (int k = 0; k < 3; k++) g.csf[k] = (float)(ext[k] / g.nc[k] * (1.0 - 1e-6));
     int ncell = g.nc[0] * g.nc[1] * g.nc[2];
+    const bool iso = g.periodic && hs.L[0] == hs.L[1] && hs.L[1] == hs.L[2];
+    // home atoms that share a walk: four share more of it, two leave fewer warps idle in a small system.  A
+    // whole update with two, four and eight: 50, 58, 59 us (864 argon atoms), 72, 84, 97 (1,800 water
+    // atoms), 170, 159, 174 (12,288), 359, 305, 338 (36,000), 948, 761, 753 (100,002), so the line is at 8,192
+    const int run = !g.periodic || n < 8192 ? 2 : 4;
     int rc;
     if (ncell > ncell_cap) {
-        if (d_cell_count) { cudaFree(d_cell_count); cudaFree(d_cell_start); cudaFree(d_cell_fill); }
-        if ((rc = dalloc(&d_cell_count, ncell)) || (rc = dalloc(&d_cell_start, ncell + 1)) || (rc = dalloc(&d_cell_fill, ncell)))
-            return rc;
+        int** const per_cell[] = {&d_cell_count, &d_cell_start, &d_cell_fill, &d_task_start};
+        for (int** p : per_cell) {
+            if (*p) cudaFree(*p);
+            if ((rc = dalloc(p, ncell + 1))) return rc;
+        }
+        if (d_tasks) cudaFree(d_tasks);
+        if ((rc = dalloc(&d_tasks, (size_t)n / 2 + ncell + 1))) return rc;
         ncell_cap = ncell;
     }
     if (!d_cell_of) {
-        if ((rc = dalloc(&d_cell_of, n)) || (rc = dalloc(&d_cell_atoms, n)) || (rc = dalloc(&d_nup, n)) || (rc = dalloc(&d_nlo, n)))
+        if ((rc = dalloc(&d_cell_of, n)) || (rc = dalloc(&d_cell_atoms, n)) || (rc = dalloc(&d_cell_pos, n)) || (rc = dalloc(&d_home, n)) || (rc = dalloc(&d_nup, n)) || (rc = dalloc(&d_nlo, n)))
             return rc;
     }
     if (cap == 0) {
@@ -1816,26 +1968,35 @@ int SingleEngine::build_list() {
         cap = (cap + 31) & ~31;
         if ((rc = dalloc(&d_nbr, (size_t)n * cap))) return rc;
     }
-    ListParams lp{rl * rl, cap, hs.maxExclSpan, {0, 0, 0}, {0, 0, 0}, 0.f, 0.f, 0.f};
+    ListParams lp{rl * rl, cap, hs.maxExclSpan, {0, 0, 0}, 0.f, 0.f, 0.f, any_frozen};
     {
+        // equal box lengths: r^2 stays in the mirrors' own units
         double t = hs.rc + hs.dcut;  // (cutoff + deltacut)^2 as List_nonBonded.cpp:842-843
         lp.cutnb2 = t * t;
         const AtomsDev A = atoms();
-        for (int k = 0; k < 3; k++) { lp.Ls[k] = A.Ls[k]; lp.Ll[k] = A.Lsl[k]; }
-        lp.lo2 = (float)(lp.cutnb2 * (1.0 - 1e-4));
-        lp.hi2 = (float)(lp.cutnb2 * (1.0 + 1e-4));
+        for (int k = 0; k < 3; k++) lp.Ls[k] = A.Ls[k];
+        const double unit2 = iso ? (hs.L[0] / 4294967296.0) * (hs.L[0] / 4294967296.0) : 1.0;
+        lp.lo2 = (float)(lp.cutnb2 * (1.0 - 1e-4) / unit2);
+        lp.hi2 = (float)(lp.cutnb2 * (1.0 + 1e-4) / unit2);
         lp.reach2 = (float)(lp.cutnb2 * (1.0 + 1e-5) + 1e-2);
     }
     for (int attempt = 0; attempt < 3; attempt++) {
         CK(cudaMemsetAsync(d_cell_count, 0, sizeof(int) * ncell, stream));
         CK(cudaMemsetAsync(d_maxrow, 0, sizeof(int), stream));
         k_cell_assign<<<(n + 255) / 256, 256, 0, stream>>>(d_pq, n, pbc, g, d_cell_of, d_cell_count);
-        k_cell_scan<<<1, 1024, 0, stream>>>(d_cell_count, ncell, d_cell_start, d_cell_fill);
+        k_cell_scan<<<1, 1024, 0, stream>>>(d_cell_count, ncell, run, d_cell_start, d_cell_fill, d_task_start);
         k_cell_scatter<<<(n + 255) / 256, 256, 0, stream>>>(d_cell_of, n, d_cell_start, d_cell_fill, d_cell_atoms);
-        k_cell_sort<<<ncell, 256, 0, stream>>>(d_cell_start, ncell, d_cell_atoms);
-        int blocks = std::min((n + 7) / 8, NB_BLOCKS * 2);
-        k_build_rows<<<blocks, 256, 0, stream>>>(d_pq, d_fx, d_frozen, n, pbc, g, lp, d_cell_of, d_cell_start, d_cell_atoms,
-                                                 d_xs, d_xd, d_nbr, d_nup, d_nlo, d_maxrow);
+        k_cell_sort<<<ncell, 128, 0, stream>>>(d_cell_start, d_task_start, ncell, run, d_fx, g, d_cell_atoms, d_cell_pos, d_home, d_tasks);
+        const int blocks = std::min((n / run + ncell + ROW_WARPS - 1) / ROW_WARPS, 152 * 16);
+#define MCG_ROWS(A_, P_, I_)                                                                                          \
+    k_build_rows<A_, P_, I_><<<blocks, 32 * ROW_WARPS, 0, stream>>>(d_pq, d_cell_pos, d_frozen, pbc, g, lp, d_cell_start, \
+                                                                d_task_start, ncell, d_home, d_tasks, d_xs, d_xd, d_nbr, d_nup, d_nlo, d_maxrow)
+        if (!g.periodic) MCG_ROWS(2, false, false);
+        else if (iso && run == 4) MCG_ROWS(4, true, true);
+        else if (iso) MCG_ROWS(2, true, true);
+        else if (run == 4) MCG_ROWS(4, true, false);
+        else MCG_ROWS(2, true, false);
+#undef MCG_ROWS
         CK(cudaGetLastError());
         int maxrow = 0;
         CK(cudaMemcpyAsync(&maxrow, d_maxrow, sizeof(int), cudaMemcpyDeviceToHost, stream));

@@ -125,6 +125,11 @@ private:
     TorsT *d_dihes = nullptr, *d_imprs = nullptr;
     int *d_nbr = nullptr, *d_nup = nullptr, *d_nlo = nullptr;
     int *d_cell_of = nullptr, *d_cell_count = nullptr, *d_cell_start = nullptr, *d_cell_fill = nullptr, *d_cell_atoms = nullptr;
+    int* d_task_start = nullptr;  // row-build tasks of each cell (home-atom runs), and the tasks (cell, first)
+    int2* d_tasks = nullptr;
+    int* d_home = nullptr;        // home atoms (places in cell order) grouped by octant of their cell
+    uint4* d_cell_pos = nullptr;  // candidates in cell order: fixed-point position, atom index
+    int any_frozen = 0;
     int ncell_cap = 0;
     double* d_part = nullptr;
     size_t part_cap = 0;

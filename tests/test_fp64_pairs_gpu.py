@@ -209,3 +209,20 @@ def test_batch_energy_of_residues_wider_than_at_creation():
     xyz[901] += [-9.0, 0.0, 2.0]
     B.set_coords(0, xyz)
     _check_chains(B, chains)
+
+
+# row-build tasks of 2 and 4 home atoms (4 from 8,192 atoms), cells with a few and many atoms, few cells
+# an axis (whole-axis stencils) and many, an orthorhombic box, and no box at all
+@pytest.mark.parametrize("kind,n", [("argon", 331), ("argon", 9001), ("water", 700), ("water", 2730), ("water", 2731), ("orbic", 5003),
+                                    ("vacuum", 3001)])
+def test_verlet_rows(kind, n):
+    s = systems.water_box(n, seed=n) if kind == "water" else _near(_charged_argon(n, n), 1)
+    if kind == "orbic":
+        s.pbc_type = "orbic"
+        s.box = (s.box[0], s.box[1] * 1.5, s.box[2] * 1.0625)
+    if kind == "vacuum":
+        s.pbc_type = "none"
+    s.frozen = (np.arange(s.natom) % 3 == 0).astype(np.uint8) if n % 2 else s.frozen
+    rows = FFieldCUDA(s, "fp64", moves=False).pairlist()
+    want = orc.Oracle(s, moves=False).verlet_rows()
+    assert all(np.array_equal(a, np.sort(b)) for a, b in zip(rows, want, strict=True))
