@@ -21,8 +21,10 @@ void set_error(const std::string& msg);
 int fail(int code, const std::string& msg);
 
 struct BondT { int a, b, type; double k, r0, beta; };
-struct AngleT { int a, b, c, type; double k, theta0; };
-struct TorsT { int a, b, c, d, type, order; double k, phi0, mult; };
+// cos0, sin0: of the reference angle, for the deviation's sine (NaN sends an angle the general way);
+// nmult: the multiplicity when it is an integer of 0..6, else -1 (term_constants sets the three)
+struct AngleT { int a, b, c, type; double k, theta0, cos0 = 0, sin0 = 0; };
+struct TorsT { int a, b, c, d, type, order; double k, phi0, mult, cos0 = 0, sin0 = 0; int nmult = -1; };
 
 // Host-side system model: AtomList + PerConditions + FField settings + topology, with the
 // reference's unit conversions applied (epsilon stored as sqrt(eps*418.4), k*418.4, radians).
@@ -51,6 +53,9 @@ struct HostSystem {
 
 // Builds a HostSystem from the ABI description (validates, converts units, builds exclusions).
 int build_host_system(const mcg_system_desc* d, HostSystem& hs);
+
+// The constants of the angle and torsion terms that only depend on their parameters.
+void term_constants(HostSystem& hs);
 
 // List_nonBonded::build_exclude_list (List_nonBonded.cpp:143-775) on the host.
 void build_exclusions(HostSystem& hs);

@@ -52,6 +52,7 @@ namespace mcg {
 
 constexpr int NB_BLOCKS = 152 * 4;   // grid of the list-driven kernels: 4 CTAs per SM
 constexpr int NB_THREADS = 256;
+constexpr int BD_BLOCKS = 152 * 2;   // largest grid of the bonded terms: their FP64 pipes are the bound
 constexpr int MAX_MOVED = 1024;
 constexpr int SORT_MAX = 2048;       // cells larger than this are sorted by one thread
 constexpr int CLS_MAX = 1024;        // parameter classes the mixed pair kernel keeps in shared memory
@@ -1006,33 +1007,44 @@ __device__ double bond_e(const BondT& b, const CrdSrc& S, const PbcDev& pbc, boo
     return 0.5 * b.k * (d - b.r0) * (d - b.r0);
 }
 
-__device__ double angle_e(const AngleT& a, const CrdSrc& S, const PbcDev& pbc) {
+// The angle and torsion terms need an angle's deviation from its reference, or the cosine of a
+// multiple of it, and both follow from sines and cosines: the library's acos, atan2 and cos are
+// some 100 FP64 operations each, at 64 cycles of a scheduler's FP64 pipe per warp.  The general form
+// (out of line) stays for what the short one does not cover: an angle more than 2^-6 off its reference
+// or nearly straight, a multiplicity that is not an integer of 0 to 6, three atoms in line.  With two
+// CTAs per SM instead of 64 in all this took the bonded terms of 100,002 water atoms from 31 us (46
+// before the minimum image went to integer compares) to 12.
+
+// asin(s) for |s| <= 2^-6: the Taylor series to s^9 (the next term is below 2^-64 of s)
+__device__ __forceinline__ double asin_small(double s) {
+    const double z = s * s;
+    const double p = fma(z, fma(z, fma(z, 35.0 / 1152.0, 5.0 / 112.0), 3.0 / 40.0), 1.0 / 6.0);
+    return fma(s * z, p, s);
+}
+__device__ __forceinline__ bool below_abs(double v, unsigned hi) { return ((unsigned)__double2hiint(v) & 0x7fffffffu) < hi; }   // NaN: false
+constexpr unsigned HI_2M6 = 0x3f900000u;        // 2^-6
+constexpr unsigned HI_ALMOST1 = 0x3feff800u;    // 1 - 2^-10
+
+__device__ __noinline__ double angle_general(double dot, double r2ab, double r2bc, double theta0) {
+    return acos(dot / (sqrt(r2ab) * sqrt(r2bc))) - theta0;
+}
+
+__device__ __forceinline__ double angle_e(const AngleT& a, const CrdSrc& S, const PbcDev& pbc) {
     double di[3], dj[3], dk[3], dab[3], dbc[3];
     S.get(a.a, di); S.get(a.b, dj); S.get(a.c, dk);
-    double rab = sqrt(ref64_dist2(di[0], di[1], di[2], dj[0], dj[1], dj[2], pbc, dab));
-    double rbc = sqrt(ref64_dist2(dk[0], dk[1], dk[2], dj[0], dj[1], dj[2], pbc, dbc));
-    double cost = (dab[0] * dbc[0] + dab[1] * dbc[1] + dab[2] * dbc[2]) / (rab * rbc);
-    double th = acos(cost) - a.theta0;
+    const double r2ab = ref64_dist2(di[0], di[1], di[2], dj[0], dj[1], dj[2], pbc, dab);
+    const double r2bc = ref64_dist2(dk[0], dk[1], dk[2], dj[0], dj[1], dj[2], pbc, dbc);
+    const double dot = fma(dab[0], dbc[0], fma(dab[1], dbc[1], dab[2] * dbc[2]));
+    const double c = dot * rsqrt64(r2ab * r2bc);
+    const double u = fma(-c, c, 1.0);
+    // sin(theta - theta0); a small one is a small deviation, theta and theta0 both well inside (0, pi)
+    const double s = fma(u * rsqrt64(u), a.cos0, -(c * a.sin0));
+    const double th = below_abs(c, HI_ALMOST1) && below_abs(s, HI_2M6) ? asin_small(s) : angle_general(dot, r2ab, r2bc, a.theta0);
     return 0.5 * a.k * th * th;
 }
 
-__device__ double tors_e(const TorsT& t, const CrdSrc& S, const PbcDev& pbc) {
-    double di[3], dj[3], dk[3], dl[3], dab[3], dbc[3], dcd[3], pb[3], pc[3];
-    S.get(t.a, di); S.get(t.b, dj); S.get(t.c, dk); S.get(t.d, dl);
-    for (int k = 0; k < 3; k++) { dab[k] = di[k] - dj[k]; dcd[k] = dk[k] - dl[k]; }
-    apply_pbc(dab, pbc); apply_pbc(dcd, pbc);
-    double rbc = sqrt(ref64_dist2(dk[0], dk[1], dk[2], dj[0], dj[1], dj[2], pbc, dbc));
-    pb[0] = dab[1] * dbc[2] - dab[2] * dbc[1];
-    pb[1] = dab[2] * dbc[0] - dab[0] * dbc[2];
-    pb[2] = dab[0] * dbc[1] - dab[1] * dbc[0];
-    double rpb = sqrt(pb[0] * pb[0] + pb[1] * pb[1] + pb[2] * pb[2]);
-    pc[0] = dbc[1] * dcd[2] - dbc[2] * dcd[1];
-    pc[1] = dbc[2] * dcd[0] - dbc[0] * dcd[2];
-    pc[2] = dbc[0] * dcd[1] - dbc[1] * dcd[0];
-    double rpc = sqrt(pc[0] * pc[0] + pc[1] * pc[1] + pc[2] * pc[2]);
-    double cosp = (pb[0] * pc[0] + pb[1] * pc[1] + pb[2] * pc[2]) / (rpb * rpc);
-    double sinp = (dbc[0] * (pc[1] * pb[2] - pc[2] * pb[1]) + dbc[1] * (pb[0] * pc[2] - pb[2] * pc[0]) +
-                   dbc[2] * (pc[0] * pb[1] - pc[1] * pb[0])) / (rpb * rpc * rbc);
+// the deviation of a harmonic torsion, or the angle itself
+__device__ __noinline__ double tors_general(const TorsT& t, double sinp, double cosp) {
     double phi = atan2(sinp, cosp);
     if (t.type == 2) {
         phi = phi - t.phi0;
@@ -1040,6 +1052,46 @@ __device__ double tors_e(const TorsT& t, const CrdSrc& S, const PbcDev& pbc) {
         return 0.5 * t.k * phi * phi;
     }
     return t.k * (1. + cos(t.mult * phi - t.phi0));
+}
+
+__device__ __forceinline__ double tors_e(const TorsT& t, const CrdSrc& S, const PbcDev& pbc) {
+    double di[3], dj[3], dk[3], dl[3], dab[3], dbc[3], dcd[3], pb[3], pc[3];
+    S.get(t.a, di); S.get(t.b, dj); S.get(t.c, dk); S.get(t.d, dl);
+    for (int k = 0; k < 3; k++) { dab[k] = di[k] - dj[k]; dcd[k] = dk[k] - dl[k]; }
+    apply_pbc(dab, pbc); apply_pbc(dcd, pbc);
+    const double rbc = sqrt(ref64_dist2(dk[0], dk[1], dk[2], dj[0], dj[1], dj[2], pbc, dbc));
+    auto cross = [](const double* x, const double* y, double* z) {
+        z[0] = fma(x[1], y[2], -(x[2] * y[1]));
+        z[1] = fma(x[2], y[0], -(x[0] * y[2]));
+        z[2] = fma(x[0], y[1], -(x[1] * y[0]));
+    };
+    auto dot = [](const double* x, const double* y) { return fma(x[0], y[0], fma(x[1], y[1], x[2] * y[2])); };
+    double pcb[3];
+    cross(dab, dbc, pb);
+    cross(dbc, dcd, pc);
+    cross(pc, pb, pcb);
+    // sin phi and cos phi times |pb| |pc| |bc|
+    const double sn = dot(dbc, pcb), cn = dot(pb, pc) * rbc;
+    const double u = fma(sn, sn, cn * cn);
+    if (!((unsigned)__double2hiint(u) - 0x00100000u < 0x7fe00000u)) {   // three atoms in line, or not finite: the reference's quotients
+        const double q = sqrt(dot(pb, pb)) * sqrt(dot(pc, pc));
+        return tors_general(t, sn / (q * rbc), dot(pb, pc) / q);
+    }
+    const double inv = rsqrt64(u), s1 = sn * inv, c1 = cn * inv;
+    if (t.type == 2) {
+        const double s = fma(s1, t.cos0, -(c1 * t.sin0)), c = fma(c1, t.cos0, s1 * t.sin0);   // of phi - phi0
+        if (!(below_abs(s, HI_2M6) && __double2hiint(c) >= 0)) return tors_general(t, s1, c1);
+        const double d = asin_small(s);
+        return 0.5 * t.k * d * d;
+    }
+    if (t.nmult < 0) return tors_general(t, s1, c1);
+    double s = 0.0, c = 1.0;                            // of n phi, by the addition theorem
+    for (int n = 0; n < t.nmult; n++) {
+        const double cc = fma(c, c1, -(s * s1));
+        s = fma(s, c1, c * s1);
+        c = cc;
+    }
+    return t.k * (1.0 + fma(c, t.cos0, s * t.sin0));
 }
 
 // part layout: 5 doubles per block (bond, ang, ub, dihe, impr)
@@ -1062,7 +1114,8 @@ __global__ void k_bonded(BondedDev B, PbcDev pbc, const double4_32a* __restrict_
     __shared__ double sh[5][32];
     int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     for (int c = 0; c < 5; c++) {
-        double v = warp_sum(e[c]);
+        // a warp holds terms of one kind or two: the others' sums are zero without the five additions
+        double v = __any_sync(0xffffffffu, __double_as_longlong(e[c]) != 0) ? warp_sum(e[c]) : 0.0;
         if (l == 0) sh[c][w] = v;
     }
     __syncthreads();
@@ -1505,7 +1558,7 @@ int SingleEngine::init(const HostSystem& h) {
     // scratch: partial sums and the ΔE ticket
     ntile = (n + TILE - 1) / TILE;
     size_t nparts = std::max<size_t>({(size_t)152 * 8, (size_t)ntile * (ntile + 1) / 2, (size_t)MAX_MOVED + 1});
-    part_cap = nparts * 3 + 2 * 64 + 5 * 64 + 16;
+    part_cap = nparts * 3 + 2 * 64 + 5 * BD_BLOCKS + 16;
     if ((rc = dalloc(&d_part, part_cap)) || (rc = dalloc(&d_ticket, 1)) ||
         (rc = dalloc(&d_maxrow, 1)))
         return rc;
@@ -1702,7 +1755,7 @@ int SingleEngine::ensure_clusters() {
     const int crc = clp.build(stream, d_fx, n, hs.L, d_nbr, d_nup, d_nlo, cap);
     launches += clp.build_launches;
     clp.build_launches = 0;
-    if (crc == MCG_OK) return ensure_part((size_t)2 * clp.ncl + 2 * 64 + 5 * 64 + 16);
+    if (crc == MCG_OK) return ensure_part((size_t)2 * clp.ncl + 2 * 64 + 5 * BD_BLOCKS + 16);
     if (crc == MCG_ECUDA) return crc;
     set_error("");
     return MCG_OK;
@@ -2057,7 +2110,7 @@ int SingleEngine::energy(double ener[10]) {
     int nterm = B.nb + B.na + B.nu + B.nd + B.ni;
     int nbd = 0;
     if (nterm > 0) {
-        nbd = std::min(64, (nterm + 255) / 256);
+        nbd = std::min(BD_BLOCKS, (nterm + 255) / 256);
         k_bonded<<<nbd, 256, 0, stream>>>(B, pbc, d_pq, bd);
     }
     k_finalize<<<1, 256, 0, stream>>>(nbp, nnb, p14, n14b, bd, nbd, d_map + 8);

@@ -14,6 +14,21 @@ void set_error(const std::string& msg) { g_err = msg; }
 int fail(int code, const std::string& msg) { g_err = msg; return code; }
 const char* last_error_cstr() { return g_err.c_str(); }
 
+void term_constants(HostSystem& hs) {
+    for (AngleT& a : hs.angles) {
+        // nearly straight reference angles take the general way: the sine says little there
+        const bool fast = a.theta0 > 0.05 && a.theta0 < PI - 0.05;
+        a.cos0 = fast ? std::cos(a.theta0) : std::nan("");
+        a.sin0 = fast ? std::sin(a.theta0) : std::nan("");
+    }
+    for (std::vector<TorsT>* v : {&hs.dihes, &hs.imprs})
+        for (TorsT& t : *v) {
+            t.cos0 = std::cos(t.phi0);
+            t.sin0 = std::sin(t.phi0);
+            t.nmult = t.mult >= 0.0 && t.mult <= 6.0 && t.mult == std::floor(t.mult) ? (int)t.mult : -1;
+        }
+}
+
 int build_host_system(const mcg_system_desc* d, HostSystem& hs) {
     if (!d) return fail(MCG_EINVAL, "null system description");
     if (d->natom <= 0) return fail(MCG_EINVAL, "natom must be positive");
@@ -98,6 +113,7 @@ int build_host_system(const mcg_system_desc* d, HostSystem& hs) {
     rc = tors(d->nimpr, d->impr_atoms, d->impr_type, d->impr_order, d->impr_k, d->impr_phi0, d->impr_mult, hs.imprs);
     if (rc) return rc;
     build_exclusions(hs);
+    term_constants(hs);
     return MCG_OK;
 }
 

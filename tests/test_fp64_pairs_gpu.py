@@ -17,6 +17,7 @@ from mc_cpp_gb300.engine import BatchChains, FFieldCUDA
 
 pytestmark = pytest.mark.gpu
 REL = 1e-13
+KCAL = 418.4
 
 
 @pytest.fixture(scope="module", autouse=True)
@@ -226,3 +227,56 @@ def test_verlet_rows(kind, n):
     rows = FFieldCUDA(s, "fp64", moves=False).pairlist()
     want = orc.Oracle(s, moves=False).verlet_rows()
     assert all(np.array_equal(a, np.sort(b)) for a, b in zip(rows, want, strict=True))
+
+
+def _bonded_chain(n, seed, angles, torsion_kinds):
+    """n charged atoms in a chain whose angles and torsions take the given values (degrees), with terms
+    referred to other values: from no deviation to the whole circle."""
+    s = systems.argon_random(n, 0.005, seed)
+    rng = np.random.default_rng(seed)
+    xyz = [np.zeros(3), np.array([1.5, 0.0, 0.0])]
+    for i in range(2, n):
+        th, ph = np.radians(angles[i % len(angles)]), rng.uniform(-np.pi, np.pi)
+        u = xyz[-1] - xyz[-2]
+        u /= np.linalg.norm(u)
+        v = np.cross(u, [0.3, 0.5, 0.81])
+        v /= np.linalg.norm(v)
+        w = np.cross(u, v)
+        xyz.append(xyz[-1] + 1.5 * (-np.cos(th) * u + np.sin(th) * (np.cos(ph) * v + np.sin(ph) * w)))
+    s.set_coords(np.array(xyz))
+    s.pbc_type, s.cut_mode = "none", "full"
+    s.eps = np.zeros(n)
+    s.angles = np.stack([np.arange(n - 2), np.arange(1, n - 1), np.arange(2, n)], 1).astype(np.int32)
+    s.angle_type = np.zeros(n - 2, np.int32)
+    s.angle_k = np.full(n - 2, 55.0)
+    s.angle_theta0 = np.array([angles[i % len(angles)] + d for i, d in zip(range(2, n), np.tile([0.0, 1e-9, 0.3, 0.8, 0.95, 5.0, -40.0], n))])
+    d4 = np.stack([np.arange(n - 3), np.arange(1, n - 2), np.arange(2, n - 1), np.arange(3, n)], 1).astype(np.int32)
+    m = n - 3
+    s.dihedrals, s.dihe_type = d4, np.array([torsion_kinds[k % len(torsion_kinds)][0] for k in range(m)], np.int32)
+    s.dihe_mult = np.array([torsion_kinds[k % len(torsion_kinds)][1] for k in range(m)], np.float64)
+    s.dihe_order = np.maximum(1, s.dihe_mult).astype(np.int32)
+    s.dihe_k, s.dihe_phi0 = rng.uniform(0.1, 2.0, m), rng.uniform(-180, 180, m)
+    s.impropers, s.impr_type = d4.copy(), np.full(m, 2, np.int32)
+    s.impr_order, s.impr_mult, s.impr_k = np.ones(m, np.int32), np.ones(m), np.full(m, 20.0)
+    a, b, c, d = (s.coords()[d4[:, k]] for k in range(4))
+    n1, n2 = np.cross(a - b, b - c), np.cross(b - c, c - d)
+    phi = np.degrees(np.arctan2((np.cross(n2, n1) * (b - c)).sum(1) / np.linalg.norm(b - c, axis=1), (n1 * n2).sum(1)))
+    s.impr_phi0 = phi + np.tile([0.0, 1e-9, 0.5, 0.89, 0.91, 60.0, 180.0, 359.7], n)[:m]
+    return s
+
+
+# angles from a right one to nearly straight, multiplicities that are and are not small integers, harmonic
+# torsions from their reference value to half a turn off it
+@pytest.mark.parametrize("angles", [[90.0, 104.52, 111.0], [3.0, 30.0, 150.0], [176.0, 177.6, 179.9]])
+@pytest.mark.parametrize("kinds", [[(1, 1), (1, 2), (1, 3)], [(1, 0), (1, 6), (1, 7), (1, 2.5)], [(2, 1), (1, 1)]])
+def test_bonded_terms(angles, kinds):
+    s = _bonded_chain(60, 8, angles, kinds)
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    want = np.array(orc.Oracle(s, moves=False).energy())
+    # an angle or torsion near its ends magnifies a coordinate's rounding by 1 / sin(theta) and the torsion
+    # by that of both its angles; a term's error is that times its slope, k |deviation|
+    amp = 1.0 / np.sin(np.radians(min(min(angles), 180 - max(angles)))) ** 2
+    dev = 2.0 ** -49 * amp * 8
+    slope = KCAL * (55.0 * np.radians(45) + 2.0 * 7) * s.natom, KCAL * 20.0 * np.pi * s.natom
+    assert abs(got[6] - want[6]) <= dev * slope[0], (got, want)
+    assert abs(got[8] - want[8]) <= dev * (slope[0] + slope[1]) and abs(got[9] - want[9]) <= dev * slope[1], (got, want)
