@@ -1156,54 +1156,72 @@ __global__ void k_finalize(const double* __restrict__ nb, int nnb, const double*
 
 // ------------------------------------------------------------------------------------------
 // Energy change of a moved set.  Blocks b < m*S take moved atom mv[b / S] against slice b % S of
-// its partners (Verlet row in switch mode, every atom in full mode) and of its 1-4 partners; block
-// m*S evaluates the listed bonded terms.  Pairs with both atoms moved are counted once, by the
-// lower index.  Spreading a row over S blocks matters most in FP64, which GB300 runs at about two
-// lane operations per clock per SM: one block per moved atom left a water move's ~1,150 partners
-// on three SMs.  The last block to finish sums the partials (a fixed tree over the block index,
-// so de is reproducible) and writes de (iu).
+// its partners (Verlet row in switch mode, every atom in full mode) and of its 1-4 partners; the blocks
+// behind them take the listed bonded terms, a block per kind present.  Pairs with both atoms moved are
+// counted once, by the lower index.
+// Bound by latency: the longest chain of dependent FP64 operations (64 cycles each on GB300, whatever a
+// warp's active lanes) between the launch and the result.  So FP64 pairs take their old and new energy on
+// two lanes, rows spread until a thread has one such term, bonded kinds run on blocks of their own with
+// the old terms on one warp and the new ones on the other, and a thread's contributions become one number
+// before the sums across lanes, warps and blocks.  The last block to finish sums the partials (a fixed
+// order, so de is reproducible) and writes de (iu).
+// A water move took 18 us (FP64 or mixed) with both sides of a pair and of all bonded terms on one
+// thread, three sums per block and two more block sums at the end; 11 and 10 now.  A move of a chain atom
+// with its dihedrals took 46 to 73 us before this and the shorter bonded terms; 14 to 19 now.
+constexpr int DE_KINDS = 5;   // bonds, angles, Urey-Bradley, dihedrals, impropers
 struct MoveDev {
     int m;
     const int* idx;        // sorted moved atoms
     const double* xyz;     // their proposed coordinates (3 per atom)
-    const int* terms;      // bonded terms touching them: (kind, index) pairs
-    int nterms;
+    const int* terms;      // bonded terms touching them, kind after kind
+    int nkind;             // kinds present, each with the end of its terms
+    int kind[DE_KINDS], kend[DE_KINDS];
 };
 
 // A small proposal travels inside the launch (kernel parameter space, read through the constant
 // cache), so that a trial move costs one launch and no copy; m = 0 means it was staged in device
 // memory and MoveDev points there.
-constexpr int INL_M = 32, INL_T = 96;
+constexpr int INL_M = 32, INL_T = 192;
 struct MoveInline {
-    int m, nterms;
+    int m;
     int idx[INL_M];
-    int terms[2 * INL_T];
+    int terms[INL_T];
     double xyz[3 * INL_M];
 };
 
-template <int P>
-__global__ void __launch_bounds__(256) k_delta_e(AtomsDev A, int n, PbcDev pbc, CutDev cut, MoveDev mv,
+// sum over the block; thread 0 has it
+__device__ __forceinline__ double block_sum(double v, double* s) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) v += s[w];
+    return v;
+}
+
+// M: the moved atoms the shared arrays hold (a small proposal's block asks for little shared memory)
+template <int P, int M>
+__global__ void __launch_bounds__(256) k_delta_e(AtomsDev A, int n, PbcDev pbc, CutDev cut, const __grid_constant__ MoveDev mv,
                                                  const int* __restrict__ nbr, const int* __restrict__ nup,
                                                  const int* __restrict__ nlo, int cap,
                                                  const int* __restrict__ fxs, const int* __restrict__ fxd,
                                                  const int* __restrict__ c14s, const int* __restrict__ c14d,
                                                  BondedDev B, int S, double* part, unsigned* ticket, double* out,
                                                  const __grid_constant__ MoveInline inl) {
-    __shared__ int s_idx[MAX_MOVED];
-    __shared__ double s_xyz[3 * MAX_MOVED];
-    __shared__ uint4 s_fx[MAX_MOVED];
+    __shared__ int s_idx[M];
+    __shared__ double s_xyz[3 * M];
+    __shared__ uint4 s_fx[P == PREC_MIX ? M : 1];
+    __shared__ double s_sum[8];
     __shared__ bool s_last;
-    if (inl.m > 0) { mv.m = inl.m; mv.idx = inl.idx; mv.xyz = inl.xyz; mv.terms = inl.terms; mv.nterms = inl.nterms; }
+    const int* idx = inl.m > 0 ? inl.idx : mv.idx;
+    const double* xyz = inl.m > 0 ? inl.xyz : mv.xyz;
+    const int* terms = inl.m > 0 ? inl.terms : mv.terms;
     const int m = mv.m;
-    for (int k = threadIdx.x; k < m; k += blockDim.x) {
-        s_idx[k] = mv.idx[k];
-        double x = mv.xyz[3 * k], y = mv.xyz[3 * k + 1], z = mv.xyz[3 * k + 2];
-        s_xyz[3 * k] = x; s_xyz[3 * k + 1] = y; s_xyz[3 * k + 2] = z;
-        if (P == PREC_MIX) {
-            uint4 f = A.fx[mv.idx[k]];
-            if (pbc.type != 0) { f.x = to_fixed(x, pbc.rL[0]); f.y = to_fixed(y, pbc.rL[1]); f.z = to_fixed(z, pbc.rL[2]); }
-            s_fx[k] = f;
-        }
+    for (int k = threadIdx.x; k < m; k += blockDim.x) s_idx[k] = idx[k];
+    for (int k = threadIdx.x; k < 3 * m; k += blockDim.x) {
+        const double v = xyz[k];
+        s_xyz[k] = v;
+        if (P == PREC_MIX && pbc.type != 0) reinterpret_cast<uint32_t*>(s_fx + k / 3)[k % 3] = to_fixed(v, pbc.rL[k % 3]);
     }
     __syncthreads();
     auto slot = [&](int j) -> int {
@@ -1223,8 +1241,9 @@ __global__ void __launch_bounds__(256) k_delta_e(AtomsDev A, int n, PbcDev pbc, 
         const int a = s_idx[ka];
         const double4_32a ao = A.pq[a];
         const double4_32a an = make_double4_32a(s_xyz[3 * ka], s_xyz[3 * ka + 1], s_xyz[3 * ka + 2], ao.w);
-        const uint4 fo = P == PREC_MIX ? A.fx[a] : make_uint4(0, 0, 0, 0);
-        const uint4 fn = P == PREC_MIX ? s_fx[ka] : make_uint4(0, 0, 0, 0);
+        const uint4 f0 = make_uint4(0, 0, 0, 0);
+        const uint4 fo = P == PREC_MIX ? A.fx[a] : f0;
+        const uint4 fn = P == PREC_MIX ? s_fx[ka] : f0;
         CutDev cutx = cut;   // full mode: no cutoff and no switch
         if (!sw) { cutx.c2f = 1.0e30f; cutx.n2f = 1.0e30f; }   // "no cutoff": finite, so c2 - 3 n2 stays finite
         float ma[3] = {0.f, 0.f, 0.f};   // the exact move of a, as the fixed-point mirror sees it
@@ -1237,21 +1256,29 @@ __global__ void __launch_bounds__(256) k_delta_e(AtomsDev A, int n, PbcDev pbc, 
                 ma[0] = (float)(an.x - ao.x); ma[1] = (float)(an.y - ao.y); ma[2] = (float)(an.z - ao.z);
             }
         }
+        // FP64: the old (side 0, subtracted) or new energy of the pair
+        auto visit64 = [&](int j, bool fourteen, bool apply_cut, int side) {
+            const int sj = slot(j);
+            if (sj >= 0 && j < a) return;       // counted by the lower index's block
+            double4_32a pa = ao, pj = A.pq[j];
+            if (side) {
+                pa = an;
+                if (sj >= 0) { pj.x = s_xyz[3 * sj]; pj.y = s_xyz[3 * sj + 1]; pj.z = s_xyz[3 * sj + 2]; }
+            }
+            double e, v;
+            pair_energy<PREC_F64>(A, pbc, cut, fourteen, pa, f0, a, pj, f0, j, apply_cut, e, v);
+            del += side ? e : -e;
+            dvd += side ? v : -v;
+        };
         auto visit = [&](int j, bool fourteen, bool apply_cut) {
             int sj = slot(j);
             if (sj >= 0 && j < a) return;       // counted by the lower index's block
-            double4_32a jo = A.pq[j];
-            uint4 gjo = P == PREC_MIX ? A.fx[j] : make_uint4(0, 0, 0, 0);
+            double4_32a jo = pbc.type != 0 ? make_double4_32a(0, 0, 0, 0) : A.pq[j];
+            uint4 gjo = A.fx[j];
             double4_32a jn = jo;
             uint4 gjn = gjo;
-            if (sj >= 0) { jn.x = s_xyz[3 * sj]; jn.y = s_xyz[3 * sj + 1]; jn.z = s_xyz[3 * sj + 2]; if (P == PREC_MIX) gjn = s_fx[sj]; }
-            if (P == PREC_F64) {
-                double e0, v0, e1, v1;
-                pair_energy<P>(A, pbc, cut, fourteen, ao, fo, a, jo, gjo, j, apply_cut, e0, v0);
-                pair_energy<P>(A, pbc, cut, fourteen, an, fn, a, jn, gjn, j, apply_cut, e1, v1);
-                del += e1 - e0;
-                dvd += v1 - v0;
-            } else {
+            if (sj >= 0) { jn.x = s_xyz[3 * sj]; jn.y = s_xyz[3 * sj + 1]; jn.z = s_xyz[3 * sj + 2]; gjn = s_fx[sj]; }
+            {
                 // d_old = j_old - a_old, d_new = j_new - a_new = d_old - m
                 float d[3], m[3];
                 if (pbc.type != 0) {
@@ -1296,74 +1323,62 @@ __global__ void __launch_bounds__(256) k_delta_e(AtomsDev A, int n, PbcDev pbc, 
                 }
             }
         };
+        // partner k of a's 1-4 pairs, of its row, or of all atoms; FP64: k = 2 partner + side
+        constexpr int SIDES = P == PREC_F64 ? 2 : 1;
+        auto at = [&](int k, int j, bool fourteen) {
+            if (P == PREC_F64) visit64(j, fourteen, sw, k & 1);
+            else visit(j, fourteen, sw);
+        };
         if (sw) {
             const int* row = nbr + (size_t)a * cap;
-            int u = nup[a], l = nlo[a];
-            for (int k = k0; k < u + l; k += kstep) {
-                int j = k < u ? row[k] : row[cap - 1 - (k - u)];
-                visit(j, false, true);
+            const int u = nup[a], l = nlo[a];
+            for (int k = k0; k < SIDES * (u + l); k += kstep) {
+                const int t = k / SIDES;
+                at(k, t < u ? row[t] : row[cap - 1 - (t - u)], false);
             }
         } else {
-            for (int j = k0; j < n; j += kstep) {
+            for (int k = k0; k < SIDES * n; k += kstep) {
+                const int j = k / SIDES;
                 if (j == a) continue;
-                int lo_ = min(a, j), hi_ = max(a, j);
+                const int lo_ = min(a, j), hi_ = max(a, j);
                 bool ex = false;
-                for (int k = fxs[lo_]; k < fxs[lo_ + 1]; k++) if (fxd[k] == hi_) { ex = true; break; }
-                if (!ex) visit(j, false, false);
+                for (int x = fxs[lo_]; x < fxs[lo_ + 1]; x++) if (fxd[x] == hi_) { ex = true; break; }
+                if (!ex) at(k, j, false);
             }
         }
-        for (int k = c14s[a] + k0; k < c14s[a + 1]; k += kstep) visit(c14d[k], true, sw);
+        const int c0 = c14s[a], c1 = c14s[a + 1];
+        for (int k = k0; k < SIDES * (c1 - c0); k += kstep) at(k, c14d[c0 + k / SIDES], true);
+        dbd = fma(CHGCHARMM * KCALTOIU, del, fma(4.0, dvd, dbd));
     } else {
-        CrdSrc S_old{A.pq, nullptr, nullptr, 0};
-        CrdSrc S_new{A.pq, s_idx, s_xyz, m};
-        for (int k = threadIdx.x; k < mv.nterms; k += blockDim.x) {
-            int kind = mv.terms[2 * k], t = mv.terms[2 * k + 1];
-            double e0 = 0, e1 = 0;
-            if (kind == 0) { e0 = bond_e(B.bonds[t], S_old, pbc, true); e1 = bond_e(B.bonds[t], S_new, pbc, true); }
-            else if (kind == 1) { e0 = angle_e(B.angles[t], S_old, pbc); e1 = angle_e(B.angles[t], S_new, pbc); }
-            else if (kind == 2) { e0 = bond_e(B.ubs[t], S_old, pbc, false); e1 = bond_e(B.ubs[t], S_new, pbc, false); }
-            else if (kind == 3) { e0 = tors_e(B.dihes[t], S_old, pbc); e1 = tors_e(B.dihes[t], S_new, pbc); }
-            else { e0 = tors_e(B.imprs[t], S_old, pbc); e1 = tors_e(B.imprs[t], S_new, pbc); }
-            dbd += e1 - e0;
+        const int q = blockIdx.x - m * S, kind = mv.kind[q];
+        const int warp = threadIdx.x >> 5, side = warp & 1;
+        const CrdSrc src{A.pq, s_idx, s_xyz, side ? m : 0};
+        for (int k = (q ? mv.kend[q - 1] : 0) + 32 * (warp >> 1) + (threadIdx.x & 31); k < mv.kend[q]; k += blockDim.x / 2) {
+            const int t = terms[k];
+            double e;
+            if (kind == 0) e = bond_e(B.bonds[t], src, pbc, true);
+            else if (kind == 1) e = angle_e(B.angles[t], src, pbc);
+            else if (kind == 2) e = bond_e(B.ubs[t], src, pbc, false);
+            else if (kind == 3) e = tors_e(B.dihes[t], src, pbc);
+            else e = tors_e(B.imprs[t], src, pbc);
+            dbd += side ? e : -e;
         }
     }
-    __shared__ double red[3];
-    block_reduce2(del, dvd, red);
-    {
-        double v = warp_sum(dbd);
-        __shared__ double sb[32];
-        if ((threadIdx.x & 31) == 0) sb[threadIdx.x >> 5] = v;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += sb[k];
-            red[2] = s;
-        }
-        __syncthreads();
-    }
+    const double sum = block_sum(dbd, s_sum);
     if (threadIdx.x == 0) {
-        part[3 * blockIdx.x] = red[0];
-        part[3 * blockIdx.x + 1] = red[1];
-        part[3 * blockIdx.x + 2] = red[2];
+        part[blockIdx.x] = sum;
         __threadfence();
-        unsigned t = atomicAdd(ticket, 1u);
-        s_last = (t == gridDim.x - 1);
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (s_last) {   // uniform over the block
         __threadfence();
-        double se = 0.0, sv = 0.0, sb = 0.0;
-        for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-            se += __ldcg(part + 3 * b);
-            sv += __ldcg(part + 3 * b + 1);
-            sb += __ldcg(part + 3 * b + 2);
-        }
-        block_reduce2(se, sv, red);
-        __shared__ double rb[2];
-        block_reduce2(sb, 0.0, rb);
+        double v = 0.0;
+        for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) v += __ldcg(part + b);
+        __syncthreads();
+        v = block_sum(v, s_sum);
         if (threadIdx.x == 0) {
-            out[0] = CHGCHARMM * KCALTOIU * red[0] + 4.0 * red[1] + rb[0];
-            out[1] = red[0]; out[2] = red[1]; out[3] = rb[0];
+            out[0] = v;
             *ticket = 0u;
         }
     }
@@ -2169,10 +2184,11 @@ int SingleEngine::delta_e(int m, const int* atoms_in, const double* nx, const do
         idx[k] = a;
         xyz[3 * k] = px; xyz[3 * k + 1] = py; xyz[3 * k + 2] = pz;
     }
-    // bonded terms touching the moved set, each once
+    // bonded terms touching the moved set, each once, kind after kind
     stamp++;
     int nt = 0;
-    const size_t tcap = (stage_bytes - 64 - off_terms) / 8;   // the last 64 bytes take de back
+    const size_t tcap = (stage_bytes - 64 - off_terms) / 8;
+    for (std::vector<int>& v : term_kind) v.clear();
     for (int k = 0; k < m; k++) {
         int a = idx[k];
         for (int t = term_start[a]; t < term_start[a + 1]; t++) {
@@ -2181,43 +2197,53 @@ int SingleEngine::delta_e(int m, const int* atoms_in, const double* nx, const do
             if (gk >= term_seen.size()) term_seen.resize(gk + 1, 0);
             if (term_seen[gk] == stamp) continue;
             term_seen[gk] = stamp;
-            if ((size_t)nt >= tcap) return fail(MCG_ECAPACITY, "too many bonded terms in one move");
-            terms[2 * nt] = kind; terms[2 * nt + 1] = ti;
-            nt++;
+            if ((size_t)nt++ >= tcap) return fail(MCG_ECAPACITY, "too many bonded terms in one move");
+            term_kind[kind].push_back(ti);
         }
     }
-    MoveDev mv;
+    MoveDev mv{};
     mv.m = m;
     mv.idx = (const int*)d_stage;
     mv.xyz = (const double*)((char*)d_stage + off_xyz);
     mv.terms = (const int*)((char*)d_stage + off_terms);
-    mv.nterms = nt;
+    int* tend = terms;
+    for (int k = 0; k < DE_KINDS; k++) {
+        if (term_kind[k].empty()) continue;
+        tend = std::copy(term_kind[k].begin(), term_kind[k].end(), tend);
+        mv.kind[mv.nkind] = k;
+        mv.kend[mv.nkind++] = (int)(tend - terms);
+    }
     MoveInline inl;
-    inl.m = 0; inl.nterms = 0;
+    inl.m = 0;
     if (m <= INL_M && nt <= INL_T) {
-        inl.m = m; inl.nterms = nt;
+        inl.m = m;
         memcpy(inl.idx, idx, 4 * (size_t)m);
         memcpy(inl.xyz, xyz, 24 * (size_t)m);
-        memcpy(inl.terms, terms, 8 * (size_t)nt);
+        memcpy(inl.terms, terms, 4 * (size_t)nt);
     } else {
-        CK(cudaMemcpyAsync(d_stage, h_stage, off_terms + (size_t)nt * 8, cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(d_stage, h_stage, off_terms + (size_t)nt * 4, cudaMemcpyHostToDevice, stream));
     }
     AtomsDev A = atoms();
     BondedDev B = bonded();
-    // slices per moved atom: about one partner per thread for a Verlet row (64 threads), about
-    // four per thread over all atoms in full mode (256 threads), at most two blocks per SM in all
+    // slices per moved atom: about one partner (FP64: one side of one) per thread for a Verlet row (64
+    // threads), about four per thread over all atoms in full mode (256 threads), at most two blocks per SM in all
     const bool sw = hs.cut == MCG_CUT_SWITCH;
     const int threads = sw ? 64 : 256;
-    const int span = sw ? cap : n;
+    const int span = (sw ? cap : n) * (hs.prec == MCG_PREC_FP64 ? 2 : 1);
     int S = (span + (sw ? 64 : 1024) - 1) / (sw ? 64 : 1024);
     S = std::max(1, std::min(S, std::max(1, 304 / m)));
-    S = std::min(S, std::max(1, MAX_MOVED / m));   // m*S + 1 partials fit the scratch
-    if (hs.prec == MCG_PREC_FP64)
-        k_delta_e<PREC_F64><<<m * S + 1, threads, 0, stream>>>(A, n, pbc, cut, mv, d_nbr, d_nup, d_nlo, cap, d_fxs,
-                                                                d_fxd, d_c14s, d_c14d, B, S, d_part, d_ticket, d_map, inl);
-    else
-        k_delta_e<PREC_MIX><<<m * S + 1, threads, 0, stream>>>(A, n, pbc, cut, mv, d_nbr, d_nup, d_nlo, cap, d_fxs,
-                                                                d_fxd, d_c14s, d_c14d, B, S, d_part, d_ticket, d_map, inl);
+    S = std::min(S, std::max(1, MAX_MOVED / m));   // m*S + 5 partials fit the scratch
+#define MCG_DELTA(P_, M_)                                                                                             \
+    k_delta_e<P_, M_><<<m * S + mv.nkind, threads, 0, stream>>>(A, n, pbc, cut, mv, d_nbr, d_nup, d_nlo, cap, d_fxs,  \
+                                                                d_fxd, d_c14s, d_c14d, B, S, d_part, d_ticket, d_map, inl)
+    if (hs.prec == MCG_PREC_FP64) {
+        if (inl.m) MCG_DELTA(PREC_F64, INL_M);
+        else MCG_DELTA(PREC_F64, MAX_MOVED);
+    } else {
+        if (inl.m) MCG_DELTA(PREC_MIX, INL_M);
+        else MCG_DELTA(PREC_MIX, MAX_MOVED);
+    }
+#undef MCG_DELTA
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream));   // de lands in mapped host memory
     *de = ((volatile double*)h_map)[0];
@@ -2682,7 +2708,7 @@ int SingleEngine::commit() {
     const int* didx = (const int*)d_stage;
     const double* dxyz = (const double*)((char*)d_stage + pending_off_xyz);
     MoveInline inl;
-    inl.m = 0; inl.nterms = 0;
+    inl.m = 0;
     if (pending_inline) {
         inl.m = pending_m;
         memcpy(inl.idx, pending_idx.data(), 4 * (size_t)pending_m);

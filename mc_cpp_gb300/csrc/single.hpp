@@ -142,6 +142,7 @@ private:
     size_t stage_bytes = 0;
     std::vector<int> term_start, term_data;
     std::vector<unsigned> term_seen;
+    std::vector<int> term_kind[5];   // scratch: a proposal's bonded terms by kind
     unsigned stamp = 0;
     int pending_m = 0;
     bool pending_inline = false;

@@ -280,3 +280,27 @@ def test_bonded_terms(angles, kinds):
     slope = KCAL * (55.0 * np.radians(45) + 2.0 * 7) * s.natom, KCAL * 20.0 * np.pi * s.natom
     assert abs(got[6] - want[6]) <= dev * slope[0], (got, want)
     assert abs(got[8] - want[8]) <= dev * (slope[0] + slope[1]) and abs(got[9] - want[9]) <= dev * slope[1], (got, want)
+
+
+# proposals inside the launch (up to 32 atoms and 192 bonded terms) and staged beside it, one block per bonded
+# kind, every precision and cutoff; mixed precision to the engine's own 1e-4 kcal/mol per trial move of a
+# residue of three atoms, independent errors of more atoms adding in quadrature
+@pytest.mark.parametrize("prec,cut", [("fp64", "switch"), ("fp64", "full"), ("mixed", "switch")])
+@pytest.mark.parametrize("m", [1, 3, 31, 32, 33, 40, 200])
+def test_trial_moves(prec, cut, m):
+    s = systems.peptide_in_water(40, 700, L=30.0, seed=6)
+    s.cut_mode = cut
+    ff = FFieldCUDA(s, prec, moves=False)
+    o = orc.Oracle(s, moves=False)
+    e0 = np.array(o.energy())
+    rng = np.random.default_rng(m)
+    idx = np.sort(rng.choice(40 if m <= 40 else s.natom, m, replace=False))
+    new = s.coords()[idx] + rng.uniform(-0.02, 0.02, (m, 3))
+    de = ff.delta_e(idx, new)
+    xyz = s.coords()
+    xyz[idx] = new
+    o.set_coords(xyz)
+    want = np.array(o.energy())[0] - e0[0]
+    # the oracle's own difference of two totals carries both sums' rounding
+    tol = 1e-4 * KCAL * max(1.0, (m / 3) ** 0.5) if prec == "mixed" else 2 * REL * _scale(s)
+    assert abs(de - want) <= tol, (de, want, tol)
