@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(256, MINB) k_energy_cluster(const uint4* __res
     __shared__ uint2 s_m[8][32];
     __shared__ __align__(16) float4 s_j[8][2][16];
     __shared__ int s_chunk[2];
+    pair_kernel_begin();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned lbit = 1u << lane;
     const int islot = lane & 7, jsub = lane >> 3;

@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(GE_THREADS, MINB) k_energy_groups(const uint4*
                                                                     const int* __restrict__ glen, int gcap, GroupGeom Gm,
                                                                     double* part) {
     extern __shared__ float4 s_cls[];
+    pair_kernel_begin();
     for (int c = threadIdx.x; c < ncls; c += blockDim.x) s_cls[c] = cls[c];
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -441,6 +442,7 @@ __global__ void __launch_bounds__(NT, MINB) k_energy_groups_x2(const uint4* __re
                                                                const int2* __restrict__ grow, const int* __restrict__ glen,
                                                                int gcap, GroupGeom Gm, double* part) {
     extern __shared__ float4 s_cls[];
+    pair_kernel_begin();
     pk_load_classes(cls, ncls, s_cls);
     const float* s_qh = (const float*)(s_cls + ncls);
     const float *s_ql = s_qh + ncls, *s_ep = s_ql + ncls, *s_sg = s_ep + ncls;
@@ -495,6 +497,7 @@ __global__ void __launch_bounds__(NT, MINB) k_energy_groups_x2r(const uint4* __r
                                                                 const int2* __restrict__ grow, const int* __restrict__ glen,
                                                                 int gcap, GroupGeom Gm, double* part) {
     extern __shared__ float4 s_cls[];
+    pair_kernel_begin();
     pk_load_classes(cls, ncls, s_cls);
     const float* s_qh = (const float*)(s_cls + ncls);
     const float *s_ql = s_qh + ncls, *s_ep = s_ql + ncls, *s_sg = s_ep + ncls;

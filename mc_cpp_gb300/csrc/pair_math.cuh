@@ -148,6 +148,12 @@ struct F32Acc {
     __device__ __forceinline__ double value() const { return (double)s + (double)c; }
 };
 
+// The start of a pair kernel and the end of what follows it (k_energy_tail, launched as its programmatic
+// dependent): once every CTA of the pair kernel has begun, the follower's may begin too; it waits for
+// the pair kernel's end before it reads the partial sums.
+__device__ __forceinline__ void pair_kernel_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pair_kernel_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
