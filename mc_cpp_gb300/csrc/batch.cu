@@ -1127,21 +1127,23 @@ __global__ void __launch_bounds__(256) k_batch_energy64(const ChainDev* __restri
                     const int2 p = ring[at];
                     const int i = p.x >> 3, j = p.y >> 3;
                     const ulonglong4_32a a = Mc[i], b = Mc[j];
-                    const double4_32a t = reinterpret_cast<const double4_32a*>(tab)[(p.x & 7) * MAX_APR + (p.y & 7)];
+                    const ulonglong4_32a t = reinterpret_cast<const ulonglong4_32a*>(tab)[(p.x & 7) * MAX_APR + (p.y & 7)];
+                    const double qq = __longlong_as_double((long long)t.x), ee = __longlong_as_double((long long)t.y);
                     const unsigned long long dx = b.x - a.x << G.sh, dy = b.y - a.y << G.sh, dz = b.z - a.z << G.sh;
                     const Fix64Dist u = G.iso ? fix64_dist2<true>(G, dx, dy, dz) : fix64_dist2<false>(G, dx, dy, dz);
                     double ys, w, ws;
-                    if (fix64_terms(G, u, sw, ys, w, ws)) {
-                        sel = fma(t.x, ys, sel);
-                        svd = fma(fma(t.z, w, -t.y), ws, svd);
+                    if (fix64_terms(G, u, sw, t.z, (int)t.w, ys, w, ws)) {
+                        sel = fma(qq, ys, sel);
+                        svd = fma(ee, fma(w, ws, -ws), svd);
                     } else {
-                        // closer than the 64-bit form reaches: the same products on an FP64 distance
+                        // closer than the 64-bit form reaches: the same terms on an FP64 distance
                         const double ex = (double)(long long)(b.x - a.x) * (C.L[0] * (1.0 / TWO64)),
                                      ey = (double)(long long)(b.y - a.y) * (C.L[1] * (1.0 / TWO64)),
                                      ez = (double)(long long)(b.z - a.z) * (C.L[2] * (1.0 / TWO64));
-                        const double y = rsqrt64(ex * ex + ey * ey + ez * ez) * G.leff, y2 = y * y, y6 = y2 * y2 * y2;
-                        sel = fma(t.x, y, sel);
-                        svd = fma(fma(t.z, y6, -t.y), y6, svd);
+                        const double y = rsqrt64(ex * ex + ey * ey + ez * ez) * G.leff;
+                        const double x2 = (t.z ? fix64_norm_to_double(t.z, (int)t.w - 64) : 0.0) * (y * y), x6 = x2 * x2 * x2;
+                        sel = fma(qq, y, sel);
+                        svd = fma(ee, fma(x6, x6, -x6), svd);
                     }
                 }
                 if (sw) tail1 = min(tail1 + 32, head1);
@@ -1151,7 +1153,7 @@ __global__ void __launch_bounds__(256) k_batch_energy64(const ChainDev* __restri
         }
         if (flush) break;
     }
-    double s = CHGCHARMM * KCALTOIU * sel + 4.0 * svd;
+    double s = CHGCHARMM * KCALTOIU * (sel / G.leff) + 4.0 * svd;
     s = warp_sum(s);
     __shared__ double sh[8];
     if (lane == 0) sh[wib] = s;

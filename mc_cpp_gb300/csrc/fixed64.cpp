@@ -54,8 +54,9 @@ Fix64Geom fix64_geom(const double L[3], double rc, double ron) {
 
 Fix64Pair fix64_pair(double qi, double ei, double si, double qj, double ej, double sj, double leff) {
     const long double s = ((long double)si + (long double)sj) / (long double)leff;
-    const long double s6 = s * s * s * s * s * s, c6 = (long double)ei * (long double)ej * s6;
-    return Fix64Pair{(double)((long double)qi * (long double)qj / (long double)leff), (double)c6, (double)(c6 * s6), 0.0};
+    int es = 0;
+    const long double f = std::frexp(s * s, &es);   // in [1/2, 1)
+    return Fix64Pair{qi * qj, ei * ej, clamp64(f * TWO64L), es};
 }
 
 }  // namespace mcg

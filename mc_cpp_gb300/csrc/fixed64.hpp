@@ -29,10 +29,13 @@ Fix64Geom fix64_geom(const double L[3], double rc, double ron);
 // Geometry of any pair of a box, without a cutoff: halved (iso: equal box lengths).
 Fix64Geom fix64_geom_full(const double L[3]);
 
-// One pair of parameter classes: el += qq / r, vd += (c12 / r^6 - c6) / r^6 with lengths in Leff
-// (qq = qi qj / Leff, c6 = ei ej (si + sj)^6 / Leff^6, c12 = c6 (si + sj)^6 / Leff^6).
+// One pair of parameter classes: el += qq Leff / r, vd += ee (w^2 - w) with w = (s / r)^6, s = si + sj.
+// el comes out times Leff: a total's Coulomb sums over class pairs cancel a hundredfold, so the products
+// are rounded as the reference rounds them, and the length's unit is taken out of the sum.
 struct alignas(32) Fix64Pair {
-    double qq, c6, c12, pad;
+    double qq, ee;       // qi qj, ei ej
+    uint64_t ms;         // s^2 = ms 2^(es - 64) Leff^2, ms of at least 2^63 (0 for s = 0)
+    int64_t es;
 };
 Fix64Pair fix64_pair(double qi, double ei, double si, double qj, double ej, double sj, double leff);
 

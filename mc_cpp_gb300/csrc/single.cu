@@ -57,7 +57,7 @@ constexpr int MAX_MOVED = 1024;
 constexpr int SORT_MAX = 2048;       // cells larger than this are sorted by one thread
 constexpr int CLS_MAX = 1024;        // parameter classes the mixed pair kernel keeps in shared memory
 // parameter classes whose pairs the FP64 kernel's table holds: 512 KB of products at 128, which stay in
-// L2 with a few rows of the matrix in L1; a system of more classes forms them per pair (9 FP64 operations)
+// L2 with a few rows of the matrix in L1; a system of more classes forms them per pair (5 FP64 operations)
 constexpr int CLS64_MAX = 128;
 
 enum { PREC_F64 = 0, PREC_MIX = 1 };
@@ -558,20 +558,23 @@ __global__ void __launch_bounds__(NB_THREADS) k_energy_list(AtomsDev A, int n, P
     block_reduce2(sel, svd, part + 2 * blockIdx.x);
 }
 
-// The pair's parameter products with lengths in Leff: from the table of class pairs, or formed here
-// for a system of more than CLS64_MAX distinct parameter sets.
+// The pair's parameters (Fix64Pair): from the table of class pairs, or formed here for a system of more
+// than CLS64_MAX distinct parameter sets.
 template <bool TABLE>
 __device__ __forceinline__ void pair64_params(const AtomsDev& A, double ileff, int i, int j, int ci, int cj, double& qq,
-                                              double& c6, double& c12) {
+                                              double& ee, unsigned long long& ms, int& es) {
     if (TABLE) {
-        const double4_32a p = reinterpret_cast<const double4_32a*>(A.pair64)[ci * A.ncls64 + cj];
-        qq = p.x; c6 = p.y; c12 = p.z;
+        const ulonglong4_32a p = reinterpret_cast<const ulonglong4_32a*>(A.pair64)[ci * A.ncls64 + cj];
+        qq = __longlong_as_double((long long)p.x);
+        ee = __longlong_as_double((long long)p.y);
+        ms = p.z;
+        es = (int)p.w;
     } else {
         const double2 a = A.es[i], b = A.es[j];
-        const double s = (a.y + b.y) * ileff, s2 = s * s, s6 = s2 * s2 * s2;
-        qq = A.pq[i].w * A.pq[j].w * ileff;
-        c6 = a.x * b.x * s6;
-        c12 = c6 * s6;
+        const double s = (a.y + b.y) * ileff;
+        qq = A.pq[i].w * A.pq[j].w;
+        ee = a.x * b.x;
+        fix64_mantissa(s * s, ms, es);
     }
 }
 
@@ -655,17 +658,18 @@ __global__ void __launch_bounds__(NB_THREADS) k_energy_list64(AtomsDev A, Fix64G
                 const int2 p = ring[at];
                 const ulonglong4_32a a = A.x64[p.x], b = A.x64[p.y];
                 const Fix64Dist u = fix64_dist2<ISO>(G, a, b);
-                double ys, w, ws;
-                if (fix64_terms(G, u, sw, ys, w, ws)) {
-                    double qq, c6, c12;
-                    pair64_params<TABLE>(A, ileff, p.x, p.y, (int)a.w, (int)b.w, qq, c6, c12);
+                double ys, w, ws, qq, ee;
+                unsigned long long ms;
+                int es;
+                pair64_params<TABLE>(A, ileff, p.x, p.y, (int)a.w, (int)b.w, qq, ee, ms, es);
+                if (fix64_terms(G, u, sw, ms, es, ys, w, ws)) {
                     sel = fma(qq, ys, sel);
-                    svd = fma(fma(c12, w, -c6), ws, svd);
+                    svd = fma(ee, fma(w, ws, -ws), svd);
                 } else {
                     double el, vd;
                     const uint4 f0 = make_uint4(0, 0, 0, 0);
                     pair_energy<PREC_F64>(A, pbc, cut, false, A.pq[p.x], f0, p.x, A.pq[p.y], f0, p.y, true, el, vd);
-                    sel += el;
+                    sel = fma(el, G.leff, sel);
                     svd += vd;
                 }
             }
@@ -675,7 +679,7 @@ __global__ void __launch_bounds__(NB_THREADS) k_energy_list64(AtomsDev A, Fix64G
         if (last) break;
         __syncwarp();
     }
-    block_reduce2(sel, svd, part + 2 * blockIdx.x);
+    block_reduce2(sel * ileff, svd, part + 2 * blockIdx.x);
 }
 
 // One batch of U entries per lane of row i: the pair terms of k_energy_list_mix.
@@ -938,22 +942,23 @@ __global__ void __launch_bounds__(A64_I) k_energy_all64(AtomsDev A, Fix64Geom G,
             }
             const ulonglong4_32a bj = sx[j - jb];
             const Fix64Dist u = fix64_dist2<ISO, true>(G, a, bj);
-            double ys, w, ws;
-            if (fix64_terms(G, u, false, ys, w, ws)) {
-                double qq, c6, c12;
-                pair64_params<TABLE>(A, ileff, i, j, (int)a.w, (int)bj.w, qq, c6, c12);
+            double ys, w, ws, qq, ee;
+            unsigned long long ms;
+            int es;
+            pair64_params<TABLE>(A, ileff, i, j, (int)a.w, (int)bj.w, qq, ee, ms, es);
+            if (fix64_terms(G, u, false, ms, es, ys, w, ws)) {
                 sel = fma(qq, ys, sel);
-                svd = fma(fma(c12, w, -c6), ws, svd);
+                svd = fma(ee, fma(w, ws, -ws), svd);
             } else {
                 double el, vd;
                 const uint4 f0 = make_uint4(0, 0, 0, 0);
                 pair_energy<PREC_F64>(A, pbc, cut, false, A.pq[i], f0, i, A.pq[j], f0, j, false, el, vd);
-                sel += el;
+                sel = fma(el, G.leff, sel);
                 svd += vd;
             }
         }
     }
-    block_reduce2(sel, svd, part + 2 * blockIdx.x);
+    block_reduce2(sel * ileff, svd, part + 2 * blockIdx.x);
 }
 
 // ---- bonded terms (FP64, device math library) ---------------------------------------------

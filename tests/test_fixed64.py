@@ -1,8 +1,8 @@
 """The 64-bit integer pair terms (csrc/fixed64.cuh) restated in Python integers, against exact rationals.
 
 The bounds are the roundings of each form: Y keeps units of 2^-59 of 1 and the iteration's remainder
-(5/2 d^3 for a seed within d = 2^-22), w = Y^6 truncates up to 3 units of 2^-60 (twice), 2^-58 and 2^-56,
-and the switch keeps 2^-57 of itself beside what two units of the squared distance do to it.
+(5/2 d^3 for a seed within d = 2^-22), w = (s Y)^6 truncates one unit of 2^-60 twice before it is cubed
+and up to 3 units of it twice after, and the switch keeps 2^-57 of itself beside what two units of the squared distance do to it.
 """
 import math
 import random
@@ -41,7 +41,7 @@ def dist2(d):
     return H >> 32, H & 0xFFFFFFFF, (s1 << 1) & 0xFFFFFFFF
 
 
-def terms(uh, um, ul, seed_error):
+def terms(uh, um, ul, seed_error, ms):
     e2 = (32 - uh.bit_length()) & ~1
     m = ((uh << 64 | um << 32 | ul) >> (32 - e2)) & M64
     f = np.float32(np.float32(1) / np.sqrt(np.float32(m >> 32)) * np.float32(1 + seed_error))
@@ -51,11 +51,14 @@ def terms(uh, um, ul, seed_error):
     assert -(1 << 31) <= es < (1 << 31)
     c = e + ((3 * ((es * es) >> 42)) >> 2)
     Y = (y0 << 32) + ((y0 * (c >> 32) + ((y0 * (c & 0xFFFFFFFF)) >> 32)) << 3)
-    w1 = hi(Y, Y) << 1
-    w2 = hi(w1, w1)
-    w3 = hi(w1, w2 << 1)
-    assert 1 << 55 <= w3 < 1 << 63 and (1 << 62) - (1 << 8) <= Y <= (1 << 63) + (1 << 8)
-    return Y, w3, e2
+    w1 = (Y * Y) >> 64 << 1
+    x = (w1 * ms) >> 64
+    assert 1 << 59 <= x < 1 << 63 and (1 << 62) - (1 << 8) <= Y <= (1 << 63) + (1 << 8)
+    lx = 63 - x.bit_length()
+    x <<= lx
+    x6 = hi(x, hi(x, x) << 2)
+    assert 1 << 59 <= x6 < 1 << 63
+    return Y, x6, e2, lx
 
 
 def test_inverse_powers():
@@ -70,17 +73,18 @@ def test_inverse_powers():
         uu = dist2(d)
         if 32 - uu[0].bit_length() > 29:
             continue
-        Y, w3, e2 = terms(*uu, rng.choice([-1, 1]) * 2.0 ** -22)
+        ms = rng.choice([1 << 63, M64, rng.randrange(1 << 63, 1 << 64)])      # s^2 = ms 2^-64
+        Y, x6, e2, lx = terms(*uu, rng.choice([-1, 1]) * 2.0 ** -22, ms)
         y = Fr(Y, 1 << 62) * (1 << (e2 // 2))
         worst_y = max(worst_y, abs(float(y * y * u - 1)) / 2)
-        worst_w = max(worst_w, abs(float(Fr(w3, 1 << 56) * (1 << (3 * e2)) * u ** 3 - 1)))
-    assert worst_y < 2.0 ** -57 and worst_w < 2.0 ** -53.5, (math.log2(worst_y), math.log2(worst_w))
+        worst_w = max(worst_w, abs(float(Fr(x6, 1 << 57) * Fr(1 << (3 * e2), 1 << (3 * lx)) * u ** 3 / Fr(ms, 1 << 64) ** 3 - 1)))
+    assert worst_y < 2.0 ** -57 and worst_w < 2.0 ** -55.5, (math.log2(worst_y), math.log2(worst_w))
 
 
 @pytest.mark.parametrize("m", [1 << 62, (1 << 62) + 1, (1 << 63) - 1, 1 << 63, M64])
 def test_mantissa_ends(m):
     for s in (-1, 0, 1):
-        Y, _, e2 = terms(m >> 32, m & 0xFFFFFFFF, 0, s * 2.0 ** -22)
+        Y, _, e2, _ = terms(m >> 32, m & 0xFFFFFFFF, 0, s * 2.0 ** -22, 1 << 63)
         assert e2 == 0 and abs(float(Fr(Y, 1 << 62) ** 2 * Fr(m, 1 << 64) - 1)) < 2.0 ** -56.5
 
 
