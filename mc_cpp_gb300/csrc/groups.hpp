@@ -60,6 +60,7 @@ private:
     void release();
     int *d_gstart = nullptr;     // first atom of each group (ngroup + 1)
     int *d_gof = nullptr;        // group of each atom
+    int *d_gslot = nullptr;      // 4 group + place in it, of each atom
     int2* d_grow = nullptr;      // group rows: (first atom of the partner group, mask | (size - 1) << 16)
     int* d_glen = nullptr;       // entries per group row
     unsigned long long* d_misc = nullptr;   // [0] entries, [1] mask bits, [2] overflow flag
