@@ -2332,11 +2332,24 @@ __device__ __forceinline__ double rp_canonical(const uint32_t* __restrict__ w, l
     return r >= 1.0 ? 0.99999999999999988898 : r;                       // nextafter(1, 0)
 }
 
-// Tools::rint wrap of one coordinate (PerConditions::applyPBC, PerConditions.cpp:244-285)
-__device__ __forceinline__ double rp_wrap(double v, double L, double rL) {
-    const double t = __dmul_rn(rL, v);
-    const double r = (double)(t >= 0.0 ? __double2int_rz(__dadd_rn(t, 0.5)) : __double2int_rz(__dsub_rn(t, 0.5)));
-    return __dsub_rn(v, __dmul_rn(L, r));
+// Energy of one pair (iu), the FP64 terms of ref64_pair with the factors of the total folded in: qa, ea are
+// the moved atom's charge and eps times K and 4, sw the switch's 1 / (rc^2 - ron^2)^3, 3 ron^2 - rc^2 and
+// bounds.  Comparisons of non-negative doubles are comparisons of their bits, on the integer pipe.
+__device__ __forceinline__ double rp_pair(double4_32a a, double4_32a b, double2 ea, double2 eb, double qa, const PbcDev& pbc,
+                                          const CutDev& cut, double k3s, double sw2s) {
+    const double dx = ref64_mic(__dsub_rn(b.x, a.x), pbc.L[0], pbc.rL[0]), dy = ref64_mic(__dsub_rn(b.y, a.y), pbc.L[1], pbc.rL[1]),
+                 dz = ref64_mic(__dsub_rn(b.z, a.z), pbc.L[2], pbc.rL[2]);
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const long long u = __double_as_longlong(r2);
+    if (u > __double_as_longlong(cut.c2)) return 0.0;
+    const double rt = rsqrt64(r2);
+    const double x = (ea.y + eb.y) * rt, x2 = x * x, x6 = x2 * x2 * x2;
+    double e = fma(ea.x * eb.x, fma(x6, x6, -x6), qa * b.w * rt);
+    if (u > __double_as_longlong(cut.n2)) {
+        const double s1 = cut.c2 - r2;
+        e *= s1 * s1 * fma(sw2s, r2, k3s);
+    }
+    return e;
 }
 
 // One thread-block cluster of RP_CL CTAs of RP_NT threads runs the steps.  On GB300 a warp's FP64
@@ -2346,9 +2359,15 @@ __device__ __forceinline__ double rp_wrap(double v, double L, double rL) {
 //    by the lanes of warp 0 in one pass, and the first accepted try is picked by ballot;
 //  - the dE terms are spread one per thread over the cluster's schedulers (CTAs first, then warps,
 //    then lanes), the old and the new energy of a pair on different threads;
-//  - each CTA's partial sums go to every CTA's shared memory, so every CTA sums them in rank order
-//    and takes the same decision; CTA 0 commits, and a cluster barrier orders the commit before
-//    the next step's reads.
+//  - each warp's sum goes to every CTA's shared memory at once, and behind the step's one cluster
+//    barrier every CTA adds the cluster's 32 sums by the same shuffles and takes the same decision;
+//  - every CTA commits the move itself (the same values to the same places), so its next reads need no
+//    barrier across the cluster.  A CTA can be at most at the next step's barrier while another still
+//    commits, and reads positions only before that barrier; the exchanged sums alternate between two
+//    buffers for the same reason.  The fixed-point mirrors, which only list builds read, follow before
+//    those (k_fix_all);
+//  - the decision compares in FP32 unless the draw is within 1e-4 of the threshold (an FP64 exp is some
+//    twenty dependent FP64 operations).
 // The launch's random words, and the move-instance tables when they fit, are copied into each
 // CTA's shared memory first: the proposal's loads are then shared-memory loads, not L2 round trips.
 // While the four warps of a CTA take the dE terms, a fifth forms the next step's uniforms: the next
@@ -2360,12 +2379,15 @@ __device__ __forceinline__ double rp_wrap(double v, double L, double rL) {
 // Measured on the 864-atom argon box (moves per second, host work included): 49.8k with one
 // 256-thread CTA (its ~200 dE terms at two warps per scheduler), 89.9k with the cluster and the
 // words read from global memory, 94.8k with them in shared memory, 99.9k with the fifth warp.
+// In runs of 500 steps, 92k so far, 107k with the FP64 operations of ref64_mic and rsqrt64, 141k with one
+// barrier and one sum a step.
 constexpr int RP_CL = 8;
 constexpr int RP_NT = 128;
 constexpr int RP_TRIES = 8;
 constexpr int RP_SPEC = 32;            // a fifth warp: the next step's uniforms, formed during this step's dE
 constexpr int RP_WORDS = 8192;        // random words of one launch, staged in each CTA's shared memory
 constexpr int RP_TAB = 3072;          // ints of the instance tables staged with them when they fit
+static_assert(RP_CL * RP_NT / 32 == 32, "the decision adds the cluster's warp sums as one warp");
 
 __device__ __forceinline__ double rp_canonical_at(const uint32_t* __restrict__ w, long long at) {
     long long cur = at;
@@ -2373,7 +2395,7 @@ __device__ __forceinline__ double rp_canonical_at(const uint32_t* __restrict__ w
 }
 
 __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
-    k_replay(AtomsDev A, double4_32a* pq, uint4* fx, PbcDev pbc, CutDev cut, const int* __restrict__ nbr,
+    k_replay(AtomsDev A, double4_32a* pq, PbcDev pbc, CutDev cut, const int* __restrict__ nbr,
              const int* __restrict__ nup, const int* __restrict__ nlo, int cap, const int* __restrict__ c14s,
              const int* __restrict__ c14d, ReplayTables T, const uint32_t* __restrict__ words, long long nwords,
              ReplayState* st, int s0, int s1, double beta) {
@@ -2385,8 +2407,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
     __shared__ double s_r[3];
     __shared__ int s_m, s_type, s_stop, s_acc;
     __shared__ long long s_cur;
-    __shared__ double s_part[2][RP_NT / 32];
-    __shared__ double2 s_cl[RP_CL];
+    __shared__ double s_cl[2][RP_CL * RP_NT / 32];   // every warp's sum, of this step and the other
     __shared__ __align__(16) uint32_t s_words[RP_WORDS];
     __shared__ int s_tab[RP_TAB];
     // the next step's uniforms, both cases (0: no acceptance draw in this step, 1: one)
@@ -2403,6 +2424,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
         for (int i = tid; i < 2 * T.nranges; i += blockDim.x) s_tab[T.ninst_all + i] = T.ranges[i];
     }
     if (tid == 0) s_sok = 0;
+    const double k3s = (cut.c2 - 3.0 * cut.n2) * cut.sw2, sw2s = 2.0 * cut.sw2;
     const int* inst_first = tab_sh ? s_tab : T.inst_first;
     const int* ranges = tab_sh ? s_tab + T.ninst_all : T.ranges;
     const int rank = (int)cluster.block_rank();
@@ -2494,7 +2516,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
                     const int k = i / 3, c = i - 3 * k;
                     const double4_32a p = pq[s_idx[k]];
                     const double pc = c == 0 ? p.x : (c == 1 ? p.y : p.z);
-                    s_xyz[i] = rp_wrap(__dadd_rn(pc, s_r[c]), pbc.L[c], pbc.rL[c]);
+                    s_xyz[i] = ref64_mic(__dadd_rn(pc, s_r[c]), pbc.L[c], pbc.rL[c]);   // PerConditions::applyPBC
                 }
         }
         __syncthreads();
@@ -2536,8 +2558,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
             }
             return -1;
         };
-        double del = 0.0, dvd = 0.0;
-        const uint4 f0 = make_uint4(0, 0, 0, 0);
+        double val = 0.0;
         int base = 0;
         for (int k = 0; k < m && warp < NW; k++) {
             const int a = s_idx[k];
@@ -2546,77 +2567,71 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
             const int cnt = u + l + n14;
             int q = (gslot - 2 * base) % G;
             if (q < 0) q += G;
-            for (; q < 2 * cnt; q += G) {
-                const int t = q >> 1, side = q & 1;
-                const bool fourteen = t >= u + l;
-                const int j = fourteen ? c14d[c14s[a] + t - u - l] : (t < u ? row[t] : row[cap - 1 - (t - u)]);
-                const int sj = slot(j);
-                if (sj >= 0 && j < a) continue;   // a pair of moved atoms, counted at its lower atom
-                double4_32a ai = pq[a], jj = pq[j];
-                if (side) {
-                    ai.x = s_xyz[3 * k]; ai.y = s_xyz[3 * k + 1]; ai.z = s_xyz[3 * k + 2];
-                    if (sj >= 0) { jj.x = s_xyz[3 * sj]; jj.y = s_xyz[3 * sj + 1]; jj.z = s_xyz[3 * sj + 2]; }
+            if (q < 2 * cnt) {
+                const double4_32a po = pq[a], pn = make_double4_32a(s_xyz[3 * k], s_xyz[3 * k + 1], s_xyz[3 * k + 2], po.w);
+                const double qa = CHGCHARMM * KCALTOIU * po.w;
+                for (; q < 2 * cnt; q += G) {
+                    const int t = q >> 1, side = q & 1;
+                    const bool fourteen = t >= u + l;
+                    const int j = fourteen ? c14d[c14s[a] + t - u - l] : (t < u ? row[t] : row[cap - 1 - (t - u)]);
+                    const int sj = slot(j);
+                    if (sj >= 0 && j < a) continue;   // a pair of moved atoms, counted at its lower atom
+                    double4_32a jj = pq[j];
+                    if (side && sj >= 0) { jj.x = s_xyz[3 * sj]; jj.y = s_xyz[3 * sj + 1]; jj.z = s_xyz[3 * sj + 2]; }
+                    double2 ea = fourteen ? A.es14[a] : A.es[a];
+                    const double2 eb = fourteen ? A.es14[j] : A.es[j];
+                    ea.x *= 4.0;
+                    const double e = rp_pair(side ? pn : po, jj, ea, eb, qa, pbc, cut, k3s, sw2s);
+                    val += side ? e : -e;
                 }
-                double e, v;
-                pair_energy<PREC_F64>(A, pbc, cut, fourteen, ai, f0, a, jj, f0, j, true, e, v);
-                del += side ? e : -e;
-                dvd += side ? v : -v;
             }
             base += cnt;
         }
-        del = warp_sum(del);
-        dvd = warp_sum(dvd);
-        if (lane == 0 && warp < NW) { s_part[0][warp] = del; s_part[1][warp] = dvd; }
-        __syncthreads();
-        if (tid == 0) {
-            double se = 0.0, sv = 0.0;
-            for (int w = 0; w < NW; w++) { se += s_part[0][w]; sv += s_part[1][w]; }
-            for (int r = 0; r < RP_CL; r++) *cluster.map_shared_rank(&s_cl[rank], r) = make_double2(se, sv);
+        double* cl = s_cl[step & 1];
+        if (warp < NW) {
+            val = warp_sum(val);
+            if (lane < RP_CL) *cluster.map_shared_rank(cl + rank * NW + warp, lane) = val;
         }
         cluster.sync();
-        if (tid == 0) {
-            double se = 0.0, sv = 0.0;
-            for (int r = 0; r < RP_CL; r++) { se += s_cl[r].x; sv += s_cl[r].y; }
-            const double de = CHGCHARMM * KCALTOIU * se + 4.0 * sv;
-            // MC_metropolis::apply_criterion (MC_metropolis.cpp:175-204); exp is CUDA's (at most 1 ulp
-            // from the exact value) where the host loop calls glibc's: the two runs can part only on a
-            // uniform within an ulp of the threshold
-            long long cur = s_cur;
-            bool accepted;
-            if (de <= 2.220446049250313e-16) accepted = true;
-            else accepted = rp_canonical(s_words, cur) < exp(-beta * de);
-            S.cursor = cur;
-            const int t = s_type;
-            if (accepted) {
-                S.acc_tmp[t]++;
-                S.etot += de;
-                S.acc++;
-            }
-            for (int tt = 0; tt < T.nmvtyp; tt++) {
-                if (T.each[tt] != 0 && (step % T.each[tt]) == 0) {
-                    const double ratio = (double)S.acc_tmp[tt] / (double)T.each[tt];
-                    S.dmax[tt] = ratio > T.target[tt] / 100 ? S.dmax[tt] * 1.10 : S.dmax[tt] * 0.9;
-                    S.acc_tmp[tt] = 0;
+        if (warp == 0) {
+            const double de = warp_sum(cl[lane]);
+            if (lane == 0) {
+                // MC_metropolis::apply_criterion (MC_metropolis.cpp:175-204); exp is CUDA's (at most 1 ulp
+                // from the exact value) where the host loop calls glibc's: the two runs can part only on a
+                // uniform within an ulp of the threshold
+                long long cur = s_cur;
+                bool accepted;
+                if (de <= 2.220446049250313e-16) accepted = true;
+                else {
+                    const double alpha = rp_canonical(s_words, cur);
+                    const float af = (float)alpha, ef = __expf((float)(-beta * de));   // off by less than 1e-5
+                    accepted = fabsf(af - ef) > 1e-4f ? af < ef : alpha < exp(-beta * de);
                 }
+                S.cursor = cur;
+                const int t = s_type;
+                if (accepted) {
+                    S.acc_tmp[t]++;
+                    S.etot += de;
+                    S.acc++;
+                }
+                for (int tt = 0; tt < T.nmvtyp; tt++) {
+                    if (T.each[tt] != 0 && (step % T.each[tt]) == 0) {
+                        const double ratio = (double)S.acc_tmp[tt] / (double)T.each[tt];
+                        S.dmax[tt] = ratio > T.target[tt] / 100 ? S.dmax[tt] * 1.10 : S.dmax[tt] * 0.9;
+                        S.acc_tmp[tt] = 0;
+                    }
+                }
+                S.steps_done = step;
+                s_acc = accepted ? 1 : 0;
             }
-            S.steps_done = step;
-            s_acc = accepted ? 1 : 0;
         }
         __syncthreads();
-        if (s_acc && rank == 0) {
-            for (int k = tid; k < m; k += blockDim.x) {
-                const int a = s_idx[k];
-                double4_32a p = pq[a];
-                p.x = s_xyz[3 * k]; p.y = s_xyz[3 * k + 1]; p.z = s_xyz[3 * k + 2];
-                pq[a] = p;
-                uint4 f = fx[a];
-                f.x = to_fixed(p.x, pbc.rL[0]); f.y = to_fixed(p.y, pbc.rL[1]); f.z = to_fixed(p.z, pbc.rL[2]);
-                fx[a] = f;
-            }
-            __threadfence();
+        if (s_acc) {
+            for (int i = tid; i < 3 * m; i += blockDim.x) reinterpret_cast<double*>(pq + s_idx[i / 3])[i % 3] = s_xyz[i];
+            __syncthreads();   // the commit before the next step's proposal
         }
-        cluster.sync();   // the commit before the next step's reads; every CTA is past this step's sums
     }
+    cluster.sync();   // no CTA leaves while another may still write into its shared memory
     if (tid == 0 && rank == 0) *st = S;
 }
 
@@ -2661,7 +2676,7 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
     ReplayState* d_st = nullptr;
     int rc = MCG_OK;
     auto done = [&](int r) {
-        // the run keeps pq and fx current; the 64-bit mirror, which it does not read, follows here
+        // the run keeps pq current; the mirrors, which it does not read, follow here
         k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
         launches++;
         if (cudaStreamSynchronize(stream) != cudaSuccess && r == MCG_OK) r = fail(MCG_ECUDA, "device run: mirrors");
@@ -2699,7 +2714,7 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
         if (cudaMemcpyAsync(d_words, w.data(), sizeof(uint32_t) * (size_t)W, cudaMemcpyHostToDevice, stream) != cudaSuccess ||
             cudaMemcpyAsync(d_st, &S, sizeof S, cudaMemcpyHostToDevice, stream) != cudaSuccess)
             return done(fail(MCG_ECUDA, "device run: upload"));
-        k_replay<<<RP_CL, RP_NT + RP_SPEC, 0, stream>>>(atoms(), d_pq, d_fx, pbc, cut, d_nbr, d_nup, d_nlo, cap, d_c14s, d_c14d, T,
+        k_replay<<<RP_CL, RP_NT + RP_SPEC, 0, stream>>>(atoms(), d_pq, pbc, cut, d_nbr, d_nup, d_nlo, cap, d_c14s, d_c14d, T,
                                               d_words, W, d_st, step, s1, beta);
         launches++;
         // while the launch runs: the next W words of the generator, in order, for the next buffer
@@ -2713,6 +2728,8 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
         if (S.status == 2) return done(fail(MCG_ENOTSUP, "device run: a move of more than 64 atoms"));
         step = S.steps_done;
         if (S.status == 0 && step % 50 == 0) {
+            k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
+            launches++;
             if ((rc = update_lists())) return done(rc);
         }
     }
