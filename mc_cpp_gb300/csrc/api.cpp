@@ -116,11 +116,20 @@ int mcg_energy_host(mcg_system* s, const double* x, const double* y, const doubl
     int rc;
     if (I.valid) {
         I.diff.clear();
-        for (int i = 0; i < n; i++)
-            if (!(x[i] == E.host_x[i] && y[i] == E.host_y[i] && z[i] == E.host_z[i])) {
-                I.diff.push_back(i);
-                if ((int)I.diff.size() > 1024) break;
-            }
+        // blocks that are the same byte for byte have no atom that differs
+        constexpr int BLOCK = 512;
+        for (int i0 = 0; i0 < n && (int)I.diff.size() <= 1024; i0 += BLOCK) {
+            const int i1 = std::min(n, i0 + BLOCK);
+            const size_t bytes = sizeof(double) * (size_t)(i1 - i0);
+            if (!std::memcmp(x + i0, E.host_x + i0, bytes) && !std::memcmp(y + i0, E.host_y + i0, bytes) &&
+                !std::memcmp(z + i0, E.host_z + i0, bytes))
+                continue;
+            for (int i = i0; i < i1; i++)
+                if (!(x[i] == E.host_x[i] && y[i] == E.host_y[i] && z[i] == E.host_z[i])) {
+                    I.diff.push_back(i);
+                    if ((int)I.diff.size() > 1024) break;
+                }
+        }
         const int m = (int)I.diff.size();
         if (m == 0) {
             *etot = I.e_base;
@@ -361,9 +370,9 @@ static int metropolis_impl(mcg_system* s, int nsteps, uint64_t seed, int accepta
     }
     std::vector<int> atoms;
     std::vector<double> nx, ny, nz;
-    std::vector<double>& X = E.host_x;
-    std::vector<double>& Y = E.host_y;
-    std::vector<double>& Z = E.host_z;
+    double* const X = E.host_x;
+    double* const Y = E.host_y;
+    double* const Z = E.host_z;
     auto wrap = [&](double& v, int k) {
         if (h.pbc != MCG_PBC_NONE) {
             double t = h.rL[k] * v;

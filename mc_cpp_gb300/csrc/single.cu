@@ -1429,18 +1429,32 @@ __global__ void k_commit(int m, const int* idx, const double* xyz, double4_32a* 
     }
 }
 
-// Fixed-point mirrors of every atom from the FP64 masters; w carries the atom's parameter class.
-__global__ void k_fix_all(int n, const double4_32a* __restrict__ pq, const int* __restrict__ cls_of, uint4* fx,
-                          ulonglong4_32a* x64, int sh, PbcDev pbc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double4_32a p = pq[i];
+// Fixed-point mirrors of an atom from its FP64 master; w carries the atom's parameter class.
+__device__ __forceinline__ void store_mirrors(int i, const double4_32a& p, unsigned cls, uint4* fx, ulonglong4_32a* x64, int sh,
+                                              const PbcDev& pbc) {
     uint4 f;
     if (pbc.type != 0) { f.x = to_fixed(p.x, pbc.rL[0]); f.y = to_fixed(p.y, pbc.rL[1]); f.z = to_fixed(p.z, pbc.rL[2]); }
     else { f.x = f.y = f.z = 0; }
-    f.w = (unsigned)cls_of[i];
+    f.w = cls;
     fx[i] = f;
-    if (x64) store_x64(x64 + i, p, pbc, sh, f.w);
+    if (x64) store_x64(x64 + i, p, pbc, sh, cls);
+}
+
+__global__ void k_fix_all(int n, const double4_32a* __restrict__ pq, const int* __restrict__ cls_of, uint4* fx,
+                          ulonglong4_32a* x64, int sh, PbcDev pbc) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) store_mirrors(i, pq[i], (unsigned)cls_of[i], fx, x64, sh, pbc);
+}
+
+// New coordinates of every atom, x, y and z after one another in page-locked host memory (read once,
+// coalesced, over the host link): the masters and their mirrors.
+__global__ void k_take_coords(int n, const double* __restrict__ xyz, double4_32a* pq, const int* __restrict__ cls_of, uint4* fx,
+                              ulonglong4_32a* x64, int sh, PbcDev pbc) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double4_32a p = make_double4_32a(xyz[i], xyz[n + i], xyz[2 * (size_t)n + i], pq[i].w);
+    pq[i] = p;
+    store_mirrors(i, p, (unsigned)cls_of[i], fx, x64, sh, pbc);
 }
 
 // ==========================================================================================
@@ -1472,6 +1486,7 @@ void SingleEngine::release() {
     for (void* p : ptrs) if (p) cudaFree(p);
     for (cudaEvent_t& e : ev_prune) if (e) { cudaEventDestroy(e); e = nullptr; }
     if (h_stage) cudaFreeHost(h_stage);
+    host_x = host_y = host_z = nullptr;   // inside h_stage
     if (h_map) cudaFreeHost(h_map);
     h_map = nullptr; d_map = nullptr;
     if (stream) cudaStreamDestroy(stream);
@@ -1605,14 +1620,19 @@ int SingleEngine::init(const HostSystem& h) {
     CK(cudaMemsetAsync(d_ticket, 0, 2 * sizeof(unsigned), stream));
     // staging for moves: idx (sorted), xyz, terms
     stage_bytes = (size_t)MAX_MOVED * (4 + 24) + 64 * 1024 * 8;
-    CK(cudaMallocHost(&h_stage, stage_bytes));
+    CK(cudaMallocHost(&h_stage, stage_bytes + sizeof(double) * 3 * (size_t)n));
+    host_x = (double*)((char*)h_stage + stage_bytes);
+    host_y = host_x + n;
+    host_z = host_y + n;
+    std::copy(hs.x.begin(), hs.x.end(), host_x);
+    std::copy(hs.y.begin(), hs.y.end(), host_y);
+    std::copy(hs.z.begin(), hs.z.end(), host_z);
     // results the host reads after a sync: de at [0, 4), the ten energy terms at [8, 18)
     CK(cudaHostAlloc((void**)&h_map, 32 * sizeof(double), cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer((void**)&d_map, h_map, 0));
     if ((rc = dalloc((char**)&d_stage, stage_bytes))) return rc;
     k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
     CK(cudaGetLastError());
-    host_x = hs.x; host_y = hs.y; host_z = hs.z;
     if (hs.cut == MCG_CUT_SWITCH) {
         if ((rc = build_list())) return rc;
     }
@@ -1850,9 +1870,9 @@ int SingleEngine::ensure_pruned() {
                                                        rp2, d_nbr, d_nup, cap, d_prn, d_pnup, d_pkept);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ev_prune[1], stream));
-    prune_x = host_x;
-    prune_y = host_y;
-    prune_z = host_z;
+    prune_x.assign(host_x, host_x + n);
+    prune_y.assign(host_y, host_y + n);
+    prune_z.assign(host_z, host_z + n);
     const double lim = std::max(0.0, 0.5 * prune_buf - 1e-3);
     prune_lim2 = lim * lim;
     prune_dirty = false;
@@ -2021,8 +2041,8 @@ int SingleEngine::build_list() {
         for (int k = 0; k < 3; k++) { ext[k] = hs.L[k]; g.lo[k] = 0; g.inv[k] = 0; }
     } else {
         for (int k = 0; k < 3; k++) {
-            const std::vector<double>& c = k == 0 ? host_x : (k == 1 ? host_y : host_z);
-            double lo = *std::min_element(c.begin(), c.end()), hi = *std::max_element(c.begin(), c.end());
+            const double* c = k == 0 ? host_x : (k == 1 ? host_y : host_z);
+            double lo = *std::min_element(c, c + n), hi = *std::max_element(c, c + n);
             ext[k] = std::max(hi - lo, 1e-6);
             g.lo[k] = lo;
             g.inv[k] = 1.0 / ext[k] * (1.0 - 1e-12);
@@ -2164,18 +2184,50 @@ int SingleEngine::energy(double ener[10]) {
     return MCG_OK;
 }
 
-int SingleEngine::set_coords(const double* x, const double* y, const double* z) {
-    std::vector<double4_32a> pq(n);
+// Whether v[0 .. n) holds an infinity or NaN: an exponent of all ones carries into the sign bit.
+static bool any_nonfinite(const double* v, int n) {
+    uint64_t carry = 0;
     for (int i = 0; i < n; i++) {
-        if (!std::isfinite(x[i]) || !std::isfinite(y[i]) || !std::isfinite(z[i]))
-            return fail(MCG_EINVAL, "non-finite coordinate at atom " + std::to_string(i));
-        pq[i] = make_double4_32a(x[i], y[i], z[i], hs.q[i]);
-        host_x[i] = x[i]; host_y[i] = y[i]; host_z[i] = z[i];
+        uint64_t b;
+        memcpy(&b, v + i, sizeof b);
+        carry |= (b & 0x7ff0000000000000ull) + 0x0010000000000000ull;
     }
-    if (!prune_dirty)
-        for (int i = 0; i < n && !prune_dirty; i++) note_moved(i);
-    CK(cudaMemcpyAsync(d_pq, pq.data(), sizeof(double4_32a) * n, cudaMemcpyHostToDevice, stream));
-    k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
+    return carry >> 63;
+}
+
+// The coordinates go into the page-locked mirror and are taken from there by one kernel.  One core's
+// passes over memory are the bound (about 25 GB/s each), so the blocks are checked, copied and compared
+// with the last prune's positions while they are in cache, in loops that vectorise (before: interleaved
+// with the charges in a fresh vector, copied from pageable memory, the mirror beside it; 100,002 atoms
+// 328 -> SET_NEW us).
+int SingleEngine::set_coords(const double* x, const double* y, const double* z) {
+    for (int i0 = 0; i0 < n; i0 += 1024) {
+        const int m = std::min(n - i0, 1024);
+        const double *bx = x + i0, *by = y + i0, *bz = z + i0;
+        if (any_nonfinite(bx, m) || any_nonfinite(by, m) || any_nonfinite(bz, m)) {
+            int i = i0;
+            while (std::isfinite(x[i]) && std::isfinite(y[i]) && std::isfinite(z[i])) i++;
+            const int rc = get_coords(host_x, host_y, host_z);   // the device still has what the mirror held
+            return rc ? rc : fail(MCG_EINVAL, "non-finite coordinate at atom " + std::to_string(i));
+        }
+        memcpy(host_x + i0, bx, sizeof(double) * m);
+        memcpy(host_y + i0, by, sizeof(double) * m);
+        memcpy(host_z + i0, bz, sizeof(double) * m);
+        if (prune_dirty) continue;
+        // a plain displacement within the limit is a wrapped one within it: only other blocks are looked
+        // at.  The squares are not negative, so one above the limit borrows into the sign bit.
+        const double *px = prune_x.data() + i0, *py = prune_y.data() + i0, *pz = prune_z.data() + i0;
+        uint64_t lim, far = 0;
+        memcpy(&lim, &prune_lim2, sizeof lim);
+        for (int i = 0; i < m; i++) {
+            const double dx = bx[i] - px[i], dy = by[i] - py[i], dz = bz[i] - pz[i], d2 = dx * dx + dy * dy + dz * dz;
+            uint64_t u;
+            memcpy(&u, &d2, sizeof u);
+            far |= lim - u;
+        }
+        for (int i = 0; far >> 63 && i < m && !prune_dirty; i++) note_moved(i0 + i);
+    }
+    k_take_coords<<<(n + 255) / 256, 256, 0, stream>>>(n, host_x, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream));
     return MCG_OK;

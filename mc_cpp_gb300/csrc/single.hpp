@@ -61,7 +61,8 @@ public:
     HostSystem hs;
     int n = 0;
     // host mirror of the coordinates (the device copy is the master once moves are committed)
-    std::vector<double> host_x, host_y, host_z;
+    // (one page-locked block, x then y then z: set_coords fills it and the device reads it from there)
+    double *host_x = nullptr, *host_y = nullptr, *host_z = nullptr;
     int64_t launches = 0;
     int last_max_row = 0;
     int cap = 0;

@@ -84,8 +84,8 @@ class FFieldCUDA:
 
     # ---- coordinates and moves
     def setCoords(self, xyz) -> None:
-        xyz = np.asarray(xyz, np.float64)
-        x, y, z = (np.ascontiguousarray(xyz[:, k]) for k in range(3))
+        xyz = np.ascontiguousarray(np.asarray(xyz, np.float64)[:, :3].T)   # one pass over the atoms
+        x, y, z = xyz
         native.check(native.lib().mcg_set_coords(self.h, native.pd(x), native.pd(y), native.pd(z)))
 
     def coords(self) -> np.ndarray:

@@ -304,3 +304,32 @@ def test_trial_moves(prec, cut, m):
     # the oracle's own difference of two totals carries both sums' rounding
     tol = 1e-4 * KCAL * max(1.0, (m / 3) ** 0.5) if prec == "mixed" else 2 * REL * _scale(s)
     assert abs(de - want) <= tol, (de, want, tol)
+
+
+# moves of several atoms in the device-resident run: pairs inside the moved set, terms of one atom's row on
+# other threads than the next's, and the order of the commits
+@pytest.mark.parametrize("apr", [1, 2, 3, 7, 64])
+def test_device_run_moves_of_several_atoms(apr):
+    s = systems.argon_fcc(6)
+    s.resid = np.arange(s.natom, dtype=np.int32) // apr + 1
+    s.moves[0].move_mode = "residue"
+    dev, host = FFieldCUDA(s, "fp64"), FFieldCUDA(s, "fp64")
+    l0 = dev.kernel_launches()
+    _, e_dev, a_dev, _ = dev.metropolis(400, 7, acceptance="physical", trace=False)
+    assert dev.kernel_launches() - l0 < 200          # on the device: a launch per 50 steps and the list builds
+    _, e_host, a_host, _ = host.metropolis(400, 7, acceptance="physical", trace=True)
+    assert a_dev == a_host and np.array_equal(dev.coords(), host.coords())
+    assert abs(e_dev - e_host) <= 1e-10 * abs(e_host)
+
+
+def test_coordinates_that_are_refused_leave_the_engine_as_it_was():
+    s = _near(_charged_argon(2500, 5), 6)
+    ff = FFieldCUDA(s, "fp64", moves=False)
+    e = ff.getE10()
+    for at, v in ((0, np.nan), (1024, np.inf), (2499, -np.inf)):
+        bad = s.coords() + 0.01
+        bad[at, at % 3] = v
+        with pytest.raises(native.McgError, match="atom %d" % at):
+            ff.setCoords(bad)
+        assert np.array_equal(ff.coords(), s.coords()) and np.array_equal(ff.getE10(), e)
+        assert ff.getE_host(s.x, s.y, s.z) == e[0]
