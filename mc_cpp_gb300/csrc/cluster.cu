@@ -14,7 +14,7 @@
 //   k_energy_cluster warp per i-cluster (taken from a work counter), 8 x 8 slot pairs per
 //                  cluster pair in two passes of 32 lanes; cluster pairs whose boxes are farther
 //                  apart than rc are skipped; one FP64 partial pair per cluster, summed in a fixed
-//                  order by k_finalize.
+//                  order by k_energy_tail.
 //
 // The pair terms are those of FField_MDBAS::computeNonBonded_switch (FField_MDBAS.cpp:336-424):
 // r^2 <= rc^2 in the list, switch S(r^2) = (rc^2-r^2)^2 (rc^2+2r^2-3ron^2)/(rc^2-ron^2)^3 above

@@ -36,7 +36,7 @@ public:
     int build(cudaStream_t st, const uint4* fx, int n, const double L[3], const int* nbr, const int* nup,
               const int* nlo, int cap);
     // Launches the per-call pack kernel and the energy kernel (variant v of kVariants); writes
-    // 2 doubles (elec, vdw, unscaled as k_finalize expects) per cluster into part, returns the
+    // 2 doubles (elec, vdw, unscaled as k_energy_tail expects) per cluster into part, returns the
     // number of partial pairs written.
     int launch_energy(cudaStream_t st, int v, const uint4* fx, const float4* prmf, const ClusterGeom& G, double* part);
     static constexpr int kVariants = 2;

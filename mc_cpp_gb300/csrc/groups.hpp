@@ -42,7 +42,7 @@ public:
     // each, all j > i).  Returns MCG_OK, or a failure status; on MCG_ECAPACITY the path is marked
     // unavailable and the caller keeps the per-atom list kernels.
     int build(cudaStream_t st, const int* rows, const int* lens, int cap);
-    // Energy kernel, variant v of kVariants: writes 2 doubles (elec, vdw, unscaled as k_finalize
+    // Energy kernel, variant v of kVariants: writes 2 doubles (elec, vdw, unscaled as k_energy_tail
     // expects) per CTA into part and returns the number of CTAs.  Needs the parameter-class table
     // (cls, ncls > 0).
     int launch_energy(cudaStream_t st, int v, const uint4* fx, const float4* cls, int ncls, const GroupGeom& G,

@@ -226,18 +226,20 @@ __device__ __forceinline__ bool stored_excluded(int lo, int hi, const int* __res
 // A warp per task: up to A home atoms of one cell share the walk over the stencil's candidates, which
 // lie in cell order (coalesced 16-byte loads, no index gather), 32 at a time.  The stencil's rows of
 // cells become ranges of the candidates, dropped or trimmed where no home atom reaches; the ranges are
-// walked as one sequence (a lane finds its range by advancing through their prefix sums), so short
-// ranges leave no lane idle, and the next 32 candidates load while these are tested.  A row lists its
+// walked as one sequence, the end of one with the beginning of the next, and the next 64 candidates load
+// while these are tested.  A row lists its
 // partners in the candidates' order, whatever the grouping.  In periodic boxes a pair is first placed by its
 // FP32 distance from the exact fixed-point mirrors (error ~2e-7 of (rc + skin)^2); the reference's FP64
 // distance decides only the pairs within 1e-4 of the list radius, so the rows are the reference's sets.
 // Before the home atoms' tests the candidates pass one against the sphere around all of them, and the
 // survivors (1,750 of 3,200 for four atoms of one octant of a water cell, 1,150 end in a row) are
 // gathered in a ring, 32 at a time.  Bound by issue.  (One atom per warp with an index gather in front
-// of every candidate took 1.48 ms on the 100,002-atom water box and 188 us at 12,288 atoms; this form
-// takes 0.70 ms and 123 us.)
+// of every candidate took 1.48 ms on the 100,002-atom water box and 188 us at 12,288 atoms.  Two candidates
+// per lane in the walk, and tasks from a counter instead of a third wave of CTAs, took a whole update of
+// the former from 754 to 653 us.)
 constexpr int ROW_WARPS = 4;
-constexpr int ROW_RING = 64;   // up to 31 pending candidates and 32 new ones
+constexpr int ROW_CTAS = 7;    // CTAs of four warps resident per SM at the kernel's 72 registers
+constexpr int ROW_RING = 128;  // up to 63 pending candidates and 64 new ones
 
 // The pairs the FP32 test does not decide: in the band around the list radius, close in index (the atom
 // itself, or perhaps excluded), or with frozen atoms about.
@@ -274,21 +276,27 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
     int2* range = s_range[wib];
     uint4* ring = s_ring[wib];
     const int ntask = task_start[ncell];
-    const int span = lp.any_frozen ? 0x3fffffff : lp.maxspan;   // frozen atoms: every pair is looked at
+    // partners within maxspan in index are looked at; with frozen atoms about, every partner
+    const unsigned span2 = lp.any_frozen ? 0xffffffffu : 2u * (unsigned)lp.maxspan;
     int longest = 0;
-    for (int task = blockIdx.x * ROW_WARPS + wib; task < ntask; task += gridDim.x * ROW_WARPS) {
+    // the first task by the warp's place, the others from a counter (max_row[1]), each fetched while the one
+    // before it is worked on: a grid of what is resident at once, without a last wave
+    int task = blockIdx.x * ROW_WARPS + wib, after = 0;
+    for (; task < ntask; task = __shfl_sync(0xffffffffu, after, 0)) {
+        if (lane == 0) after = gridDim.x * ROW_WARPS + atomicAdd(max_row + 1, 1);
         const int2 tk = tasks[task];
         const int c = tk.x, m = min(A, cell_start[c + 1] - tk.y);
         const int ctr[3] = {c % g.nc[0], (c / g.nc[0]) % g.nc[1], c / (g.nc[0] * g.nc[1])};
         // the home atoms: candidate entries tk.y .. tk.y + m; a missing one repeats the first and is not stored
         uint32_t hx[A][3];
-        int hi[A], up[A], back[A];
+        int hi[A], up[A], back[A], first[A];
         int* row[A];
 #pragma unroll
         for (int k = 0; k < A; k++) {
             const uint4 p = cell_pos[home[tk.y + (k < m ? k : 0)]];
             hx[k][0] = p.x; hx[k][1] = p.y; hx[k][2] = p.z;
             hi[k] = (int)p.w;
+            first[k] = hi[k] - lp.maxspan;
             up[k] = 0;
             back[k] = lp.cap - 1;
             row[k] = nbr + (size_t)p.w * lp.cap;
@@ -364,8 +372,8 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
                 re0 = cell_start[rowc + a1 + 1];
             }
         }
-        // the non-empty ranges in order; a walk over them takes 32 candidates at a time, the end of one
-        // range together with the beginning of the next
+        // the non-empty ranges in order; a walk over them takes 64 candidates at a time, two per lane, the
+        // end of one range together with the beginning of the next
         const unsigned b1 = __ballot_sync(0xffffffffu, re1 > rb1), b0 = __ballot_sync(0xffffffffu, re0 > rb0);
         const int nrange = __popc(b1) + __popc(b0);
         __syncwarp();
@@ -373,43 +381,50 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
         if (re0 > rb0) range[__popc(b1 & (below << 1 | 1u)) + __popc(b0 & below)] = make_int2(rb0, re0);
         if (lane < 2) range[nrange + lane] = make_int2(0, 0);
         __syncwarp();
+        constexpr uint32_t NONE = 0xffffffffu;
         int rg = 0;
         int2 cur = range[0], nxt = range[1];
-        auto fetch = [&]() -> uint4 {
-            const int rem = cur.y - cur.x;                       // at least 1 until the walk's end
-            const int at = lane < rem ? cur.x + lane : nxt.x + lane - rem;
-            const bool have = lane < rem || at < nxt.y;
-            if (rem > 32) {
-                cur.x += 32;
+        auto fetch = [&](uint4& c0, uint4& c1) {
+            const int rem = cur.y - cur.x, skip = nxt.x - rem;   // at least 1 until the walk's end
+            const int l1 = lane + 32;
+            const int at0 = lane < rem ? cur.x + lane : skip + lane, at1 = l1 < rem ? cur.x + l1 : skip + l1;
+            c0.w = c1.w = NONE;
+            if (lane < rem || at0 < nxt.y) c0 = cell_pos[at0];
+            if (l1 < rem || at1 < nxt.y) c1 = cell_pos[at1];
+            if (rem > 64) {
+                cur.x += 64;
             } else {
-                cur = make_int2(min(nxt.x + 32 - rem, nxt.y), nxt.y);
+                cur = make_int2(min(skip + 64, nxt.y), nxt.y);
                 rg++;
-                nxt = rg + 1 < nrange ? range[rg + 1] : make_int2(0, 0);
+                nxt = range[min(rg + 1, nrange)];
                 if (cur.x == cur.y && rg < nrange) {             // the next range was used up whole
                     cur = nxt;
                     rg++;
-                    nxt = rg + 1 < nrange ? range[rg + 1] : make_int2(0, 0);
+                    nxt = range[min(rg + 1, nrange)];
                 }
             }
-            return have ? cell_pos[at] : make_uint4(0, 0, 0, 0xffffffffu);
         };
         bool more = rg < nrange;
-        uint4 next = fetch();
+        uint4 n0 = make_uint4(0, 0, 0, NONE), n1 = n0;
+        fetch(n0, n1);
         int head = 0, tail = 0;            // candidates within reach of the home atoms, pending in the ring
+        auto within = [&](const uint4& c) {
+            if (!PERIODIC) return c.w != NONE;
+            const float dx = __int2float_rn((int)(c.x - ball[0])) * lp.Ls[0], dy = __int2float_rn((int)(c.y - ball[1])) * lp.Ls[1],
+                        dz = __int2float_rn((int)(c.z - ball[2])) * lp.Ls[2];
+            return c.w != NONE && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= ball2;
+        };
         while (more || head != tail) {
-            if (more) {
-                const uint4 cd = next;
+            if (more && head - tail < 64) {
+                const uint4 c0 = n0, c1 = n1;
                 more = rg < nrange;
-                if (more) next = fetch();
-                bool near = cd.w != 0xffffffffu;
-                if (PERIODIC) {
-                    const float dx = __int2float_rn((int)(cd.x - ball[0])) * lp.Ls[0], dy = __int2float_rn((int)(cd.y - ball[1])) * lp.Ls[1],
-                                dz = __int2float_rn((int)(cd.z - ball[2])) * lp.Ls[2];
-                    near = near && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= ball2;
-                }
-                const unsigned b = __ballot_sync(0xffffffffu, near);
-                if (near) ring[(head + __popc(b & below)) & (ROW_RING - 1)] = cd;
-                head += __popc(b);
+                if (more) fetch(n0, n1);
+                const bool in0 = within(c0), in1 = within(c1);
+                const unsigned m0 = __ballot_sync(0xffffffffu, in0), m1 = __ballot_sync(0xffffffffu, in1);
+                const int h1 = head + __popc(m0);
+                if (in0) ring[(head + __popc(m0 & below)) & (ROW_RING - 1)] = c0;
+                if (in1) ring[(h1 + __popc(m1 & below)) & (ROW_RING - 1)] = c1;
+                head = h1 + __popc(m1);
                 __syncwarp();
                 if (more && head - tail < 32) continue;
             }
@@ -434,11 +449,10 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
                         const float dx = ux * lp.Ls[0], dy = uy * lp.Ls[1], dz = uz * lp.Ls[2];
                         r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
                     }
-                    if (r2 <= hi2) {
-                        in |= 1u << k;
-                        if (!(r2 < lo2)) band |= 1u << k;
-                        if ((unsigned)(j - hi[k] + span) <= 2u * (unsigned)span) look |= 1u << k;
-                    }
+                    const unsigned near = r2 <= hi2 ? 1u << k : 0u;
+                    in |= near;
+                    band |= r2 < lo2 ? 0u : near;
+                    look |= (unsigned)(j - first[k]) <= span2 ? near : 0u;
                 }
             } else if (j >= 0) {
                 in = band = (1u << A) - 1u;
@@ -456,7 +470,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
 #pragma unroll
             for (int k = 0; k < A; k++) {
                 const bool mine = in >> k & 1u, above = j > hi[k];
-                const unsigned b = __ballot_sync(0xffffffffu, mine), bu = __ballot_sync(0xffffffffu, mine && above);
+                const unsigned b = __ballot_sync(0xffffffffu, mine), bu = b & __ballot_sync(0xffffffffu, above);
                 const int rank = __popc((above ? bu : b ^ bu) & below), at = up[k] + rank;
                 // the front of the row grows up, its back down; a row that would pass its capacity is not stored
                 const int off = above ? at : back[k] - rank;
@@ -735,7 +749,7 @@ __device__ __forceinline__ void mix_batch(const int (&j)[U], const uint4 (&fj)[U
 // by q_i (float-float) and eps_i into float-float totals; no FP64 arithmetic until the block sum.
 // The switch is formed unscaled as A^2 B with A = rc^2 - u, B = 2u + rc^2 - 3 ron^2 and u = r^2
 // raised to ron^2; inv_f1 = 1 / (that FP32 polynomial at ron^2) scales the block sums, so inner
-// pairs have S = 1 exactly.  Same terms as mixed_pair (unscaled, k_finalize scales).
+// pairs have S = 1 exactly.  Same terms as mixed_pair (unscaled, k_energy_tail scales).
 // U list entries in flight per lane; MINB resident CTAs per SM requested from the register
 // allocator (occupancy against registers); the engine times the variants once and keeps the fastest.
 // Without the class table (TYPED below), both gathers of an entry (position and parameters) are
@@ -1615,7 +1629,7 @@ int SingleEngine::init(const HostSystem& h) {
     size_t nparts = std::max<size_t>({(size_t)152 * 8, (size_t)ntile * (ntile + 1) / 2, (size_t)MAX_MOVED + 1});
     part_cap = nparts * 3 + 2 * 64 + 5 * BD_BLOCKS + 16;
     if ((rc = dalloc(&d_part, part_cap)) || (rc = dalloc(&d_ticket, 2)) ||
-        (rc = dalloc(&d_maxrow, 1)))
+        (rc = dalloc(&d_maxrow, 2)))
         return rc;
     CK(cudaMemsetAsync(d_ticket, 0, 2 * sizeof(unsigned), stream));
     // staging for moves: idx (sorted), xyz, terms
@@ -2095,12 +2109,12 @@ int SingleEngine::build_list() {
     }
     for (int attempt = 0; attempt < 3; attempt++) {
         CK(cudaMemsetAsync(d_cell_count, 0, sizeof(int) * ncell, stream));
-        CK(cudaMemsetAsync(d_maxrow, 0, sizeof(int), stream));
+        CK(cudaMemsetAsync(d_maxrow, 0, 2 * sizeof(int), stream));
         k_cell_assign<<<(n + 255) / 256, 256, 0, stream>>>(d_pq, n, pbc, g, d_cell_of, d_cell_count);
         k_cell_scan<<<1, 1024, 0, stream>>>(d_cell_count, ncell, run, d_cell_start, d_cell_fill, d_task_start);
         k_cell_scatter<<<(n + 255) / 256, 256, 0, stream>>>(d_cell_of, n, d_cell_start, d_cell_fill, d_cell_atoms);
         k_cell_sort<<<ncell, 128, 0, stream>>>(d_cell_start, d_task_start, ncell, run, d_fx, g, d_cell_atoms, d_cell_pos, d_home, d_tasks);
-        const int blocks = std::min((n / run + ncell + ROW_WARPS - 1) / ROW_WARPS, 152 * 16);
+        const int blocks = std::min((n / run + ncell + ROW_WARPS - 1) / ROW_WARPS, 152 * ROW_CTAS);
 #define MCG_ROWS(A_, P_, I_)                                                                                          \
     k_build_rows<A_, P_, I_><<<blocks, 32 * ROW_WARPS, 0, stream>>>(d_pq, d_cell_pos, d_frozen, pbc, g, lp, d_cell_start, \
                                                                 d_task_start, ncell, d_home, d_tasks, d_xs, d_xd, d_nbr, d_nup, d_nlo, d_maxrow)
