@@ -2445,8 +2445,8 @@ __device__ __forceinline__ double rp_pair(double4_32a a, double4_32a b, double2 
 // Measured on the 864-atom argon box (moves per second, host work included): 49.8k with one
 // 256-thread CTA (its ~200 dE terms at two warps per scheduler), 89.9k with the cluster and the
 // words read from global memory, 94.8k with them in shared memory, 99.9k with the fifth warp.
-// In runs of 500 steps, 92k so far, 107k with the FP64 operations of ref64_mic and rsqrt64, 141k with one
-// barrier and one sum a step.
+// In runs of 500 steps, 92k so far, 107k with the FP64 operations of ref64_mic and rsqrt64, 142k with one
+// barrier and one sum a step, 152k with the terms off the fifth warp's scheduler and its draw used.
 constexpr int RP_CL = 8;
 constexpr int RP_NT = 128;
 constexpr int RP_TRIES = 8;
@@ -2479,6 +2479,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
     // the next step's uniforms, both cases (0: no acceptance draw in this step, 1: one)
     __shared__ double s_sx[2 * RP_TRIES], s_sy[2 * RP_TRIES], s_sz[2 * RP_TRIES], s_sq[2 * RP_TRIES];
     __shared__ int s_st[2], s_sg[2], s_sok;
+    __shared__ double s_alpha;      // this step's acceptance uniform, when the fifth warp could form it
     __shared__ long long s_sbase;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = RP_NT / 32, G = RP_CL * RP_NT;
@@ -2494,7 +2495,9 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
     const int* inst_first = tab_sh ? s_tab : T.inst_first;
     const int* ranges = tab_sh ? s_tab + T.ninst_all : T.ranges;
     const int rank = (int)cluster.block_rank();
-    const int gslot = rank + RP_CL * (warp + NW * lane);   // this thread's place in the spread order
+    // this thread's place in the order the terms are dealt: CTAs first, then the lanes of warps 1 and 2, then
+    // those of 3 and 0.  Up to 512 terms (255 partners of one atom) leave warp 0's scheduler to the fifth warp
+    const int gslot = rank + RP_CL * (2 * lane + (warp == 1 || warp == 2 ? warp - 1 : 64 + (warp == 0)));
     if (tid == 0) S = *st;
     cluster.sync();   // every CTA of the cluster is running before any writes into its shared memory
     for (int step = s0 + 1; step <= s1; step++) {
@@ -2532,10 +2535,9 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
                     if (ok) {
                         const int k = __ffs(ok) - 1;
                         first = k;
-                        if (lane == k) {
-                            const double dm = S.dmax[t];
+                        if (lane < 3) {   // a component per lane: one product's latency
                             const int e = sv * RP_TRIES + k;
-                            s_r[0] = __dmul_rn(s_sx[e], dm); s_r[1] = __dmul_rn(s_sy[e], dm); s_r[2] = __dmul_rn(s_sz[e], dm);
+                            s_r[lane] = __dmul_rn(lane == 0 ? s_sx[e] : lane == 1 ? s_sy[e] : s_sz[e], S.dmax[t]);
                         }
                     }
                     pass0 = 1;
@@ -2609,7 +2611,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
                 s_sx[lane] = x; s_sy[lane] = y; s_sz[lane] = z;
                 s_sq[lane] = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
             }
-            if (lane == 0) { s_sbase = b; s_sok = ok ? 1 : 0; }
+            if (lane == 0) { s_sbase = b; s_sok = ok ? 1 : 0; s_alpha = c; }   // uniform 0 is the draw, if there is one
         }
         // dE of the moved set over its Verlet partners and 1-4 pairs, FP64 (as k_delta_e): term
         // (k, t, side) of the moved atoms' partner lists, numbered in list order, goes to the thread
@@ -2655,7 +2657,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
         }
         double* cl = s_cl[step & 1];
         if (warp < NW) {
-            val = warp_sum(val);
+            if (__any_sync(0xffffffffu, __double_as_longlong(val) != 0)) val = warp_sum(val);
             if (lane < RP_CL) *cluster.map_shared_rank(cl + rank * NW + warp, lane) = val;
         }
         cluster.sync();
@@ -2669,7 +2671,8 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
                 bool accepted;
                 if (de <= 2.220446049250313e-16) accepted = true;
                 else {
-                    const double alpha = rp_canonical(s_words, cur);
+                    const double alpha = s_sok ? s_alpha : rp_canonical_at(s_words, cur);
+                    cur += 2;
                     const float af = (float)alpha, ef = __expf((float)(-beta * de));   // off by less than 1e-5
                     accepted = fabsf(af - ef) > 1e-4f ? af < ef : alpha < exp(-beta * de);
                 }
