@@ -1028,16 +1028,15 @@ __device__ __forceinline__ double master_to_f64(unsigned long long v, double L) 
 // (fixed64.cuh; the masters are box fractions already).  Two kernels:
 //  - k_batch_extent: each chain's largest distance from a residue's first atom to its other atoms, from
 //    the mirrors, so that residues whose first atoms are farther than rc + 2 extents share no pair;
-//  - k_batch_energy64: a CTA per E64_RES residues of a chain, a warp per residue r.  Its lanes test
+//  - k_batch_energy64: a CTA per tile_res residues of a chain, a warp per residue r.  Its lanes test
 //    the first atoms of all residues q > r by FP32 distance; the residue pairs within reach go to a ring,
 //    32 of them at a time are split into atom pairs, placed by FP32 distance again, and the atom pairs
 //    within rc go to two rings (inside ron, or switched), each evaluated with all 32 lanes busy.
 // Nothing depends on the neighbour lists.  The tests are FP32 and cheap: a chain of 8,192 residues takes
 // about 2,600 warp instructions of them per residue, beside some 11,000 for its pair terms.
-// 64 water chains of 512 to 8,192 molecules: 3.5 ms, 308 ms with a thread per atom over all later atoms
+// 64 water chains of 512 to 8,192 molecules: 3.6 ms, 308 ms with a thread per atom over all later atoms
 // in FP64.
 constexpr int E64_RING = 64;      // up to 31 pending entries and 32 new ones
-constexpr int E64_RES = 32;       // residues of a CTA (8 when that leaves SMs without one)
 
 __global__ void __launch_bounds__(256) k_batch_extent(const ChainDev* __restrict__ chains, const uint4* __restrict__ F,
                                                       int* ext2) {
@@ -1969,7 +1968,13 @@ int mcg_batch_create(const mcg_system_desc* descs, int nchains, const mcg_batch_
     BK(cudaMemsetAsync(B->d_state, 0, sizeof(ChainState) * nchains, B->stream));
     std::vector<int>& tc = B->tile_chain;
     std::vector<int> tf;
-    B->tile_res = res0 >= (int64_t)4 * B->nsm * E64_RES ? E64_RES : 8;   // four CTAs of the larger tiles per SM, or the smaller
+    // Residues of a CTA of k_batch_energy64: fewer leave half-filled rings (and at one atom per residue hardly
+    // fill them once), more leave SMs idle behind the last wave.  Water chains with 8, 16 and 32: 1,024 residues
+    // 112, 192, 342 us; 36,400 794, 833, 975; 171,500 3662, 3606, 3715; 701,800 14.77, 14.39, 14.44 ms.  Argon
+    // chains: 78,500 residues 377, 297, 285 us; 1,263,000 5.49, 3.93, 3.34 ms.
+    const bool atoms = apr_all == 1;
+    const int large = atoms ? 32 : 16;
+    B->tile_res = res0 >= (int64_t)(atoms ? 4 : 64) * B->nsm * large ? large : 8;
     for (int c = 0; c < nchains; c++)
         for (int f = 0; f < B->chains[c].nres; f += B->tile_res) { tc.push_back(c); tf.push_back(f); }
     B->ntiles = (int)tc.size();

@@ -916,11 +916,12 @@ __global__ void __launch_bounds__(TILE) k_energy_all(AtomsDev A, int n, PbcDev p
 // memory; units are numbered over the upper triangle row tile by row tile and dealt to the CTAs in
 // turn.  Short columns, because a thread's walk along them is serial: a box of 1,536 atoms has 312
 // units (12 x 13 / 2 = 78 with square tiles, for 152 SMs), and a CTA's partial sum covers all its units.
-// 12,288 atoms (75 M pairs): the whole energy call takes 0.58 ms, 3.78 ms with the pair terms in FP64.
+// 12,288 atoms (75 M pairs): the whole energy call takes 0.62 ms, 3.78 ms with the pair terms in FP64.
 constexpr int A64_I = 128, A64_J = 32;
+constexpr int A64_CTAS = 10;   // per SM; 8: 641 against 622 us for a call at 12,288 atoms
 
 template <bool ISO, bool TABLE>
-__global__ void __launch_bounds__(A64_I) k_energy_all64(AtomsDev A, Fix64Geom G, PbcDev pbc, CutDev cut, int n,
+__global__ void __launch_bounds__(A64_I, A64_CTAS) k_energy_all64(AtomsDev A, Fix64Geom G, PbcDev pbc, CutDev cut, int n,
                                                         const int* __restrict__ fxs, const int* __restrict__ fxd,
                                                         int units, double* part) {
     __shared__ ulonglong4_32a sx[A64_J];
@@ -1626,7 +1627,7 @@ int SingleEngine::init(const HostSystem& h) {
     term_start[n] = (int)term_data.size() / 2;
     // scratch: partial sums and the ΔE ticket
     ntile = (n + TILE - 1) / TILE;
-    size_t nparts = std::max<size_t>({(size_t)152 * 8, (size_t)ntile * (ntile + 1) / 2, (size_t)MAX_MOVED + 1});
+    size_t nparts = std::max<size_t>({(size_t)152 * A64_CTAS, (size_t)ntile * (ntile + 1) / 2, (size_t)MAX_MOVED + 1});
     part_cap = nparts * 3 + 2 * 64 + 5 * BD_BLOCKS + 16;
     if ((rc = dalloc(&d_part, part_cap)) || (rc = dalloc(&d_ticket, 2)) ||
         (rc = dalloc(&d_maxrow, 2)))
@@ -2159,7 +2160,7 @@ int SingleEngine::energy(double ener[10]) {
         if (uses_fix64()) {
             const long long tiles = (n + A64_I - 1) / A64_I, c0 = (n + A64_J - 1) / A64_J;
             const int units = (int)(tiles * c0 - (A64_I / A64_J) * tiles * (tiles - 1) / 2);
-            nnb = std::min(units, 152 * 8);
+            nnb = std::min(units, 152 * A64_CTAS);
 #define MCG_ALL64(ISO_, TAB_)                                                                                         \
     k_energy_all64<ISO_, TAB_><<<nnb, A64_I, 0, stream>>>(A, fix64, pbc, cut, n, d_fxs, d_fxd, units, nbp)
             if (fix64.iso && ncls64) MCG_ALL64(true, true);

@@ -181,16 +181,18 @@ def test_moves_keep_the_mirror_current():
 
 def _check_chains(B, chains):
     e = B.energy_fp64()
-    for k, s in enumerate(chains):
-        t = s.copy()
+    for k in range(0, len(chains), 1 if len(chains) < 8 else 9):
+        t = chains[k].copy()
         t.set_coords(B.coords(k))
         want = np.array(orc.Oracle(t, moves=False).energy())
         assert abs(e[k] - (want[3] + want[4])) <= REL * _scale(t), (k, e[k], want)
 
 
-# tiles of 8 or 32 residues (the larger from 19,456 residues in all), residue sizes 1 and 3 and both
+# tiles of 8 residues, of 32 (one-atom residues from 19,456 in all) and of 16 (others from 155,648), residue sizes 1
+# and 3 and both
 @pytest.mark.parametrize("sizes", [[("water", 513)], [("argon", 331), ("argon", 513)], [("water", 512), ("argon", 640), ("water", 519)],
-                                   [("water", 6500), ("water", 6489), ("water", 6511)]])
+                                   [("water", 6500), ("water", 6489), ("water", 6511)],
+                                   [("argon", 2001 + k) for k in range(10)], [("water", 8177 + k) for k in range(20)]])
 def test_batch_energy(sizes):
     chains = [systems.water_box(n, seed=n) if kind == "water" else systems.argon_random(n, 0.0213, n) for kind, n in sizes]
     if len(chains) == 2:
