@@ -52,7 +52,8 @@ namespace mcg {
 
 constexpr int NB_BLOCKS = 152 * 4;   // grid of the list-driven kernels: 4 CTAs per SM
 constexpr int NB_THREADS = 256;
-constexpr int BD_BLOCKS = 152 * 2;   // largest grid of the bonded terms: their FP64 pipes are the bound
+constexpr int BD_BLOCKS = 152 * 4;   // largest grid of the bonded terms: a term per thread up to 155,648 (two CTAs per
+                                     // SM: 116 against 111 us for the mixed energy of 100,002 water atoms; one: 121)
 constexpr int MAX_MOVED = 1024;
 constexpr int SORT_MAX = 2048;       // cells larger than this are sorted by one thread
 constexpr int CLS_MAX = 1024;        // parameter classes the mixed pair kernel keeps in shared memory
@@ -1022,9 +1023,9 @@ __device__ double bond_e(const BondT& b, const CrdSrc& S, const PbcDev& pbc, boo
 // multiple of it, and both follow from sines and cosines: the library's acos, atan2 and cos are
 // some 100 FP64 operations each, at 64 cycles of a scheduler's FP64 pipe per warp.  The general form
 // (out of line) stays for what the short one does not cover: an angle more than 2^-6 off its reference
-// or nearly straight, a multiplicity that is not an integer of 0 to 6, three atoms in line.  With two
-// CTAs per SM instead of 64 in all this took the bonded terms of 100,002 water atoms from 31 us (46
-// before the minimum image went to integer compares) to 12.
+// or nearly straight, a multiplicity that is not an integer of 0 to 6, three atoms in line.  With a grid
+// of two CTAs per SM instead of 64 in all this took the bonded terms of 100,002 water atoms from 31 us
+// (46 before the minimum image went to integer compares) to 12; a term per thread (BD_BLOCKS) came after.
 
 // asin(s) for |s| <= 2^-6: the Taylor series to s^9 (the next term is below 2^-64 of s)
 __device__ __forceinline__ double asin_small(double s) {
