@@ -19,7 +19,7 @@
 //   k_cell_assign / k_cell_scan / k_cell_scatter / k_cell_sort / k_build_rows   Verlet build
 //   k_energy_list<P>   switch energy over the half list (warp per row)        FField_MDBAS.cpp:336-424
 //   k_energy_list64    the same in FP64 for periodic boxes, on 64-bit integer pair terms
-//   k_energy_all<P>    full energy over all pairs (triangular tile grid)      FField_MDBAS.cpp:194-265
+//   k_energy_all*      full energy over all pairs (triangle of tiles)         FField_MDBAS.cpp:194-265
 //   k_energy_all64     the same in FP64 for periodic boxes, on 64-bit integer pair terms
 //   k_energy_tail<P>   1-4 pairs                                               FField_MDBAS.cpp:267-318,426-488
 //                      bonds, Urey-Bradley, angles, dihedrals, impropers       FField_MDBAS.cpp:490-786
@@ -28,6 +28,7 @@
 //   k_commit           write accepted coordinates
 #include <algorithm>
 #include <array>
+#include <climits>
 #include <map>
 #include <cmath>
 #include <cstring>
@@ -863,17 +864,15 @@ __global__ void __launch_bounds__(NB_THREADS) k_prune_rows(const uint4* __restri
     if (lane == 0 && kept) atomicAdd(kept_total, kept);
 }
 
-// Full energy: all pairs j > i not in the full-mode exclusion row of i, no cutoff.  Triangular
-// grid of TILE x TILE blocks; each thread owns one i and walks a shared-memory j tile with the
-// reference's sorted-row cursor (FField_MDBAS.cpp:227-234).
+// Full energy without a box, FP64: all pairs j > i not in the full-mode exclusion row of i, no cutoff.
+// Triangular grid of TILE x TILE blocks; each thread owns one i and walks a shared-memory j tile with
+// the reference's sorted-row cursor (FField_MDBAS.cpp:227-234).
 constexpr int TILE = 128;
 
-template <int P>
 __global__ void __launch_bounds__(TILE) k_energy_all(AtomsDev A, int n, PbcDev pbc, CutDev cut,
                                                      const int* __restrict__ fxs, const int* __restrict__ fxd,
                                                      int ntile, double* part) {
     __shared__ double4_32a spq[TILE];
-    __shared__ uint4 sfx[TILE];
     pair_kernel_begin();
     // block -> (I, J) with I <= J, row-major over the upper triangle
     int b = blockIdx.x;
@@ -882,66 +881,170 @@ __global__ void __launch_bounds__(TILE) k_energy_all(AtomsDev A, int n, PbcDev p
     int J = I + b;
     int i = I * TILE + threadIdx.x;
     int jt = J * TILE + threadIdx.x;
-    if (jt < n) {
-        spq[threadIdx.x] = A.pq[jt];
-        if (P == PREC_MIX) sfx[threadIdx.x] = A.fx[jt];
-    }
+    if (jt < n) spq[threadIdx.x] = A.pq[jt];
     __syncthreads();
     double sel = 0.0, svd = 0.0;
     if (i < n) {
-        double4_32a pi = A.pq[i];
-        uint4 fi = P == PREC_MIX ? A.fx[i] : make_uint4(0, 0, 0, 0);
-        int xb = fxs[i], xe = fxs[i + 1];
-        int cur = xb;
-        int j0 = max(J * TILE, i + 1);
+        const double4_32a pi = A.pq[i];
+        const uint4 f0 = make_uint4(0, 0, 0, 0);
+        int cur = fxs[i];
+        const int xe = fxs[i + 1], j0 = max(J * TILE, i + 1), jend = min(n, J * TILE + TILE);
         while (cur < xe && fxd[cur] < j0) cur++;
-        int jend = min(n, J * TILE + TILE);
-        F32Acc fe, fv;
         for (int j = j0; j < jend; j++) {
             if (cur < xe && fxd[cur] == j) { cur++; continue; }
-            int t = j - J * TILE;
             double el, vd;
-            pair_energy<P>(A, pbc, cut, false, pi, fi, i, spq[t], P == PREC_MIX ? sfx[t] : make_uint4(0, 0, 0, 0), j,
-                           false, el, vd);
-            if (P == PREC_F64) { sel += el; svd += vd; }
-            else { fe.add((float)el); fv.add((float)vd); }
+            pair_energy<PREC_F64>(A, pbc, cut, false, pi, f0, i, spq[j - J * TILE], f0, j, false, el, vd);
+            sel += el;
+            svd += vd;
         }
-        if (P == PREC_MIX) { sel = fe.value(); svd = fv.value(); }
     }
     block_reduce2(sel, svd, part + 2 * blockIdx.x);
 }
 
+// The other full energies deal units of ALL_I rows (a thread each) against ALL_J columns staged in shared
+// memory to the CTAs in turn; units are numbered over the upper triangle row tile by row tile.  Short
+// columns, because a thread's walk along them is serial: a box of 1,536 atoms has 312 units (12 x 13 / 2
+// = 78 with square tiles, for 152 SMs), and a CTA's partial sum covers all its units.
+constexpr int ALL_I = 128, ALL_J = 32, ALL_STEP = ALL_I / ALL_J;
+
+static long long all_units(int n) {
+    const long long tiles = (n + ALL_I - 1) / ALL_I, c0 = (n + ALL_J - 1) / ALL_J;
+    return tiles * c0 - ALL_STEP * tiles * (tiles - 1) / 2;
+}
+
+// Unit -> its row tile (returned) and first column; c0 column chunks in row tile 0, each next tile has
+// ALL_STEP fewer.  The float estimate is put right by steps of one.
+__device__ __forceinline__ int all_unit(long long unit, int c0, int& jb) {
+    auto first = [&](int I) { return (long long)I * c0 - (long long)ALL_STEP * I * (I - 1) / 2; };
+    const float b = c0 + 0.5f * ALL_STEP;
+    int I = (int)((b - sqrtf(fmaxf(b * b - 2.0f * ALL_STEP * (float)unit, 0.0f))) / ALL_STEP);
+    while (I > 0 && first(I) > unit) I--;
+    while (first(I + 1) <= unit) I++;
+    jb = I * ALL_I + (int)(unit - first(I)) * ALL_J;
+    return I;
+}
+
+// TwoSum on both halves: s becomes s + v, c takes what that rounds off
+__device__ __forceinline__ void two_sum_to(float2& s, float2& c, float2 v) {
+    const float2 neg = make_float2(-1.0f, -1.0f);
+    const float2 t = __fadd2_rn(s, v), b = __ffma2_rn(s, neg, t);
+    c = __fadd2_rn(c, __fadd2_rn(__ffma2_rn(__ffma2_rn(b, neg, t), neg, s), __ffma2_rn(b, neg, v)));
+    s = t;
+}
+
+// Mixed-precision full energy: the pair terms of mixed_pair without the switch for two columns at a time,
+// the halves of float2 values, summed per thread and half as float-float over all its units, in FP64
+// across the CTA.  A column that is not to count (excluded, not above the row, past the last atom) takes
+// 1/r = 0, which makes its terms exactly 0.  Bound by the FP32 pipe.  The columns' positions and
+// parameters come from shared memory, the row's and the next excluded atom stay in registers.
+// Without a box a displacement is an FP64 difference rounded to FP32, and those are the bound.
+// Whole energy calls, against a column at a time in square tiles with the exclusion row read at every
+// column: 12,288 water atoms (75 M pairs) 170 us, was 227; 36,864 1360, was 1652 (one column at a time
+// in these units: 1475); 4,096 argon atoms 37, was 56.
+constexpr int ALLMIX_CTAS = 5;   // per SM; 3,000 water atoms, 36,864: 4 take 31 and 1388 us, 5 34 and 1360, 8 37 and 1359
+
+template <bool BOX>
+__global__ void __launch_bounds__(ALL_I, ALLMIX_CTAS) k_energy_all_mix(AtomsDev A, int n,
+                                                                       const int* __restrict__ fxs,
+                                                                       const int* __restrict__ fxd, long long units,
+                                                                       double* part) {
+    __shared__ __align__(8) uint32_t sp[3][ALL_J];
+    __shared__ double sd[3][BOX ? 1 : ALL_J];
+    __shared__ __align__(8) float sprm[4][ALL_J];        // q hi, q lo, eps, sig
+    pair_kernel_begin();
+    const int c0 = (n + ALL_J - 1) / ALL_J;
+    const float2 zero = make_float2(0.0f, 0.0f), neg = make_float2(-1.0f, -1.0f);
+    auto both = [](float v) { return make_float2(v, v); };
+    float2 eh = zero, el = zero, vh = zero, vl = zero;
+    for (long long unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        int jb;
+        const int i = all_unit(unit, c0, jb) * ALL_I + threadIdx.x, je = min(n, jb + ALL_J);
+        __syncthreads();
+        if (threadIdx.x < ALL_J) {
+            const int t = threadIdx.x, jt = min(jb + t, n - 1);
+            if (BOX) {
+                const uint4 f = A.fx[jt];
+                sp[0][t] = f.x; sp[1][t] = f.y; sp[2][t] = f.z;
+            } else {
+                const double4_32a p = A.pq[jt];
+                sd[0][t] = p.x; sd[1][t] = p.y; sd[2][t] = p.z;
+            }
+            const float2 q = A.qf[jt], e = A.esf[jt];
+            sprm[0][t] = q.x; sprm[1][t] = q.y; sprm[2][t] = e.x; sprm[3][t] = e.y;
+        }
+        __syncthreads();
+        if (i >= n) continue;
+        uint4 fi = make_uint4(0, 0, 0, 0);
+        double4_32a pi = make_double4_32a(0, 0, 0, 0);
+        if (BOX) fi = A.fx[i];
+        else pi = A.pq[i];
+        const float2 qi = A.qf[i], ei = A.esf[i];
+        int cur = fxs[i];
+        const int xe = fxs[i + 1];
+        while (cur < xe && fxd[cur] < jb) cur++;
+        int next = cur < xe ? fxd[cur] : INT_MAX;     // the reference's sorted-row cursor (FField_MDBAS.cpp:227-234)
+        for (int j = max(jb, (i + 1) & ~1); j < je; j += 2) {
+            const int t = j - jb;
+            bool on0 = j > i, on1 = j + 1 < je;
+            if (next <= j + 1) {                 // rows hold partners above i only
+                for (; next <= j + 1; next = ++cur < xe ? fxd[cur] : INT_MAX) {
+                    if (next == j) on0 = false;
+                    else on1 = false;
+                }
+            }
+            auto col = [&](const float* v) { return *reinterpret_cast<const float2*>(v + t); };
+            float2 dx, dy, dz;
+            if (BOX) {
+                auto diff = [&](int k, uint32_t f) {
+                    const uint2 c = *reinterpret_cast<const uint2*>(&sp[k][t]);
+                    const float2 d = make_float2(__int2float_rn((int)(c.x - f)), __int2float_rn((int)(c.y - f)));
+                    return __ffma2_rn(d, both(A.Ls[k]), __fmul2_rn(d, both(A.Lsl[k])));
+                };
+                dx = diff(0, fi.x); dy = diff(1, fi.y); dz = diff(2, fi.z);
+            } else {
+                auto diff = [&](int k, double p) { return make_float2((float)(sd[k][t] - p), (float)(sd[k][t + 1] - p)); };
+                dx = diff(0, pi.x); dy = diff(1, pi.y); dz = diff(2, pi.z);
+            }
+            const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
+            float2 y = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+            y = __fmul2_rn(y, __ffma2_rn(__fmul2_rn(__fmul2_rn(both(-0.5f), r2), y), y, both(1.5f)));   // one Newton step
+            y.x = on0 ? y.x : 0.0f;
+            y.y = on1 ? y.y : 0.0f;
+            // the float-float charge product (ff_mul)
+            const float2 qh = col(sprm[0]), ql = col(sprm[1]);
+            const float2 ph = __fmul2_rn(both(qi.x), qh), nph = __fmul2_rn(both(-qi.x), qh);
+            const float2 pl = __fadd2_rn(__ffma2_rn(both(qi.x), qh, nph), __ffma2_rn(both(qi.x), ql, __fmul2_rn(both(qi.y), qh)));
+            two_sum_to(eh, el, __ffma2_rn(ph, y, __fmul2_rn(pl, y)));
+            const float2 s = __fadd2_rn(both(ei.y), col(sprm[3]));
+            const float2 x2 = __fmul2_rn(__fmul2_rn(s, s), __fmul2_rn(y, y)), x6 = __fmul2_rn(__fmul2_rn(x2, x2), x2);
+            const float2 l = __ffma2_rn(x6, x6, __fmul2_rn(neg, x6));
+            two_sum_to(vh, vl, __fmul2_rn(__fmul2_rn(both(ei.x), col(sprm[2])), l));
+        }
+    }
+    block_reduce2(((double)eh.x + (double)eh.y) + ((double)el.x + (double)el.y),
+                  ((double)vh.x + (double)vh.y) + ((double)vl.x + (double)vl.y), part + 2 * blockIdx.x);
+}
+
 // FP64 full energy for periodic boxes, on 64-bit integer pair terms (fixed64.cuh): three FP64
 // operations a pair, about 230 cycles of a scheduler's FP64 pipe per warp, beside some 150 integer
-// and FP32 ones.  A unit of work is A64_I rows (a thread each) against A64_J columns staged in shared
-// memory; units are numbered over the upper triangle row tile by row tile and dealt to the CTAs in
-// turn.  Short columns, because a thread's walk along them is serial: a box of 1,536 atoms has 312
-// units (12 x 13 / 2 = 78 with square tiles, for 152 SMs), and a CTA's partial sum covers all its units.
+// and FP32 ones.
 // 12,288 atoms (75 M pairs): the whole energy call takes 0.62 ms, 3.78 ms with the pair terms in FP64.
-constexpr int A64_I = 128, A64_J = 32;
 constexpr int A64_CTAS = 10;   // per SM; 8: 641 against 622 us for a call at 12,288 atoms
 
 template <bool ISO, bool TABLE>
-__global__ void __launch_bounds__(A64_I, A64_CTAS) k_energy_all64(AtomsDev A, Fix64Geom G, PbcDev pbc, CutDev cut, int n,
+__global__ void __launch_bounds__(ALL_I, A64_CTAS) k_energy_all64(AtomsDev A, Fix64Geom G, PbcDev pbc, CutDev cut, int n,
                                                         const int* __restrict__ fxs, const int* __restrict__ fxd,
-                                                        int units, double* part) {
-    __shared__ ulonglong4_32a sx[A64_J];
+                                                        long long units, double* part) {
+    __shared__ ulonglong4_32a sx[ALL_J];
     pair_kernel_begin();
     const double ileff = 1.0 / G.leff;
-    const int c0 = (n + A64_J - 1) / A64_J;      // columns chunks of row tile 0; each next tile has A64_I / A64_J fewer
-    constexpr int STEP = A64_I / A64_J;
+    const int c0 = (n + ALL_J - 1) / ALL_J;
     double sel = 0.0, svd = 0.0;
-    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
-        // row tile I: the last with I c0 - STEP I (I - 1) / 2 <= unit
-        auto first = [&](int I) { return (long long)I * c0 - (long long)STEP * I * (I - 1) / 2; };
-        const float b = c0 + 0.5f * STEP;
-        int I = (int)((b - sqrtf(fmaxf(b * b - 2.0f * STEP * unit, 0.0f))) / STEP);
-        while (I > 0 && first(I) > unit) I--;
-        while (first(I + 1) <= unit) I++;
-        const int jb = I * A64_I + (int)(unit - first(I)) * A64_J, je = min(n, jb + A64_J);
-        const int i = I * A64_I + threadIdx.x;
+    for (long long unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        int jb;
+        const int i = all_unit(unit, c0, jb) * ALL_I + threadIdx.x, je = min(n, jb + ALL_J);
         __syncthreads();
-        if (threadIdx.x < A64_J && jb + threadIdx.x < n) sx[threadIdx.x] = A.x64[jb + threadIdx.x];
+        if (threadIdx.x < ALL_J && jb + threadIdx.x < n) sx[threadIdx.x] = A.x64[jb + threadIdx.x];
         __syncthreads();
         if (i >= n) continue;
         const ulonglong4_32a a = A.x64[i];
@@ -1628,7 +1731,7 @@ int SingleEngine::init(const HostSystem& h) {
     term_start[n] = (int)term_data.size() / 2;
     // scratch: partial sums and the ΔE ticket
     ntile = (n + TILE - 1) / TILE;
-    size_t nparts = std::max<size_t>({(size_t)152 * A64_CTAS, (size_t)ntile * (ntile + 1) / 2, (size_t)MAX_MOVED + 1});
+    size_t nparts = std::max<size_t>({(size_t)152 * std::max(A64_CTAS, ALLMIX_CTAS), (size_t)ntile * (ntile + 1) / 2, (size_t)MAX_MOVED + 1});
     part_cap = nparts * 3 + 2 * 64 + 5 * BD_BLOCKS + 16;
     if ((rc = dalloc(&d_part, part_cap)) || (rc = dalloc(&d_ticket, 2)) ||
         (rc = dalloc(&d_maxrow, 2)))
@@ -2157,22 +2260,24 @@ int SingleEngine::energy(double ener[10]) {
     if (hs.cut == MCG_CUT_SWITCH) {
         nnb = launch_nonbonded(nbp);
     } else {
-        nnb = ntile * (ntile + 1) / 2;
+        const long long units = all_units(n);
         if (uses_fix64()) {
-            const long long tiles = (n + A64_I - 1) / A64_I, c0 = (n + A64_J - 1) / A64_J;
-            const int units = (int)(tiles * c0 - (A64_I / A64_J) * tiles * (tiles - 1) / 2);
-            nnb = std::min(units, 152 * A64_CTAS);
+            nnb = (int)std::min<long long>(units, 152 * A64_CTAS);
 #define MCG_ALL64(ISO_, TAB_)                                                                                         \
-    k_energy_all64<ISO_, TAB_><<<nnb, A64_I, 0, stream>>>(A, fix64, pbc, cut, n, d_fxs, d_fxd, units, nbp)
+    k_energy_all64<ISO_, TAB_><<<nnb, ALL_I, 0, stream>>>(A, fix64, pbc, cut, n, d_fxs, d_fxd, units, nbp)
             if (fix64.iso && ncls64) MCG_ALL64(true, true);
             else if (fix64.iso) MCG_ALL64(true, false);
             else if (ncls64) MCG_ALL64(false, true);
             else MCG_ALL64(false, false);
 #undef MCG_ALL64
-        } else if (hs.prec == MCG_PREC_FP64)
-            k_energy_all<PREC_F64><<<nnb, TILE, 0, stream>>>(A, n, pbc, cut, d_fxs, d_fxd, ntile, nbp);
-        else
-            k_energy_all<PREC_MIX><<<nnb, TILE, 0, stream>>>(A, n, pbc, cut, d_fxs, d_fxd, ntile, nbp);
+        } else if (hs.prec == MCG_PREC_FP64) {
+            nnb = ntile * (ntile + 1) / 2;
+            k_energy_all<<<nnb, TILE, 0, stream>>>(A, n, pbc, cut, d_fxs, d_fxd, ntile, nbp);
+        } else {
+            nnb = (int)std::min<long long>(units, 152 * ALLMIX_CTAS);
+            if (pbc.type != 0) k_energy_all_mix<true><<<nnb, ALL_I, 0, stream>>>(A, n, d_fxs, d_fxd, units, nbp);
+            else k_energy_all_mix<false><<<nnb, ALL_I, 0, stream>>>(A, n, d_fxs, d_fxd, units, nbp);
+        }
     }
     const BondedDev B = bonded();
     const int nterm = B.nb + B.na + B.nu + B.nd + B.ni;

@@ -112,6 +112,25 @@ def test_full_energy_with_exclusions():
 
 
 # boxes on both sides of twice the pairs' reach (the smallest accepted holds the cutoff sphere exactly)
+# The mixed-precision full energy at the edges of its units (128 rows by 32 columns), with and without
+# exclusions.  A pair's FP32 r^2 is off by some 6 units of 2^-24 and x^12 takes it to the sixth power:
+# 50 such units, 3e-6, with the products behind; the sums are float-float.
+@pytest.mark.parametrize("kind,n", [("argon", m) for m in (2, 31, 32, 33, 127, 128, 129, 160, 161, 257, 1000)] +
+                         [("water", m) for m in (1, 11, 43, 85, 173)])
+@pytest.mark.parametrize("box", ["cubic", "orbic", "none"])
+def test_full_energy_mixed(kind, n, box):
+    s = _near(_charged_argon(n, 41), 42) if kind == "argon" else systems.water_box(n, seed=43)
+    s.cut_mode = "full"
+    if box == "orbic":
+        s.box = (s.box[0], s.box[1] * 1.5, s.box[2] * 1.0625)
+    s.pbc_type = box
+    got = FFieldCUDA(s, "mixed", moves=False).getE10()
+    want = np.array(orc.Oracle(s, moves=False).energy())
+    assert np.all(np.isfinite(got)), got
+    tol = 4e-6 * _scale(s)
+    assert abs(got[3] - want[3]) <= tol and abs(got[4] - want[4]) <= tol, (got, want, tol)
+
+
 @pytest.mark.parametrize("L", [24.0, 24.002, 24.003, 25.0])
 @pytest.mark.parametrize("box", ["cubic", "orbic"])
 def test_switched_energy_smallest_boxes(L, box):
