@@ -1273,21 +1273,28 @@ __global__ void __launch_bounds__(256) k_energy_tail(BondedDev B, int nbd, Atoms
     __syncthreads();
     if (!s_last) return;   // uniform over the block
     __threadfence();
-    // components: nonbonded elec and vdw, 1-4 elec and vdw, the five bonded ones
-    for (int c = w; c < 9; c += blockDim.x >> 5) {
-        if (c < 2) pair_kernel_wait();
-        const double* src = c < 2 ? nb + c : (c < 4 ? s14 + (c - 2) : bd + (c - 4));
-        const int count = c < 2 ? nnb : (c < 4 ? n14b : nbd), step = c < 4 ? 2 : 5;
+    // The partial sums, eight loads in flight: 1-4 elec and vdw and the five bonded components by a warp
+    // each, then, when the pair kernel has ended, its two by four warps each: only those are left to do
+    // after it (up to 1,520 partial sums; a warp per component took 63 against 60 us for a full FP64
+    // energy of 3,000 atoms, 56.5 against 54.5 for a mixed one of a peptide box of 18,040).
+    auto sum = [](const double* src, int count, int step, int k0, int dk) {
         double v = 0.0;
-        for (int k = l; k < count; k += 32) v += __ldcg(src + (size_t)k * step);
-        v = warp_sum(v);
-        if (l == 0) sh[c][0] = v;
+#pragma unroll 8
+        for (int k = k0; k < count; k += dk) v += __ldcg(src + (size_t)k * step);
+        return warp_sum(v);
+    };
+    if (w < 7) {
+        const double v = w < 2 ? sum(s14 + w, n14b, 2, l, 32) : sum(bd + (w - 2), nbd, 5, l, 32);
+        if (l == 0) sh[2 + w][0] = v;
     }
+    pair_kernel_wait();
+    const double v = sum(nb + (w & 1), nnb, 2, 32 * (w >> 1) + l, 128);
+    if (l == 0) sh[w & 1][w >> 1] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
         const double K = CHGCHARMM * KCALTOIU;
-        double elec = K * sh[0][0];
-        double vdw = 4.0 * sh[1][0];
+        double elec = K * ((sh[0][0] + sh[0][1]) + (sh[0][2] + sh[0][3]));
+        double vdw = 4.0 * ((sh[1][0] + sh[1][1]) + (sh[1][2] + sh[1][3]));
         elec += K * sh[2][0];
         vdw += 4.0 * sh[3][0];
         double bond = sh[4][0], ang = sh[5][0], ub = sh[6][0], dihe = sh[7][0], impr = sh[8][0];
