@@ -1213,7 +1213,7 @@ __device__ __forceinline__ double tors_e(const TorsT& t, const CrdSrc& S, const 
 // pairs (the n14b blocks behind), and the sums.  It is launched as the pair kernel's programmatic
 // dependent: once every CTA of that has started (pair_kernel_begin) this one's begin too where they
 // fit, so the FP64 terms run beside the pair kernel, and only the last block to finish waits for the
-// pair kernel's partial sums.  That block adds all partials in a fixed order, a warp per component.
+// pair kernel's partial sums.  That block adds all partials in a fixed order.
 // Whole energy calls against separate kernels for bonded terms, 1-4 pairs and sums: 864 argon atoms
 // 29.6 -> 24.5 us, 12,288 water atoms in full mode 579 -> 566, 100,002 in FP64 577 -> 539.  The packed
 // group kernels of the mixed energy leave no registers beside them (2 x 256 threads of 128): 122 either way.
