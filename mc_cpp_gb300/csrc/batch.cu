@@ -1174,23 +1174,26 @@ __global__ void __launch_bounds__(256) k_batch_energy_res(const ChainDev* __rest
                                                           double* e_res, int64_t nres_total, const int* __restrict__ only,
                                                           const int* __restrict__ any) {
     if (any && !*any) return;   // a masked recompute with no chain to recompute
-    // A warp per residue r.  Lanes scan r's list 32 entries at a time; the entries q > r whose
-    // first atom lies within rc + 2 extents of r's are compacted into the warp's ring in shared
-    // memory, and each time 32 are pending every lane evaluates one residue pair: all atom pairs
-    // of (r, q), with r's atoms in registers.  Atom pairs beyond rc take r^2 = rc^2, where the
+    // A warp per residue r.  Lanes read r's list 64 entries at a time and compact the entries q > r,
+    // half of them, into a first ring in shared memory; those whose first atom lies within rc + 2
+    // extents of r's go on, 32 tested at a time, to a second one, and each time 32 are pending there
+    // every lane evaluates one residue pair: all atom pairs of (r, q), with r's atoms in registers.
+    // Bound by issue (73% of the slots): 64 water chains (1 M atoms) took 1003 us testing the list's
+    // 32 entries with half the lanes idle, 946 so.  Atom pairs beyond rc take r^2 = rc^2, where the
     // switch is exactly 0 (no divergent skip).  Coulomb and LJ are summed per lane as float-float
     // pairs (TwoSum), so the result does not depend on the list order beyond ~1e-14; the warp
     // sums in FP64.
     constexpr int A = APR ? APR : MAX_APR;
     constexpr int ERING = 64;
-    __shared__ int s_q[8][ERING];
+    constexpr int CRING = 128;           // fewer than 32 left and one step's 64 fit
+    __shared__ int s_q[8][ERING], s_c[8][CRING];
     CutDev cut;
     cut.mode = 1; cut.c2 = 0; cut.n2 = 0; cut.sw2 = 0;
     cut.c2f = G.c2f; cut.n2f = G.n2f; cut.sw2f = G.sw2f;
     const float c2 = G.c2f;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
-    int* ring = s_q[wib];
+    int *ring = s_q[wib], *cand = s_c[wib];
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t gr = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; gr < nres_total; gr += warps) {
         const int c = res_chain[gr];
@@ -1259,29 +1262,43 @@ __global__ void __launch_bounds__(256) k_batch_energy_res(const ChainDev* __rest
                 }
             }
         };
-        int head = 0, tail = 0;
-        for (int e0 = 0; e0 < nl; e0 += 32) {
-            const int e = e0 + lane;
-            const int q = e < nl ? (int)row[e] : -1;
+        int head = 0, tail = 0, chead = 0, ctail = 0;
+        for (int e0 = 0;;) {
+            while (chead - ctail < 32 && e0 < nl) {
+                const int e = e0 + lane;
+                const int q0 = e < nl ? (int)row[e] : -1, q1 = e + 32 < nl ? (int)row[e + 32] : -1;
+                const bool k0 = q0 > r, k1 = q1 > r;
+                const unsigned b0 = __ballot_sync(0xffffffffu, k0), b1 = __ballot_sync(0xffffffffu, k1);
+                if (k0) cand[(chead + __popc(b0 & lt_mask)) & (CRING - 1)] = q0;
+                chead += __popc(b0);
+                if (k1) cand[(chead + __popc(b1 & lt_mask)) & (CRING - 1)] = q1;
+                chead += __popc(b1);
+                e0 += 64;
+            }
+            __syncwarp();
+            const int nc = min(32, chead - ctail);
             bool keep = false;
-            if (q > r) {
+            int q = 0;
+            if (lane < nc) {
                 // first atoms farther than rc + 2 extents: no atom pair of the two residues is within rc
+                q = cand[(ctail + lane) & (CRING - 1)];
                 const uint4 q0 = Fc[q * apr];
                 const float dx = fdelta(pa[0].x, q0.x, Ls0, Ll0), dy = fdelta(pa[0].y, q0.y, Ls1, Ll1),
                             dz = fdelta(pa[0].z, q0.z, Ls2, Ll2);
                 keep = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= G.pair2;
             }
+            ctail += nc;
             const unsigned bal = __ballot_sync(0xffffffffu, keep);
             if (keep) ring[(head + __popc(bal & lt_mask)) & (ERING - 1)] = q;
             head += __popc(bal);
-            if (head - tail >= 32) {
-                __syncwarp();
-                eval(ring[(tail + lane) & (ERING - 1)]);
-                tail += 32;
-            }
             __syncwarp();
+            const bool last = e0 >= nl && chead == ctail;
+            if (head - tail >= 32 || last) {
+                if (lane < head - tail) eval(ring[(tail + lane) & (ERING - 1)]);
+                tail = min(head, tail + 32);
+            }
+            if (last && head == tail) break;
         }
-        if (lane < head - tail) eval(ring[(tail + lane) & (ERING - 1)]);
         __syncwarp();
         // float-float butterfly over the lanes (GB300's FP64 rate is 1/64 of FP32); lane 0 adds the
         // two parts in FP64

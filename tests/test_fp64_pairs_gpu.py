@@ -223,6 +223,22 @@ def test_batch_energy(sizes):
     _check_chains(B, chains)
 
 
+# The mixed recompute over residue lists: rows that start at an odd entry, lists of no entry to some 30
+# (dilute chains) and of hundreds, residue sizes 1 and 3 and both.  The pair terms' error is as in
+# test_full_energy_mixed; the switch polynomial's few units come on top of its 50.
+@pytest.mark.parametrize("kinds", [["argon"], ["water"], ["argon", "water"]])
+@pytest.mark.parametrize("cap", [0, 1023])
+def test_batch_energy_mixed_lists(kinds, cap):
+    chains = []
+    for kind in kinds:
+        for n, density in ((90, 2e-4), (200, 2e-3), (700, 0.0213)) if kind == "argon" else ((517, 0.0), (600, 0.0)):
+            chains.append(systems.argon_random(n, density, n) if kind == "argon" else systems.water_box(n, seed=n))
+    B = BatchChains(chains, seed=3, list_capacity=cap)
+    got, want = B.energy_mixed(), B.energy_fp64()
+    for k, s in enumerate(chains):
+        assert abs(got[k] - want[k]) <= 4e-6 * _scale(s), (k, got[k], want[k])
+
+
 def test_batch_energy_of_residues_wider_than_at_creation():
     chains = [systems.water_box(600, seed=1)]
     B = BatchChains(chains, seed=3)
