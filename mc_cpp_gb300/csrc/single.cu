@@ -77,8 +77,19 @@ struct Grid {
     int periodic;
 };
 
+// The five kernels of a list build follow each other as programmatic dependents, so a kernel's CTAs are
+// placed while the one before it runs and begin at its end; each touches memory only behind this.  With
+// that, the counters zeroed by the scan instead of two memsets, and the longest row written to mapped
+// memory by the last CTA instead of a copy, a whole update takes 33 us at 864 argon atoms (47 without),
+// 51 at 1,800 water atoms (70), 135 at 12,288 (146) and 650 at 100,002 (661).
+__device__ __forceinline__ void list_step() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __global__ void k_cell_assign(const double4_32a* __restrict__ pq, int n, PbcDev pbc, Grid g, int* cell_of,
                               int* cell_count) {
+    list_step();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double4_32a p = pq[i];
@@ -97,10 +108,12 @@ __global__ void k_cell_assign(const double4_32a* __restrict__ pq, int n, PbcDev 
 }
 
 // Exclusive scans by one block (cells are few) of the cell counts and of the cells' row-build tasks
-// (runs of at most `run` home atoms), carried together in the halves of a 64-bit sum.
-__global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int run, int* cell_start, int* cell_fill,
-                            int* task_start) {
+// (runs of at most `run` home atoms), carried together in the halves of a 64-bit sum.  The counts are zero
+// again afterwards, for the next build, and so are the row build's counters (max_row).
+__global__ void k_cell_scan(int* cell_count, int ncell, int run, int* cell_start, int* cell_fill, int* task_start, int* max_row) {
     __shared__ unsigned long long sw[32];
+    list_step();
+    if (threadIdx.x < 3) max_row[threadIdx.x] = 0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned long long carry = 0;
     for (int base = 0; base < ncell; base += blockDim.x) {
@@ -124,7 +137,7 @@ __global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int r
         }
         __syncthreads();
         const unsigned long long at = carry + (w ? sw[w - 1] : 0ull) + s - own;
-        if (i < ncell) { cell_start[i] = (int)(unsigned)at; cell_fill[i] = 0; task_start[i] = (int)(at >> 32); }
+        if (i < ncell) { cell_start[i] = (int)(unsigned)at; cell_fill[i] = 0; cell_count[i] = 0; task_start[i] = (int)(at >> 32); }
         carry += sw[31];
         __syncthreads();
     }
@@ -133,6 +146,7 @@ __global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int r
 
 __global__ void k_cell_scatter(const int* __restrict__ cell_of, int n, const int* __restrict__ cell_start,
                                int* cell_fill, int* cell_atoms) {
+    list_step();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int c = cell_of[i];
@@ -150,6 +164,7 @@ __global__ void k_cell_sort(const int* __restrict__ cell_start, const int* __res
     __shared__ uint8_t oct[SORT_MAX];
     int c = blockIdx.x;
     if (c >= ncell) return;
+    list_step();
     int b = cell_start[c], e = cell_start[c + 1], m = e - b;
     for (int k = threadIdx.x; k * run < m; k += blockDim.x) tasks[task_start[c] + k] = make_int2(c, b + k * run);
     if (m > SORT_MAX) {
@@ -270,13 +285,14 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
                                                                const int* __restrict__ home, const int2* __restrict__ tasks,
                                                                const int* __restrict__ xs,
                                                                const int* __restrict__ xd, int* nbr, int* nup, int* nlo,
-                                                               int* max_row) {
+                                                               int* max_row, int* longest_row) {
     __shared__ int2 s_range[ROW_WARPS][66];
     __shared__ uint4 s_ring[ROW_WARPS][ROW_RING];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
     int2* range = s_range[wib];
     uint4* ring = s_ring[wib];
+    list_step();
     const int ntask = task_start[ncell];
     // partners within maxspan in index are looked at; with frozen atoms about, every partner
     const unsigned span2 = lp.any_frozen ? 0xffffffffu : 2u * (unsigned)lp.maxspan;
@@ -490,6 +506,11 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
             }
     }
     if (lane == 0 && longest > 0) atomicMax(max_row, longest);
+    __syncthreads();
+    if (threadIdx.x == 0) {   // max_row[2] counts the CTAs done
+        __threadfence();
+        if (atomicAdd(max_row + 2, 1) == (int)gridDim.x - 1) *longest_row = atomicMax(max_row, 0);
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1741,7 +1762,7 @@ int SingleEngine::init(const HostSystem& h) {
     size_t nparts = std::max<size_t>({(size_t)152 * std::max(A64_CTAS, ALLMIX_CTAS), (size_t)ntile * (ntile + 1) / 2, (size_t)MAX_MOVED + 1});
     part_cap = nparts * 3 + 2 * 64 + 5 * BD_BLOCKS + 16;
     if ((rc = dalloc(&d_part, part_cap)) || (rc = dalloc(&d_ticket, 2)) ||
-        (rc = dalloc(&d_maxrow, 2)))
+        (rc = dalloc(&d_maxrow, 3)))
         return rc;
     CK(cudaMemsetAsync(d_ticket, 0, 2 * sizeof(unsigned), stream));
     // staging for moves: idx (sorted), xyz, terms
@@ -2181,7 +2202,7 @@ int SingleEngine::build_list() {
     int ncell = g.nc[0] * g.nc[1] * g.nc[2];
     const bool iso = g.periodic && hs.L[0] == hs.L[1] && hs.L[1] == hs.L[2];
     // home atoms that share a walk: four share more of it, two leave fewer warps idle in a small system.  A
-    // whole update with two, four and eight: 50, 58, 59 us (864 argon atoms), 72, 84, 97 (1,800 water
+    // whole update with two, four and eight, each some 14 us more than now: 50, 58, 59 us (864 argon atoms), 72, 84, 97 (1,800 water
     // atoms), 170, 159, 174 (12,288), 359, 305, 338 (36,000), 948, 761, 753 (100,002), so the line is at 8,192
     const int run = !g.periodic || n < 8192 ? 2 : 4;
     int rc;
@@ -2191,6 +2212,7 @@ int SingleEngine::build_list() {
             if (*p) cudaFree(*p);
             if ((rc = dalloc(p, ncell + 1))) return rc;
         }
+        CK(cudaMemsetAsync(d_cell_count, 0, sizeof(int) * (ncell + 1), stream));   // every scan leaves it zero
         if (d_tasks) cudaFree(d_tasks);
         if ((rc = dalloc(&d_tasks, (size_t)n / 2 + ncell + 1))) return rc;
         ncell_cap = ncell;
@@ -2220,26 +2242,34 @@ int SingleEngine::build_list() {
         lp.reach2 = (float)(lp.cutnb2 * (1.0 + 1e-5) + 1e-2);
     }
     for (int attempt = 0; attempt < 3; attempt++) {
-        CK(cudaMemsetAsync(d_cell_count, 0, sizeof(int) * ncell, stream));
-        CK(cudaMemsetAsync(d_maxrow, 0, 2 * sizeof(int), stream));
-        k_cell_assign<<<(n + 255) / 256, 256, 0, stream>>>(d_pq, n, pbc, g, d_cell_of, d_cell_count);
-        k_cell_scan<<<1, 1024, 0, stream>>>(d_cell_count, ncell, run, d_cell_start, d_cell_fill, d_task_start);
-        k_cell_scatter<<<(n + 255) / 256, 256, 0, stream>>>(d_cell_of, n, d_cell_start, d_cell_fill, d_cell_atoms);
-        k_cell_sort<<<ncell, 128, 0, stream>>>(d_cell_start, d_task_start, ncell, run, d_fx, g, d_cell_atoms, d_cell_pos, d_home, d_tasks);
+        cudaLaunchAttribute after[1];
+        after[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        after[0].val.programmaticStreamSerializationAllowed = 1;
+        auto launch = [&](auto kernel, int blocks, int threads, auto... args) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(blocks);
+            cfg.blockDim = dim3(threads);
+            cfg.stream = stream;
+            cfg.attrs = after;
+            cfg.numAttrs = 1;
+            return cudaLaunchKernelEx(&cfg, kernel, args...);
+        };
+        CK(launch(k_cell_assign, (n + 255) / 256, 256, d_pq, n, pbc, g, d_cell_of, d_cell_count));
+        CK(launch(k_cell_scan, 1, 1024, d_cell_count, ncell, run, d_cell_start, d_cell_fill, d_task_start, d_maxrow));
+        CK(launch(k_cell_scatter, (n + 255) / 256, 256, d_cell_of, n, d_cell_start, d_cell_fill, d_cell_atoms));
+        CK(launch(k_cell_sort, ncell, 128, d_cell_start, d_task_start, ncell, run, d_fx, g, d_cell_atoms, d_cell_pos, d_home, d_tasks));
         const int blocks = std::min((n / run + ncell + ROW_WARPS - 1) / ROW_WARPS, 152 * ROW_CTAS);
 #define MCG_ROWS(A_, P_, I_)                                                                                          \
-    k_build_rows<A_, P_, I_><<<blocks, 32 * ROW_WARPS, 0, stream>>>(d_pq, d_cell_pos, d_frozen, pbc, g, lp, d_cell_start, \
-                                                                d_task_start, ncell, d_home, d_tasks, d_xs, d_xd, d_nbr, d_nup, d_nlo, d_maxrow)
+    CK(launch(k_build_rows<A_, P_, I_>, blocks, 32 * ROW_WARPS, d_pq, d_cell_pos, d_frozen, pbc, g, lp, d_cell_start, \
+              d_task_start, ncell, d_home, d_tasks, d_xs, d_xd, d_nbr, d_nup, d_nlo, d_maxrow, (int*)(d_map + 24)))
         if (!g.periodic) MCG_ROWS(2, false, false);
         else if (iso && run == 4) MCG_ROWS(4, true, true);
         else if (iso) MCG_ROWS(2, true, true);
         else if (run == 4) MCG_ROWS(4, true, false);
         else MCG_ROWS(2, true, false);
 #undef MCG_ROWS
-        CK(cudaGetLastError());
-        int maxrow = 0;
-        CK(cudaMemcpyAsync(&maxrow, d_maxrow, sizeof(int), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
+        const int maxrow = *(volatile int*)(h_map + 24);
         last_max_row = maxrow;
         if (maxrow <= cap) {
             clp_dirty = uses_pair_variants();   // the cluster form follows on first use

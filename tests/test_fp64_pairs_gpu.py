@@ -266,6 +266,21 @@ def test_verlet_rows(kind, n):
     assert all(np.array_equal(a, np.sort(b)) for a, b in zip(rows, want, strict=True))
 
 
+# builds after each other on one handle, without a box: the cell grid grows and shrinks between them and
+# the rows outgrow their capacity; the counters that one build leaves behind are the next one's
+def test_verlet_rows_of_successive_builds():
+    s = _near(_charged_argon(1200, 17), 18)
+    s.pbc_type = "none"
+    xyz = s.coords()
+    ff = FFieldCUDA(s, "fp64", moves=False)
+    for scale in (1.0, 1.9, 0.6, 1.2, 1.2):
+        s.set_coords(xyz * scale)
+        ff.setCoords(s.coords())
+        ff.askListUpdate(0)
+        want = orc.Oracle(s, moves=False).verlet_rows()
+        assert all(np.array_equal(a, np.sort(b)) for a, b in zip(ff.pairlist(), want, strict=True))
+
+
 def _bonded_chain(n, seed, angles, torsion_kinds):
     """n charged atoms in a chain whose angles and torsions take the given values (degrees), with terms
     referred to other values: from no deviation to the whole circle."""
