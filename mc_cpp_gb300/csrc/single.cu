@@ -2590,7 +2590,8 @@ __device__ __forceinline__ double rp_pair(double4_32a a, double4_32a b, double2 
 // 256-thread CTA (its ~200 dE terms at two warps per scheduler), 89.9k with the cluster and the
 // words read from global memory, 94.8k with them in shared memory, 99.9k with the fifth warp.
 // In runs of 500 steps, 92k so far, 107k with the FP64 operations of ref64_mic and rsqrt64, 142k with one
-// barrier and one sum a step, 152k with the terms off the fifth warp's scheduler and its draw used.
+// barrier and one sum a step, 152k with the terms off the fifth warp's scheduler and its draw used, 163k with
+// shorter list builds, 169k with the words and the state in page-locked memory (three copies a launch before).
 constexpr int RP_CL = 8;
 constexpr int RP_NT = 128;
 constexpr int RP_TRIES = 8;
@@ -2608,7 +2609,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
     k_replay(AtomsDev A, double4_32a* pq, PbcDev pbc, CutDev cut, const int* __restrict__ nbr,
              const int* __restrict__ nup, const int* __restrict__ nlo, int cap, const int* __restrict__ c14s,
              const int* __restrict__ c14d, ReplayTables T, const uint32_t* __restrict__ words, long long nwords,
-             ReplayState* st, int s0, int s1, double beta) {
+             const __grid_constant__ ReplayState init, ReplayState* st, int s0, int s1, double beta) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ ReplayState S;
@@ -2642,7 +2643,7 @@ __global__ void __cluster_dims__(RP_CL, 1, 1) __launch_bounds__(RP_NT + RP_SPEC)
     // this thread's place in the order the terms are dealt: CTAs first, then the lanes of warps 1 and 2, then
     // those of 3 and 0.  Up to 512 terms (255 partners of one atom) leave warp 0's scheduler to the fifth warp
     const int gslot = rank + RP_CL * (2 * lane + (warp == 1 || warp == 2 ? warp - 1 : 64 + (warp == 0)));
-    if (tid == 0) S = *st;
+    if (tid == 0) S = init;
     cluster.sync();   // every CTA of the cluster is running before any writes into its shared memory
     for (int step = s0 + 1; step <= s1; step++) {
         if (warp == 0) {
@@ -2883,34 +2884,37 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
     first.push_back((int)ranges.size() / 2);
     S.etot = *etot;
     constexpr long long W = RP_WORDS;        // random words per launch
-    int* d_first = nullptr;
-    int* d_ranges = nullptr;
-    uint32_t* d_words = nullptr;
-    ReplayState* d_st = nullptr;
+    // In the page-locked staging memory: a launch's words and the state it leaves, which the kernel reads
+    // and writes there (few and once a launch), and the instance tables on their way to the device; tables
+    // larger than it get their own memory.
+    uint32_t* const w = (uint32_t*)h_stage;
+    ReplayState* const left = (ReplayState*)(w + W);
+    static_assert(sizeof(ReplayState) <= 256, "place of the tables");
+    const size_t tab_at = sizeof(uint32_t) * W + 256, nfirst = first.size();
+    first.insert(first.end(), ranges.begin(), ranges.end());
+    const size_t tab_bytes = sizeof(int) * first.size();
+    pending_m = 0;                           // the staged proposal makes way
+    int* d_tab = nullptr;
     int rc = MCG_OK;
     auto done = [&](int r) {
         // the run keeps pq current; the mirrors, which it does not read, follow here
         k_fix_all<<<(n + 255) / 256, 256, 0, stream>>>(n, d_pq, d_cls_of, d_fx, d_x64, fix64.sh, pbc);
         launches++;
         if (cudaStreamSynchronize(stream) != cudaSuccess && r == MCG_OK) r = fail(MCG_ECUDA, "device run: mirrors");
-        if (d_first) cudaFree(d_first);
-        if (d_ranges) cudaFree(d_ranges);
-        if (d_words) cudaFree(d_words);
-        if (d_st) cudaFree(d_st);
+        if (d_tab) cudaFree(d_tab);
         return r;
     };
-    if ((rc = dalloc(&d_first, first.size())) || (rc = dalloc(&d_ranges, std::max<size_t>(1, ranges.size()))) ||
-        (rc = dalloc(&d_words, (size_t)W)) || (rc = dalloc(&d_st, 1)))
-        return done(rc);
-    if (cudaMemcpyAsync(d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess ||
-        (!ranges.empty() &&
-         cudaMemcpyAsync(d_ranges, ranges.data(), sizeof(int) * ranges.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess))
+    const bool staged = tab_at + tab_bytes <= stage_bytes;
+    if (!staged && (rc = dalloc(&d_tab, first.size()))) return done(rc);
+    int* const tab = staged ? (int*)d_stage : d_tab;
+    if (staged) memcpy((char*)h_stage + tab_at, first.data(), tab_bytes);
+    if (cudaMemcpyAsync(tab, staged ? (const void*)((char*)h_stage + tab_at) : first.data(), tab_bytes, cudaMemcpyHostToDevice, stream) !=
+        cudaSuccess)
         return done(fail(MCG_ECUDA, "device run: table upload"));
-    T.inst_first = d_first;
-    T.ranges = d_ranges;
-    T.ninst_all = (int)first.size();
+    T.inst_first = tab;
+    T.ranges = tab + nfirst;
+    T.ninst_all = (int)nfirst;
     T.nranges = (int)ranges.size() / 2;
-    std::vector<uint32_t> w((size_t)W);
     std::vector<uint32_t> stash;     // the generator's next words, drawn while the previous launch ran
     size_t stash_at = 0;
     long long filled = 0;
@@ -2918,26 +2922,24 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
     while (step < nsteps) {
         // the words not consumed yet, then the generator's next ones (from the stash first)
         const long long keep = filled - S.cursor;
-        if (keep > 0 && S.cursor > 0) std::memmove(w.data(), w.data() + S.cursor, sizeof(uint32_t) * (size_t)keep);
+        if (keep > 0 && S.cursor > 0) std::memmove(w, w + S.cursor, sizeof(uint32_t) * (size_t)keep);
         filled = std::max(0LL, keep);
-        while (filled < W) w[(size_t)filled++] = stash_at < stash.size() ? stash[stash_at++] : gen();
+        const int s1 = std::min(nsteps, (step / 50 + 1) * 50);     // up to the next list update
+        // a step takes 17 words on average; a launch that ran out of them goes on with a full buffer
+        const long long need = S.status == 1 ? W : std::min(W, 32LL * (s1 - step) + 512);
+        while (filled < need) w[filled++] = stash_at < stash.size() ? stash[stash_at++] : gen();
         S.cursor = 0;
         S.status = 0;
-        const int s1 = std::min(nsteps, (step / 50 + 1) * 50);     // up to the next list update
-        if (cudaMemcpyAsync(d_words, w.data(), sizeof(uint32_t) * (size_t)W, cudaMemcpyHostToDevice, stream) != cudaSuccess ||
-            cudaMemcpyAsync(d_st, &S, sizeof S, cudaMemcpyHostToDevice, stream) != cudaSuccess)
-            return done(fail(MCG_ECUDA, "device run: upload"));
         k_replay<<<RP_CL, RP_NT + RP_SPEC, 0, stream>>>(atoms(), d_pq, pbc, cut, d_nbr, d_nup, d_nlo, cap, d_c14s, d_c14d, T,
-                                              d_words, W, d_st, step, s1, beta);
+                                              w, filled & ~3LL, S, left, step, s1, beta);
         launches++;
-        // while the launch runs: the next W words of the generator, in order, for the next buffer
+        // while the launch runs: the generator's next words, in order, for the next buffer
         stash.erase(stash.begin(), stash.begin() + (long)stash_at);
         stash_at = 0;
-        while ((long long)stash.size() < W) stash.push_back(gen());
-        if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpyAsync(&S, d_st, sizeof S, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-            cudaStreamSynchronize(stream) != cudaSuccess)
+        while ((long long)stash.size() < need) stash.push_back(gen());
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)
             return done(fail(MCG_ECUDA, "device run: replay kernel"));
+        memcpy(&S, left, sizeof S);
         if (S.status == 2) return done(fail(MCG_ENOTSUP, "device run: a move of more than 64 atoms"));
         step = S.steps_done;
         if (S.status == 0 && step % 50 == 0) {
@@ -2960,8 +2962,8 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
 
 int SingleEngine::commit() {
     if (pending_m <= 0) return fail(MCG_EINVAL, "no pending proposal to commit");
-    // the pending proposal is still staged on the device: only delta_e writes d_stage, and each
-    // delta_e call replaces the pending proposal.  Stream order puts the update before any later
+    // the pending proposal is still staged on the device: only delta_e and a device run write d_stage,
+    // and each replaces the pending proposal.  Stream order puts the update before any later
     // call's work, so the host does not wait for it.
     const int* didx = (const int*)d_stage;
     const double* dxyz = (const double*)((char*)d_stage + pending_off_xyz);
