@@ -727,6 +727,7 @@ int GroupPairs::build(cudaStream_t st, const int* rows, const int* lens, int cap
     GK(cudaMemsetAsync(d_misc, 0, 3 * sizeof(unsigned long long), st));
     const int blocks = std::min((ngroup + GB_WARPS - 1) / GB_WARPS, 152 * 16);
     // a row's work on the bitmap grows with the number of groups, so the hash table keeps the largest systems
+    // (list update and energy: 1241 us against 1505 at 33,334 groups, 2564 against 2785 at 65,000)
     if (ngroup <= GBM_GROUPS) {
         const int words = (ngroup + 1023) / 1024 * 32;
         const size_t smem = (size_t)GB_WARPS * sizeof(unsigned) * (words + words / 2 + 2 * GH_MAX);
