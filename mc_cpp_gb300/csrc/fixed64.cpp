@@ -44,8 +44,7 @@ Fix64Geom fix64_geom(const double L[3], double rc, double ron) {
     const long double c2 = (long double)rc * rc, d = c2 - (long double)ron * ron;
     G.c2 = clamp64(c2 / l2 * TWO64L);
     const long double dq = d / l2 * TWO64L;            // rc^2 - ron^2 in units of 2^-64
-    const long double span = std::min(c2 / l2 * TWO64L, dq * (1.0L + 0.00390625L));
-    while (G.sD < 63 && std::ldexp(span, G.sD + 1) < TWO64L) G.sD++;
+    while (G.sD < 63 && std::ldexp(dq, G.sD + 1) < TWO64L) G.sD++;
     G.rD = clamp64(std::ldexp(1.0L, 126) / std::ldexp(dq, G.sD));
     G.in2 = (float)(ron * ron * (1.0 - 1e-4));
     G.out2 = (float)(rc * rc * (1.0 + 1e-4));

@@ -19,7 +19,7 @@
 //   at most 2^-55 and 2^-54 in its rounding to a double (12 multiplications of a rounded quotient reach
 //   2^-49).  Rounding s^6 and s^12 to doubles instead would be an error common to all pairs of two classes.
 // * The switch is v^2 (3 - 2 v) with v = (rc^2 - u) / (rc^2 - ron^2) clamped to [0, 1] (the
-//   reference's polynomial in another variable), to 2^-57 of itself (beside u's own last place).
+//   reference's polynomial in another variable), to 2^-56 of itself (beside u's own last place).
 // Totals against 113-bit sums, RMS over eight boxes each (FP64 pair terms in brackets): 2,400 water atoms
 // switched, Coulomb 5.3e-16 (9.3e-16), Lennard-Jones 1.1e-16 (2.4e-16); 1,200 in full mode 1.4e-16
 // (3.2e-16) and 1.0e-16 (3.0e-16); 2,000 argon atoms 0.6e-16 (1.0e-16).
@@ -133,7 +133,8 @@ __device__ __forceinline__ bool fix64_terms(const Fix64Geom& G, const Fix64Dist&
     ys = __longlong_as_double((long long)(((unsigned long long)(1022 + k) << 52) + ((Y + 512) >> 10)));
     ws = w;
     if (sw) {
-        // v and v^2 with a shift of their own, so the switch keeps its relative accuracy near rc
+        // v and v^2 with a shift of their own, so the switch keeps its relative accuracy near rc.  rD is at
+        // most 2^63 (fix64_geom), so v stays below 2^63 and v << 1 within 64 bits, at every box length
         const unsigned long long uh = (unsigned long long)u.hi << 32 | u.mid;
         const unsigned long long dl = uh < G.c2 ? G.c2 - uh : 0ull;
         int ld = __clzll((long long)dl);

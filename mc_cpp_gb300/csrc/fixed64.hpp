@@ -16,8 +16,9 @@ struct Fix64Geom {
     int up;                  // displacement = high half of (difference x ratio) << up: 2, or 1 when halved
     int64_t ratio[3];        // L[k] / max(L) in units of 2^-62
     uint64_t c2;             // (rc / Leff)^2 in units of 2^-64
-    int sD;                  // (c2 - u) << sD fits 64 bits for every u above ron^2 (1 - 2^-8)
-    uint64_t rD;             // 2^126 / ((rc^2 - ron^2) / Leff^2 << sD): v = (rc^2 - u) / (rc^2 - ron^2)
+    int sD;                  // rc^2 - ron^2, in units of 2^-64 Leff^2, shifted left by sD has bit 63 for its leading bit
+    uint64_t rD;             // 2^126 / ((rc^2 - ron^2) / Leff^2 << sD), at most 2^63, so that a normalised
+                             // rc^2 - u times it stays below 2^63: v = (rc^2 - u) / (rc^2 - ron^2)
     float Ls[3], Ll[3];      // L / 2^32 as float-float: FP32 displacement from the high words
     float in2, out2;         // FP32 r^2 below in2 lies inside ron, above out2 beyond rc (A^2)
     double leff;

@@ -625,7 +625,7 @@ __device__ __forceinline__ void pair64_params(const AtomsDev& A, double ileff, i
 //    the cutoff, and the switch is formed only for the pairs that need it;
 //  - a pair's distance and powers are 64-bit integers (fixed64.cuh), with 3 FP64 operations.
 // The FP32 placement has a margin of 1e-4 in r^2; a pair placed within rc that lies beyond takes a
-// switch factor of exactly 0, and one placed outside ron a factor of 1 to 2^-58.
+// switch factor of exactly 0, and one placed outside ron that lies inside a factor of 1 to 2^-56.
 // The rings are drained at one place in the code, after a chunk of E64_U entries per lane: with the
 // evaluation inlined behind every entry the kernel stalled on instruction fetch (0.69 against 0.61 ms on
 // the 100,002-atom water box).  That box takes 0.53 ms, 69 G pairs/s (4.2 ms with the pair terms in

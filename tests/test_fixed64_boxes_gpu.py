@@ -1,0 +1,68 @@
+"""FP64 switched totals over the normalisation of the switch's constants, against the FP64 oracle.
+
+(rc^2 - ron^2) in units of the box's squared length is held as a normalised 64-bit mantissa, so box lengths
+that put it just below a power of two are where the integer switch is tightest: 26.54, 37.58, 53.0976 (the
+5,000-molecule water box), 75.15 and 106.25 A at 12 and 10 A.  Tolerance as in test_fp64_pairs_gpu: a term
+carries at most about 40 roundings on either side, a sum as many as its longest chain of additions.
+"""
+import numpy as np
+import pytest
+
+import oracle as orc
+from mc_cpp_gb300 import build, native, systems
+from mc_cpp_gb300.engine import BatchChains, FFieldCUDA
+
+pytestmark = pytest.mark.gpu
+REL = 1e-13
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    build.build()
+    orc.build()
+    if native.lib().mcg_device_count() < 1:
+        pytest.fail("no CUDA device visible to libmcgpu.so")
+
+
+def _atoms(L, box, n=3000, charges=None):
+    """n charged atoms shaken off a lattice in a box of length L (times 1.25 along y for "orbic")."""
+    s = systems.argon_random(n, n / L ** 3, 7)
+    rng = np.random.default_rng(8)
+    s.q = rng.normal(0.0, 0.3, n) if charges is None else np.full(n, charges)
+    s.box = (L, L, L)
+    s.set_coords(s.coords() + rng.uniform(-0.3, 0.3, (n, 3)))
+    if box == "orbic":
+        s.pbc_type = "orbic"
+        s.box = (L, L * 1.25, L)
+    return s
+
+
+def _oracle(s):
+    """The oracle's components, and the scale of its sums: the same system with all charges positive."""
+    t = s.copy()
+    t.q = np.abs(t.q)
+    e, a = np.array(orc.Oracle(s, moves=False).energy()), orc.Oracle(t, moves=False).energy()
+    return e, abs(a[3]) + 4 * abs(a[4])
+
+
+LENGTHS = [26.54, 37.58, 53.0976, 75.15, 106.25]
+
+
+@pytest.mark.parametrize("L", LENGTHS)
+@pytest.mark.parametrize("box", ["cubic", "orbic"])
+def test_switched_energy(L, box):
+    s = _atoms(L, box, 900 if L < 30 else 3000)
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    want, scale = _oracle(s)
+    assert abs(got[3] - want[3]) <= REL * scale and abs(got[4] - want[4]) <= REL * scale, (got, want, scale)
+
+
+@pytest.mark.parametrize("box", ["cubic", "orbic"])
+def test_batch_total(box):
+    chains = [_atoms(L, box, 900 if L < 30 else 1500, charges=0.2) for L in LENGTHS]
+    got = BatchChains(chains, dmax_trn=0.05, dmax_rot=1.0, seed=1).energy_fp64()
+    for e, s in zip(got, chains):
+        want, scale = _oracle(s)
+        # a batch holds box fractions to 2^-64 and converts the coordinates once: 2^-53 L of a coordinate,
+        # which moves a pair's x^12 by 12 sqrt(3) 2^-52 L / r; the closest pairs here are 1.2 A apart
+        assert abs(e - want[3] - want[4]) <= (2 * REL + 21 * 2.0 ** -52 * s.box[0] / 1.2) * scale, (e, want, scale)
