@@ -1139,10 +1139,11 @@ __global__ void __launch_bounds__(256) k_batch_energy64(const ChainDev* __restri
                         const double ex = (double)(long long)(b.x - a.x) * (C.L[0] * (1.0 / TWO64)),
                                      ey = (double)(long long)(b.y - a.y) * (C.L[1] * (1.0 / TWO64)),
                                      ez = (double)(long long)(b.z - a.z) * (C.L[2] * (1.0 / TWO64));
-                        const double y = rsqrt64(ex * ex + ey * ey + ez * ez) * G.leff;
+                        const double r2 = ex * ex + ey * ey + ez * ez, y = rsqrt64(r2) * G.leff;
                         const double x2 = (t.z ? fix64_norm_to_double(t.z, (int)t.w - 64) : 0.0) * (y * y), x6 = x2 * x2 * x2;
-                        sel = fma(qq, y, sel);
-                        svd = fma(ee, fma(x6, x6, -x6), svd);
+                        const double v = fmin(fmax((G.rc2 - r2) * G.id2, 0.0), 1.0), S = sw ? v * v * fma(-2.0, v, 3.0) : 1.0;
+                        sel = fma(qq, y * S, sel);
+                        svd = fma(ee, fma(x6, x6, -x6) * S, svd);
                     }
                 }
                 if (sw) tail1 = min(tail1 + 32, head1);

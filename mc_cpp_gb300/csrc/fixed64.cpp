@@ -46,6 +46,8 @@ Fix64Geom fix64_geom(const double L[3], double rc, double ron) {
     const long double dq = d / l2 * TWO64L;            // rc^2 - ron^2 in units of 2^-64
     while (G.sD < 63 && std::ldexp(dq, G.sD + 1) < TWO64L) G.sD++;
     G.rD = clamp64(std::ldexp(1.0L, 126) / std::ldexp(dq, G.sD));
+    G.rc2 = rc * rc;
+    G.id2 = 1.0 / (G.rc2 - ron * ron);
     G.in2 = (float)(ron * ron * (1.0 - 1e-4));
     G.out2 = (float)(rc * rc * (1.0 + 1e-4));
     return G;

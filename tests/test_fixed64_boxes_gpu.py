@@ -66,3 +66,19 @@ def test_batch_total(box):
         # a batch holds box fractions to 2^-64 and converts the coordinates once: 2^-53 L of a coordinate,
         # which moves a pair's x^12 by 12 sqrt(3) 2^-52 L / r; the closest pairs here are 1.2 A apart
         assert abs(e - want[3] - want[4]) <= (2 * REL + 21 * 2.0 ** -52 * s.box[0] / 1.2) * scale, (e, want, scale)
+
+
+# Pairs closer than the 64-bit form reaches (some 2^-15 of the longest box length) in a long box, with the
+# switch beginning at 0: it leaves 3 (r / rc)^4, 6e-9, of a pair's energy.  The pairs lie along x, whose
+# coordinates the masters hold to 2^-53 of 30 A.
+@pytest.mark.parametrize("cuton", [0.0, 10.0])
+def test_batch_total_close_pairs(cuton):
+    n, r, L = 40, 0.08, (30.0, 30.0, 3000.0)
+    s = systems.argon_random(n, 0.0213, 3)
+    s.pbc_type, s.box, s.cuton = "orbic", L, cuton
+    s.q, s.eps = np.full(n, 0.2), np.zeros(n)
+    z = np.repeat(np.arange(n // 2) * 140.0 - 1400.0, 2)
+    s.set_coords(np.stack([np.tile([3.0, 3.0 + r], n // 2), np.zeros(n), z], 1))
+    got = BatchChains([s], dmax_trn=0.05, dmax_rot=1.0, seed=1).energy_fp64()[0]
+    want, scale = _oracle(s)
+    assert abs(got - want[3] - want[4]) <= (2 * REL + 2 * 2.0 ** -52 * 30.0 / r) * scale, (got, want, scale)
