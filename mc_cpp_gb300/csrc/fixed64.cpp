@@ -11,6 +11,18 @@ namespace {
 constexpr long double TWO64L = 18446744073709551616.0L;
 
 uint64_t clamp64(long double v) { return v >= TWO64L ? ~0ull : (v <= 0.0L ? 0ull : (uint64_t)v); }
+
+// A displacement's component is off by the positions' unit, or by the units that its scaling drops.  Pairs so
+// close that this passes 2^-53 of their distance are left to FP64, whose differences of nearby coordinates
+// are exact: r^-12 is off by some 5 times that share (RMS), 6e-16, where the FP64 form's is off by 1.1e-15.
+// A squared distance with e leading zero bits, e even, is at least 2^-(e + 2) of Leff^2.  Cubic boxes of 100 A
+// switched, 60 A in full mode: 0.05 and 0.06 A; a box of 10,000 A: 4.9 A.
+int close_limit(const Fix64Geom& G, double lmax) {
+    const double unit = std::ldexp(std::max(lmax, G.iso ? G.leff : std::ldexp(G.leff, G.up)), -64);
+    int e = 28;
+    while (e >= 0 && std::ldexp(G.leff, -(e / 2 + 1)) < std::ldexp(unit, 53)) e -= 2;
+    return e;
+}
 }  // namespace
 
 Fix64Geom fix64_geom_full(const double L[3]) {
@@ -25,6 +37,7 @@ Fix64Geom fix64_geom_full(const double L[3]) {
         G.Ls[k] = (float)ls;
         G.Ll[k] = (float)(ls - (double)G.Ls[k]);
     }
+    G.emax = close_limit(G, lmax);
     return G;
 }
 
@@ -40,6 +53,7 @@ Fix64Geom fix64_geom(const double L[3], double rc, double ron) {
     } else {
         G.iso = 0;   // halved, by the general form
     }
+    G.emax = close_limit(G, lmax);
     const long double l2 = (long double)G.leff * (long double)G.leff;
     const long double c2 = (long double)rc * rc, d = c2 - (long double)ron * ron;
     G.c2 = clamp64(c2 / l2 * TWO64L);

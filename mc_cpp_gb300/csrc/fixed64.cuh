@@ -23,7 +23,8 @@
 // Totals against 113-bit sums, RMS over eight boxes each (FP64 pair terms in brackets): 2,400 water atoms
 // switched, Coulomb 5.3e-16 (9.3e-16), Lennard-Jones 1.1e-16 (2.4e-16); 1,200 in full mode 1.4e-16
 // (3.2e-16) and 1.0e-16 (3.0e-16); 2,000 argon atoms 0.6e-16 (1.0e-16).
-// A pair closer than about Leff 2^-14 (some 2e-3 A) does not fit the shift and is left to the caller.
+// A pair closer than some 2^-11 of a box length (0.05 A in a box of 100 A; the geometry's emax), where the
+// positions' unit would tell, is left to the caller.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -105,7 +106,7 @@ __device__ __forceinline__ Fix64Dist fix64_dist2(const Fix64Geom& G, const ulong
 }
 
 // w = (s / r)^6 for s^2 = ms 2^(es - 64) Leff^2 (ms of at least 2^63, or 0), and ys = Leff / r and ws = w
-// times the switch factor (1 unless sw, 0 beyond rc).  False when the pair is too close for the shift.
+// times the switch factor (1 unless sw, 0 beyond rc).  False when the pair is too close for the form.
 __device__ __forceinline__ bool fix64_terms(const Fix64Geom& G, const Fix64Dist& u, bool sw, unsigned long long ms, int es,
                                             double& ys, double& w, double& ws) {
     const int e2 = __clz((int)u.hi) & ~1;
@@ -147,7 +148,7 @@ __device__ __forceinline__ bool fix64_terms(const Fix64Geom& G, const Fix64Dist&
         ys *= s;
         ws *= s;
     }
-    return e2 <= 28;
+    return e2 <= G.emax;
 }
 
 }  // namespace mcg

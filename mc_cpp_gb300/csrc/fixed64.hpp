@@ -21,6 +21,7 @@ struct Fix64Geom {
                              // rc^2 - u times it stays below 2^63: v = (rc^2 - u) / (rc^2 - ron^2)
     float Ls[3], Ll[3];      // L / 2^32 as float-float: FP32 displacement from the high words
     float in2, out2;         // FP32 r^2 below in2 lies inside ron, above out2 beyond rc (A^2)
+    int emax;                // pairs whose squared distance has more leading zero bits are left to FP64
     double rc2, id2;         // rc^2 and 1 / (rc^2 - ron^2), for the pairs left to FP64
     double leff;
 };

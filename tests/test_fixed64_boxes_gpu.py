@@ -5,6 +5,9 @@ that put it just below a power of two are where the integer switch is tightest: 
 5,000-molecule water box), 75.15 and 106.25 A at 12 and 10 A.  Tolerance as in test_fp64_pairs_gpu: a term
 carries at most about 40 roundings on either side, a sum as many as its longest chain of additions.
 """
+from decimal import Decimal, localcontext
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
@@ -82,3 +85,37 @@ def test_batch_total_close_pairs(cuton):
     got = BatchChains([s], dmax_trn=0.05, dmax_rot=1.0, seed=1).energy_fp64()[0]
     want, scale = _oracle(s)
     assert abs(got - want[3] - want[4]) <= (2 * REL + 2 * 2.0 ** -52 * 30.0 / r) * scale, (got, want, scale)
+
+
+# One pair in boxes of up to a million A: what the box fractions' unit is worth grows with the box, so close
+# pairs are left to FP64 there.  The exact value in rationals; beside it the FP64 form carries 3 roundings of r^2
+# (half of each counts), 1 of 1/r, 2 of x = s / r, 12 times those, and 6 more: 60, with the switch's own
+# (8 roundings, none of them cancelling at these distances) and the totals' factors 72.
+@pytest.mark.parametrize("L", [30.0, 100.0, 1e3, 1e4, 1e5, 1e6])
+@pytest.mark.parametrize("shape", ["cubic", "slab"])
+@pytest.mark.parametrize("cut", ["full", "switch"])
+def test_one_pair_in_a_large_box(L, shape, cut):
+    K, rng = 332.0716 * 418.4, np.random.default_rng(11)
+    for r in (1.1, 1.7, 2.5, 3.3, 4.1, 10.7):
+        s = systems.argon_random(2, 0.0213, 3)
+        v = rng.normal(size=3)
+        a = rng.uniform(-3.0, 3.0, 3)
+        s.set_coords(np.stack([a, a + r * v / np.linalg.norm(v)]))
+        s.pbc_type, s.box = ("cubic", (L, L, L)) if shape == "cubic" else ("orbic", (30.0, L, 31.0))
+        s.cut_mode, s.q = cut, np.array([0.4, -0.3])
+        got = FFieldCUDA(s, "fp64", moves=False).getE10()
+        d2 = sum((Fraction(p) - Fraction(q)) ** 2 for p, q in zip(*s.coords()))
+        S = Fraction(1)
+        if cut == "switch" and d2 > 100:
+            S = (144 - d2) ** 2 * (144 + 2 * d2 - 300) / Fraction(44) ** 3
+        with localcontext() as c:
+            c.prec = 50
+            root = (Decimal(d2.numerator) / Decimal(d2.denominator)).sqrt()
+        e = np.sqrt(s.eps * 418.4)
+        x6 = (Fraction(s.sig[0]) + Fraction(s.sig[1])) ** 6 / d2 ** 3
+        elec = Fraction(s.q[0]) * Fraction(s.q[1]) * Fraction(K) * S / Fraction(root)
+        vdw = 4 * Fraction(e[0]) * Fraction(e[1]) * (x6 * x6 - x6) * S
+        # (x6 - 1) can cancel: its scale is that of x^12 + x^6
+        scale = float(4 * Fraction(e[0]) * Fraction(e[1]) * (x6 * x6 + x6) * S)
+        assert abs(got[3] - float(elec)) <= 72 * 2.0 ** -53 * abs(float(elec)), (r, got[3], float(elec))
+        assert abs(got[4] - float(vdw)) <= 72 * 2.0 ** -53 * scale, (r, got[4], float(vdw), scale)

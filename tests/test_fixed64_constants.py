@@ -16,7 +16,7 @@ from fractions import Fraction as Fr
 
 import pytest
 
-from test_fixed64 import M64, hi
+from test_fixed64 import M64, dist2, hi
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "mc_cpp_gb300", "csrc")
@@ -27,7 +27,7 @@ int main() {
     double L[3], rc, ron;
     while (std::scanf("%la %la %la %la %la", &L[0], &L[1], &L[2], &rc, &ron) == 5) {
         const mcg::Fix64Geom G = mcg::fix64_geom(L, rc, ron);
-        std::printf("%d %d %d %llu %d %llu %a\n", G.sh, G.iso, G.up, (unsigned long long)G.c2, G.sD, (unsigned long long)G.rD, G.leff);
+        std::printf("%d %d %d %llu %d %llu %a %d\n", G.sh, G.iso, G.up, (unsigned long long)G.c2, G.sD, (unsigned long long)G.rD, G.leff, G.emax);
     }
 }
 """
@@ -46,7 +46,7 @@ def geoms(tmp_path_factory):
     def get(cases):
         text = "".join("%s\n" % " ".join(float(v).hex() for v in c) for c in cases)
         out = subprocess.run([exe], input=text, stdout=subprocess.PIPE, text=True, check=True).stdout.split("\n")
-        return [(int(a), int(b), int(c), int(d), int(e), int(f), float.fromhex(g)) for a, b, c, d, e, f, g in
+        return [(int(a), int(b), int(c), int(d), int(e), int(f), float.fromhex(g), int(h)) for a, b, c, d, e, f, g, h in
                 (line.split() for line in out if line)]
     return get
 
@@ -69,7 +69,7 @@ def _boxes(rc, ron):
 
 
 def _check_switch(case, g, rng, samples):
-    sh, iso, up, c2, sD, rD, leff = g
+    sh, iso, up, c2, sD, rD, leff, _ = g
     rc, ron = Fr(case[3]), Fr(case[4])
     l2 = Fr(leff) ** 2
     D = rc * rc - ron * ron
@@ -127,3 +127,29 @@ def test_switch_over_the_normalisation_halved(geoms, L):
 def test_switch_of_common_boxes(geoms, L):
     case = (L, L, L, 12.0, 10.0)
     _check_switch(case, geoms([case])[0], random.Random(5), 2000)
+
+
+# Pairs that the 64-bit form keeps: their distance from positions rounded to 2^-64 of the box, against the exact
+# one.  Each component is off by a unit of each position (and by the units its scaling drops), at most 2^-53 of r
+# in each of three, so r^2 by at most 2 sqrt(3) 2^-53 3.
+@pytest.mark.parametrize("L", [(30.0, 30.0, 30.0), (100.0, 100.0, 100.0), (1e3, 1e3, 1e3), (9e4, 9e4, 9e4), (40.0, 40.0, 700.0), (31.0, 5e3, 47.0)])
+def test_close_limit(geoms, L):
+    sh, iso, up, _, _, _, leff, emax = geoms([(*L, 12.0, 10.0)])[0]
+    rng, kept = random.Random(6), 0
+    for _ in range(3000):
+        a = [rng.uniform(-5, 5) for _ in range(3)]
+        v = [rng.gauss(0, 1) for _ in range(3)]
+        r = 12.0 * 10 ** rng.uniform(-4, 0) / math.sqrt(sum(x * x for x in v))
+        b = [p + x * r for p, x in zip(a, v)]
+        exact = sum((Fr(q) - Fr(p)) ** 2 for p, q in zip(a, b))
+        d = [round(Fr(q) / Fr(l) * 2 ** 64) - round(Fr(p) / Fr(l) * 2 ** 64) for p, q, l in zip(a, b, L)]
+        d = [x << sh for x in d]
+        if not iso:
+            d = [((x * int(Fr(l) / Fr(max(L)) * 2 ** 62)) >> 64) << up for x, l in zip(d, L)]
+        uh, um, ul = dist2(d)
+        if (32 - uh.bit_length()) & ~1 > emax:
+            continue
+        kept += 1
+        u = Fr(uh << 64 | um << 32 | ul, 1 << 96) * Fr(leff) ** 2
+        assert abs(float(u / exact - 1)) <= 6 * math.sqrt(3) * 2.0 ** -53, (a, b, float(exact))
+    assert (kept > 50) == (math.ldexp(leff, -emax // 2 - 1) < 11.0), kept     # some pairs are kept wherever any is in reach
