@@ -69,9 +69,10 @@ Fix64Geom fix64_geom(const double L[3], double rc, double ron) {
 
 Fix64Pair fix64_pair(double qi, double ei, double si, double qj, double ej, double sj, double leff) {
     const long double s = ((long double)si + (long double)sj) / (long double)leff;
+    if (!std::isfinite(s)) return Fix64Pair{qi * qj, std::nan(""), 0, 0};
     int es = 0;
     const long double f = std::frexp(s * s, &es);   // in [1/2, 1)
-    return Fix64Pair{qi * qj, ei * ej, clamp64(f * TWO64L), es};
+    return Fix64Pair{qi * qj, ei * ej, es < FIX64_ES_MIN ? 0 : clamp64(f * TWO64L), std::min(es, FIX64_ES_MAX)};
 }
 
 }  // namespace mcg

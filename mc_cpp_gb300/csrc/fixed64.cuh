@@ -61,12 +61,15 @@ __device__ __forceinline__ unsigned long long fix64_mulhi(unsigned long long a, 
     return (unsigned long long)ah * bh + __umulhi(ah, bl) + __umulhi(al, bh);
 }
 
-// v = ms 2^(es - 64) with ms of at least 2^63 (0 for v = 0), for a finite v that is not negative
-__device__ __forceinline__ void fix64_mantissa(double v, unsigned long long& ms, int& es) {
+// v = ms 2^(es - 64) with ms of at least 2^63 for a v that is not negative, its exponent within the limits of
+// fix64_pair; false when v is not finite
+__device__ __forceinline__ bool fix64_mantissa(double v, unsigned long long& ms, int& es) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     const int e = (int)(b >> 52);
-    ms = e ? (b << 11) | (1ull << 63) : 0ull;       // a subnormal s^2 is no distance
     es = e - 1022;
+    ms = es < FIX64_ES_MIN ? 0ull : (b << 11) | (1ull << 63);
+    es = min(es, FIX64_ES_MAX);
+    return e < 2047;
 }
 
 struct Fix64Dist {

@@ -40,6 +40,10 @@ struct alignas(32) Fix64Pair {
     uint64_t ms;         // s^2 = ms 2^(es - 64) Leff^2, ms of at least 2^63 (0 for s = 0)
     int64_t es;
 };
+// Exponents of s^2 for which w is a normal double at every distance: a smaller s has no w (FP64's is below
+// 2^-900), a larger one's square is infinite (FP64's from an exponent of 172 on).  A sum of sigmas that is not
+// finite makes the pair's energy NaN, as FP64 does.
+constexpr int FIX64_ES_MIN = -320, FIX64_ES_MAX = 300;
 Fix64Pair fix64_pair(double qi, double ei, double si, double qj, double ej, double sj, double leff);
 
 }  // namespace mcg

@@ -612,7 +612,7 @@ __device__ __forceinline__ void pair64_params(const AtomsDev& A, double ileff, i
         const double s = (a.y + b.y) * ileff;
         qq = A.pq[i].w * A.pq[j].w;
         ee = a.x * b.x;
-        fix64_mantissa(s * s, ms, es);
+        if (!fix64_mantissa(s * s, ms, es)) ee = __longlong_as_double(0x7ff8000000000000ll);   // NaN
     }
 }
 

@@ -1,5 +1,6 @@
 // Single-system engine (host object owning the device state of one FField_CUDA).
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <random>
 #include <vector>
@@ -112,7 +113,9 @@ private:
     int ncls = 0;
     // FP64 energies in periodic boxes run on 64-bit integer pair terms (k_energy_list<PREC_F64> and
     // k_energy_all<PREC_F64> are left with systems without a box, whose coordinates have no fixed range)
-    bool uses_fix64() const { return hs.prec == MCG_PREC_FP64 && hs.pbc != MCG_PBC_NONE; }
+    bool uses_fix64() const {
+        return hs.prec == MCG_PREC_FP64 && hs.pbc != MCG_PBC_NONE && std::isfinite(hs.L[0] + hs.L[1] + hs.L[2]);
+    }
     Fix64Geom fix64{};
     ulonglong4_32a* d_x64 = nullptr;
     Fix64Pair* d_pair64 = nullptr;   // ncls64 x ncls64; ncls64 = 0: products formed per pair

@@ -119,3 +119,37 @@ def test_one_pair_in_a_large_box(L, shape, cut):
         scale = float(4 * Fraction(e[0]) * Fraction(e[1]) * (x6 * x6 + x6) * S)
         assert abs(got[3] - float(elec)) <= 72 * 2.0 ** -53 * abs(float(elec)), (r, got[3], float(elec))
         assert abs(got[4] - float(vdw)) <= 72 * 2.0 ** -53 * scale, (r, got[4], float(vdw), scale)
+
+
+# sigmas whose powers leave the range of a double: a tiny one's x^6 is 0, a huge one's energy is not finite, nor is
+# that of one that is not finite itself; 200 charges leave the class table
+@pytest.mark.parametrize("sig", [1e-30, 1e-47, 1e-60, 1e-155, 1e-300, 1e60, 1e200, float("inf"), float("nan")])
+@pytest.mark.parametrize("cut", ["full", "switch"])
+@pytest.mark.parametrize("classes", [1, 200])
+def test_extreme_sigma(sig, cut, classes):
+    n = 300
+    s = _atoms(30.0, "cubic", n)
+    s.q = np.resize(np.linspace(-0.4, 0.4, classes) if classes > 1 else [0.3], n)
+    s.cut_mode, s.sig = cut, s.sig.copy()
+    s.sig[:] = sig
+    got = FFieldCUDA(s, "fp64", moves=False).getE10()
+    want, scale = _oracle(s)
+    assert abs(got[3] - want[3]) <= REL * abs(_oracle_elec(s)), (got, want)
+    assert np.isfinite(got[4]) == np.isfinite(want[4]), (got, want)
+    if np.isfinite(want[4]):
+        assert abs(got[4] - want[4]) <= REL * abs(want[4]) + 1e-250, (got, want)
+
+
+def _oracle_elec(s):
+    t = s.copy()
+    t.q = np.abs(t.q)
+    return orc.Oracle(t, moves=False).energy()[3]
+
+
+@pytest.mark.parametrize("sig", [1e-60, 1e-300])
+def test_extreme_sigma_batch(sig):
+    s = _atoms(30.0, "cubic", 300, charges=0.2)
+    s.sig = np.full(300, sig)
+    got = BatchChains([s], dmax_trn=0.05, dmax_rot=1.0, seed=1).energy_fp64()[0]
+    want, _ = _oracle(s)
+    assert abs(got - want[3] - want[4]) <= (2 * REL + 2 * 2.0 ** -52 * 30.0 / 1.2) * abs(want[3]), (got, want)
