@@ -955,15 +955,18 @@ __device__ __forceinline__ void two_sum_to(float2& s, float2& c, float2 v) {
 }
 
 // Mixed-precision full energy: the pair terms of mixed_pair without the switch for two columns at a time,
-// the halves of float2 values, summed per thread and half as float-float over all its units, in FP64
-// across the CTA.  A column that is not to count (excluded, not above the row, past the last atom) takes
+// the halves of float2 values, summed per thread and half as float-float over ALLMIX_FLUSH units, 64 pairs a
+// half, in FP64 beyond: float-float holds 48 bits of its largest partial sum, and over thousands of pairs of one
+// thread that showed (the Lennard-Jones energy of 36,864 argon atoms moved by 1.2e-14 with their order, by 2.2e-16
+// so; 2% of the time).  A column that is not to count (excluded, not above the row, past the last atom) takes
 // 1/r = 0, which makes its terms exactly 0.  Bound by the FP32 pipe.  The columns' positions and
 // parameters come from shared memory, the row's and the next excluded atom stay in registers.
 // Without a box a displacement is an FP64 difference rounded to FP32, and those are the bound.
 // Whole energy calls, against a column at a time in square tiles with the exclusion row read at every
-// column: 12,288 water atoms (75 M pairs) 170 us, was 227; 36,864 1360, was 1652 (one column at a time
+// column: 12,288 water atoms (75 M pairs) 171 us, was 227; 36,864 1384, was 1652 (one column at a time
 // in these units: 1475); 4,096 argon atoms 37, was 56.
-constexpr int ALLMIX_CTAS = 5;   // per SM; 3,000 water atoms, 36,864: 4 take 31 and 1388 us, 5 34 and 1360, 8 37 and 1359
+constexpr int ALLMIX_FLUSH = 4;
+constexpr int ALLMIX_CTAS = 5;   // per SM; 3,000 water atoms, 36,864: 4 take 31 and 1388 us, 5 34 and 1360, 8 37 and 1359 (float-float throughout)
 
 template <bool BOX>
 __global__ void __launch_bounds__(ALL_I, ALLMIX_CTAS) k_energy_all_mix(AtomsDev A, int n,
@@ -978,7 +981,15 @@ __global__ void __launch_bounds__(ALL_I, ALLMIX_CTAS) k_energy_all_mix(AtomsDev 
     const float2 zero = make_float2(0.0f, 0.0f), neg = make_float2(-1.0f, -1.0f);
     auto both = [](float v) { return make_float2(v, v); };
     float2 eh = zero, el = zero, vh = zero, vl = zero;
+    double sel = 0.0, svd = 0.0;
+    auto flush = [&]() {
+        sel += ((double)eh.x + (double)eh.y) + ((double)el.x + (double)el.y);
+        svd += ((double)vh.x + (double)vh.y) + ((double)vl.x + (double)vl.y);
+        eh = el = vh = vl = zero;
+    };
+    int since = 0;   // units since the float-float sums went to FP64
     for (long long unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        if (since++ == ALLMIX_FLUSH) { flush(); since = 1; }
         int jb;
         const int i = all_unit(unit, c0, jb) * ALL_I + threadIdx.x, je = min(n, jb + ALL_J);
         __syncthreads();
@@ -1043,8 +1054,8 @@ __global__ void __launch_bounds__(ALL_I, ALLMIX_CTAS) k_energy_all_mix(AtomsDev 
             two_sum_to(vh, vl, __fmul2_rn(__fmul2_rn(both(ei.x), col(sprm[2])), l));
         }
     }
-    block_reduce2(((double)eh.x + (double)eh.y) + ((double)el.x + (double)el.y),
-                  ((double)vh.x + (double)vh.y) + ((double)vl.x + (double)vl.y), part + 2 * blockIdx.x);
+    flush();
+    block_reduce2(sel, svd, part + 2 * blockIdx.x);
 }
 
 // FP64 full energy for periodic boxes, on 64-bit integer pair terms (fixed64.cuh): three FP64
