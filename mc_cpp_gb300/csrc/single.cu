@@ -259,17 +259,15 @@ constexpr int ROW_WARPS = 4;
 constexpr int ROW_CTAS = 7;    // CTAs of four warps resident per SM at the kernel's 72 registers
 constexpr int ROW_RING = 128;  // up to 63 pending candidates and 64 new ones
 
-// The pairs the FP32 test does not decide: in the band around the list radius, close in index (the atom
-// itself, or perhaps excluded), or with frozen atoms about.
-__device__ __noinline__ bool row_pair(const double4_32a* __restrict__ pq, const uint8_t* __restrict__ frozen, const PbcDev& pbc,
-                                      const ListParams& lp, const int* __restrict__ xs, const int* __restrict__ xd, int i, int j,
+// The pairs the FP32 test does not decide: in the band around the list radius, or close in index (the atom
+// itself, or perhaps excluded).
+__device__ __noinline__ bool row_pair(const double4_32a* __restrict__ pq, const PbcDev& pbc, const ListParams& lp, const int* __restrict__ xs, const int* __restrict__ xd, int i, int j,
                                       bool exact) {
     if (j == i) return false;
     if (exact) {
         const double4_32a pi = pq[i], pj = pq[j];
         if (!(ref64_dist2(pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, pbc) <= lp.cutnb2)) return false;
     }
-    if (lp.any_frozen && frozen[i] && frozen[j]) return false;
     return !stored_excluded(min(i, j), max(i, j), xs, xd, lp.maxspan);
 }
 
@@ -295,8 +293,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
     uint4* ring = s_ring[wib];
     list_step();
     const int ntask = task_start[ncell];
-    // partners within maxspan in index are looked at; with frozen atoms about, every partner
-    const unsigned span2 = lp.any_frozen ? 0xffffffffu : 2u * (unsigned)lp.maxspan;
+    const unsigned span2 = 2u * (unsigned)lp.maxspan;   // partners within maxspan in index are looked at
     int longest = 0;
     // the first task by the warp's place, the others from a counter (max_row[1]), each fetched while the one
     // before it is worked on: a grid of what is resident at once, without a last wave
@@ -310,6 +307,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
         uint32_t hx[A][3];
         int hi[A], up[A], back[A], first[A];
         int* row[A];
+        unsigned fixed = 0;              // the frozen ones among them
 #pragma unroll
         for (int k = 0; k < A; k++) {
             const uint4 p = cell_pos[home[tk.y + (k < m ? k : 0)]];
@@ -319,6 +317,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
             up[k] = 0;
             back[k] = lp.cap - 1;
             row[k] = nbr + (size_t)p.w * lp.cap;
+            if (lp.any_frozen) fixed |= (unsigned)(frozen[p.w] != 0) << k;
         }
         // per axis: the offsets scanned, and the home atoms' extent inside the cell (in cell widths) for
         // the distance from them to a cell d away along that axis.  FP32 throughout (FP64 here, at
@@ -476,13 +475,15 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
             } else if (j >= 0) {
                 in = band = (1u << A) - 1u;
             }
+            // two frozen atoms are no pair: a look at the candidate's flag, once for all home atoms
+            if (fixed && in && frozen[j]) { in &= ~fixed; look &= ~fixed; band &= ~fixed; }
             if (look | band) {
                 for (unsigned l = look | band; l; l &= l - 1) {
                     const int k = __ffs(l) - 1;
                     int i = hi[0];
 #pragma unroll
                     for (int q = 1; q < A; q++) if (k == q) i = hi[q];
-                    if (!row_pair(pq, frozen, pbc, lp, xs, xd, i, j, band >> k & 1u)) in &= ~(1u << k);
+                    if (!row_pair(pq, pbc, lp, xs, xd, i, j, band >> k & 1u)) in &= ~(1u << k);
                 }
             }
             __syncwarp();
