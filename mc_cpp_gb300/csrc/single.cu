@@ -160,7 +160,8 @@ __global__ void k_cell_scatter(const int* __restrict__ cell_of, int n, const int
 // the octant of the cell they lie in (places in cell order), and of the row build's tasks: runs of at
 // most `run` of these.  The grouping only decides which rows are built together.
 __global__ void k_cell_sort(const int* __restrict__ cell_start, const int* __restrict__ task_start, int ncell, int run,
-                            const uint4* __restrict__ fx, Grid g, int* cell_atoms, uint4* cell_pos, int* home, int2* tasks) {
+                            const uint4* __restrict__ fx, const double4_32a* __restrict__ pq, Grid g, int* cell_atoms, uint4* cell_pos,
+                            int* home, int2* tasks) {
     __shared__ int sh[SORT_MAX];
     __shared__ uint8_t oct[SORT_MAX];
     int c = blockIdx.x;
@@ -198,13 +199,24 @@ __global__ void k_cell_sort(const int* __restrict__ cell_start, const int* __res
     }
     for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
         const int a = cell_atoms[i];
-        uint4 p = fx[a];
+        uint4 p = fx[a];       // box fractions; without a box, FP32 distances from the atoms' lowest coordinates
+        unsigned hx, hy, hz;   // the half of the cell along each axis
+        if (g.periodic) {
+            hx = (unsigned)((unsigned long long)p.x * (2 * g.nc[0]) >> 32);
+            hy = (unsigned)((unsigned long long)p.y * (2 * g.nc[1]) >> 32);
+            hz = (unsigned)((unsigned long long)p.z * (2 * g.nc[2]) >> 32);
+        } else {
+            const double4_32a q = pq[a];
+            const float x = (float)(q.x - g.lo[0]), y = (float)(q.y - g.lo[1]), z = (float)(q.z - g.lo[2]);
+            p = make_uint4(__float_as_uint(x), __float_as_uint(y), __float_as_uint(z), 0u);
+            hx = (unsigned)(x * (float)g.inv[0] * (float)(2 * g.nc[0]));
+            hy = (unsigned)(y * (float)g.inv[1] * (float)(2 * g.nc[1]));
+            hz = (unsigned)(z * (float)g.inv[2] * (float)(2 * g.nc[2]));
+        }
         p.w = (unsigned)a;
         cell_pos[i] = p;
-        if (m <= SORT_MAX) {   // the half of the cell along each axis, from the box fraction
-            const unsigned hx = (unsigned)((unsigned long long)p.x * (2 * g.nc[0]) >> 32) & 1u,
-                           hy = (unsigned)((unsigned long long)p.y * (2 * g.nc[1]) >> 32) & 1u,
-                           hz = (unsigned)((unsigned long long)p.z * (2 * g.nc[2]) >> 32) & 1u;
+        if (m <= SORT_MAX) {
+            hx &= 1u; hy &= 1u; hz &= 1u;
             oct[i - b] = (uint8_t)(hz << 2 | hy << 1 | (hx ^ hy));   // neighbouring octants share a face
         } else {
             home[i] = i;
@@ -220,14 +232,17 @@ __global__ void k_cell_sort(const int* __restrict__ cell_start, const int* __res
     }
 }
 
+constexpr double LIST_EXTENT = 20.0;
+
 struct ListParams {
     double cutnb2;
     int cap;
     int maxspan;
-    // periodic boxes: FP32 prefilter on the fixed-point mirrors.  A pair whose FP32 r^2 lies below
-    // lo2 is inside, above hi2 outside; only the band between takes the reference's FP64 test.
-    // (A^2, or units of (L 2^-32)^2 when the box lengths are equal)
-    float Ls[3];
+    // FP32 prefilter.  A pair whose FP32 r^2 lies below lo2 is inside, above hi2 outside; only the band between
+    // takes the reference's FP64 test.  (A^2, or units of (L 2^-32)^2 in boxes of equal lengths.)  Without a box the
+    // candidates hold FP32 coordinates, off by 2^-25 of the atoms' extent: up to an extent of LIST_EXTENT list radii
+    // that moves a distance by 2e-6 of the radius, inside the margins; atoms spread farther are all in the band.
+    float Ls[3];            // length of a unit of the candidates' coordinates (1 without a box)
     float lo2, hi2;
     float reach2;   // rows of cells farther than this (squared, with a margin) are not scanned
     int any_frozen;
@@ -246,15 +261,17 @@ __device__ __forceinline__ bool stored_excluded(int lo, int hi, const int* __res
 // cells become ranges of the candidates, dropped or trimmed where no home atom reaches; the ranges are
 // walked as one sequence, the end of one with the beginning of the next, and the next 64 candidates load
 // while these are tested.  A row lists its
-// partners in the candidates' order, whatever the grouping.  In periodic boxes a pair is first placed by its
-// FP32 distance from the exact fixed-point mirrors (error ~2e-7 of (rc + skin)^2); the reference's FP64
-// distance decides only the pairs within 1e-4 of the list radius, so the rows are the reference's sets.
+// partners in the candidates' order, whatever the grouping.  A pair is first placed by its FP32 distance, in
+// periodic boxes from the exact fixed-point mirrors (error ~2e-7 of (rc + skin)^2), without a box from FP32
+// coordinates (at most 5e-6 of it, ListParams); the reference's FP64 distance decides only the pairs within
+// 1e-4 of the list radius, so the rows are the reference's sets.
 // Before the home atoms' tests the candidates pass one against the sphere around all of them, and the
 // survivors (1,750 of 3,200 for four atoms of one octant of a water cell, 1,150 end in a row) are
 // gathered in a ring, 32 at a time.  Bound by issue.  (One atom per warp with an index gather in front
 // of every candidate took 1.48 ms on the 100,002-atom water box and 188 us at 12,288 atoms.  Two candidates
 // per lane in the walk, and tasks from a counter instead of a third wave of CTAs, took a whole update of
-// the former from 754 to 653 us.)
+// the former from 754 to 653 us.  Without a box, where every candidate took the FP64 test: 36,000 water atoms
+// 1756 us, 299 with the FP32 coordinates.)
 constexpr int ROW_WARPS = 4;
 constexpr int ROW_CTAS = 7;    // CTAs of four warps resident per SM at the kernel's 72 registers
 constexpr int ROW_RING = 128;  // up to 63 pending candidates and 64 new ones
@@ -349,20 +366,27 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
                 else if (PERIODIC) { dlo[k] = -2; dhi[k] = 2; }
                 else { dlo[k] = max(-2, -ctr[k]); dhi[k] = min(2, g.nc[k] - 1 - ctr[k]); }
             }
-            if (PERIODIC) {   // the sphere around the home atoms: the middle of their extent, and its radius
-                float far2 = 0.f;
-                for (int k = 0; k < 3; k++) {
+            // the sphere around the home atoms: the middle of their extent, and its radius
+            float far2 = 0.f;
+            for (int k = 0; k < 3; k++) {
+                float e;
+                if (PERIODIC) {
                     const int d = (int)(q3[k] - hx[0][k]);
                     const int mn = __reduce_min_sync(0xffffffffu, d), mx = __reduce_max_sync(0xffffffffu, d);
                     const int mid = mn + (int)((unsigned)(mx - mn) >> 1);
                     ball[k] = hx[0][k] + (uint32_t)mid;
-                    const float e = (float)(d - mid) * lp.Ls[k];
-                    far2 = fmaf(e, e, far2);
+                    e = (float)(d - mid) * lp.Ls[k];
+                } else {
+                    const float mn = __uint_as_float(__reduce_min_sync(0xffffffffu, q3[k])),
+                                mx = __uint_as_float(__reduce_max_sync(0xffffffffu, q3[k])), mid = 0.5f * (mn + mx);
+                    ball[k] = __float_as_uint(mid);
+                    e = __uint_as_float(q3[k]) - mid;
                 }
-                far2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(far2)));
-                const float reach = sqrtf(lp.reach2) + sqrtf(far2);
-                ball2 = reach * reach;
+                far2 = fmaf(e, e, far2);
             }
+            far2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(far2)));
+            const float reach = sqrtf(lp.reach2) + sqrtf(far2);
+            ball2 = lp.lo2 < 0.f ? lp.hi2 : reach * reach;
         }
         auto gap2 = [&](int k, int d) -> float {   // squared lower bound on |displacement| along axis k
             if (whole[k] || d == 0) return 0.f;
@@ -426,10 +450,12 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
         uint4 n0 = make_uint4(0, 0, 0, NONE), n1 = n0;
         fetch(n0, n1);
         int head = 0, tail = 0;            // candidates within reach of the home atoms, pending in the ring
+        // difference of two coordinates in the candidates' unit
+        auto diff = [](uint32_t c, uint32_t h) {
+            return PERIODIC ? __int2float_rn((int)(c - h)) : __uint_as_float(c) - __uint_as_float(h);
+        };
         auto within = [&](const uint4& c) {
-            if (!PERIODIC) return c.w != NONE;
-            const float dx = __int2float_rn((int)(c.x - ball[0])) * lp.Ls[0], dy = __int2float_rn((int)(c.y - ball[1])) * lp.Ls[1],
-                        dz = __int2float_rn((int)(c.z - ball[2])) * lp.Ls[2];
+            const float dx = diff(c.x, ball[0]) * lp.Ls[0], dy = diff(c.y, ball[1]) * lp.Ls[1], dz = diff(c.z, ball[2]) * lp.Ls[2];
             return c.w != NONE && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= ball2;
         };
         while (more || head != tail) {
@@ -454,26 +480,21 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_build_rows(const double4_32a
             // bit k: the candidate is in home atom k's row; close to it in index; in the band (one branch
             // for all that have to be looked at)
             unsigned in = 0, look = 0, band = 0;
-            if (PERIODIC) {
-                const float lo2 = j >= 0 ? lp.lo2 : -1.0f, hi2 = j >= 0 ? lp.hi2 : -1.0f;
+            const float lo2 = j >= 0 ? lp.lo2 : -1.0f, hi2 = j >= 0 ? lp.hi2 : -1.0f;
 #pragma unroll
-                for (int k = 0; k < A; k++) {
-                    const float ux = __int2float_rn((int)(cd.x - hx[k][0])), uy = __int2float_rn((int)(cd.y - hx[k][1])),
-                                uz = __int2float_rn((int)(cd.z - hx[k][2]));
-                    float r2;
-                    if (ISO) {
-                        r2 = fmaf(ux, ux, fmaf(uy, uy, uz * uz));   // in units of (L 2^-32)^2, as lo2 and hi2
-                    } else {
-                        const float dx = ux * lp.Ls[0], dy = uy * lp.Ls[1], dz = uz * lp.Ls[2];
-                        r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    }
-                    const unsigned near = r2 <= hi2 ? 1u << k : 0u;
-                    in |= near;
-                    band |= r2 < lo2 ? 0u : near;
-                    look |= (unsigned)(j - first[k]) <= span2 ? near : 0u;
+            for (int k = 0; k < A; k++) {
+                const float ux = diff(cd.x, hx[k][0]), uy = diff(cd.y, hx[k][1]), uz = diff(cd.z, hx[k][2]);
+                float r2;
+                if (ISO) {
+                    r2 = fmaf(ux, ux, fmaf(uy, uy, uz * uz));   // in units of (L 2^-32)^2 in a box, as lo2 and hi2
+                } else {
+                    const float dx = ux * lp.Ls[0], dy = uy * lp.Ls[1], dz = uz * lp.Ls[2];
+                    r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
                 }
-            } else if (j >= 0) {
-                in = band = (1u << A) - 1u;
+                const unsigned near = r2 <= hi2 ? 1u << k : 0u;
+                in |= near;
+                band |= r2 < lo2 ? 0u : near;
+                look |= (unsigned)(j - first[k]) <= span2 ? near : 0u;
             }
             // two frozen atoms are no pair: a look at the candidate's flag, once for all home atoms
             if (fixed && in && frozen[j]) { in &= ~fixed; look &= ~fixed; band &= ~fixed; }
@@ -2217,7 +2238,7 @@ int SingleEngine::build_list() {
     // home atoms that share a walk: four share more of it, two leave fewer warps idle in a small system.  A
     // whole update with two, four and eight, each some 14 us more than now: 50, 58, 59 us (864 argon atoms), 72, 84, 97 (1,800 water
     // atoms), 170, 159, 174 (12,288), 359, 305, 338 (36,000), 948, 761, 753 (100,002), so the line is at 8,192
-    const int run = !g.periodic || n < 8192 ? 2 : 4;
+    const int run = n < 8192 ? 2 : 4;
     int rc;
     if (ncell > ncell_cap) {
         int** const per_cell[] = {&d_cell_count, &d_cell_start, &d_cell_fill, &d_task_start};
@@ -2248,11 +2269,12 @@ int SingleEngine::build_list() {
         double t = hs.rc + hs.dcut;  // (cutoff + deltacut)^2 as List_nonBonded.cpp:842-843
         lp.cutnb2 = t * t;
         const AtomsDev A = atoms();
-        for (int k = 0; k < 3; k++) lp.Ls[k] = A.Ls[k];
+        for (int k = 0; k < 3; k++) lp.Ls[k] = g.periodic ? A.Ls[k] : 1.0f;
         const double unit2 = iso ? (hs.L[0] / 4294967296.0) * (hs.L[0] / 4294967296.0) : 1.0;
         lp.lo2 = (float)(lp.cutnb2 * (1.0 - 1e-4) / unit2);
         lp.hi2 = (float)(lp.cutnb2 * (1.0 + 1e-4) / unit2);
         lp.reach2 = (float)(lp.cutnb2 * (1.0 + 1e-5) + 1e-2);
+        if (!g.periodic && std::max(ext[0], std::max(ext[1], ext[2])) > LIST_EXTENT * t) { lp.lo2 = -1.0f; lp.hi2 = HUGE_VALF; }
     }
     for (int attempt = 0; attempt < 3; attempt++) {
         cudaLaunchAttribute after[1];
@@ -2270,12 +2292,13 @@ int SingleEngine::build_list() {
         CK(launch(k_cell_assign, (n + 255) / 256, 256, d_pq, n, pbc, g, d_cell_of, d_cell_count));
         CK(launch(k_cell_scan, 1, 1024, d_cell_count, ncell, run, d_cell_start, d_cell_fill, d_task_start, d_maxrow));
         CK(launch(k_cell_scatter, (n + 255) / 256, 256, d_cell_of, n, d_cell_start, d_cell_fill, d_cell_atoms));
-        CK(launch(k_cell_sort, ncell, 128, d_cell_start, d_task_start, ncell, run, d_fx, g, d_cell_atoms, d_cell_pos, d_home, d_tasks));
+        CK(launch(k_cell_sort, ncell, 128, d_cell_start, d_task_start, ncell, run, d_fx, d_pq, g, d_cell_atoms, d_cell_pos, d_home, d_tasks));
         const int blocks = std::min((n / run + ncell + ROW_WARPS - 1) / ROW_WARPS, 152 * ROW_CTAS);
 #define MCG_ROWS(A_, P_, I_)                                                                                          \
     CK(launch(k_build_rows<A_, P_, I_>, blocks, 32 * ROW_WARPS, d_pq, d_cell_pos, d_frozen, pbc, g, lp, d_cell_start, \
               d_task_start, ncell, d_home, d_tasks, d_xs, d_xd, d_nbr, d_nup, d_nlo, d_maxrow, (int*)(d_map + 24)))
-        if (!g.periodic) MCG_ROWS(2, false, false);
+        if (!g.periodic && run == 4) MCG_ROWS(4, false, true);
+        else if (!g.periodic) MCG_ROWS(2, false, true);
         else if (iso && run == 4) MCG_ROWS(4, true, true);
         else if (iso) MCG_ROWS(2, true, true);
         else if (run == 4) MCG_ROWS(4, true, false);

@@ -1,5 +1,7 @@
-"""Verlet rows of the list build's other forms, as sets against the FP64 oracle's: systems with frozen atoms
-(a flag per home atom and candidate).
+"""Verlet rows of the list build's other forms, as sets against the FP64 oracle's: systems without a box (FP32
+coordinates place most pairs, up to an extent of 20 list radii; beyond it the FP64 test takes all) and frozen
+atoms (a flag per home atom and candidate).  Partners are put within 1e-9 to 1e-3 of the list radius, on both
+sides, where FP32 may not decide.
 """
 import numpy as np
 import pytest
@@ -24,6 +26,35 @@ def _compare(s):
     want = orc.Oracle(s, moves=False).verlet_rows()
     assert all(np.array_equal(a, np.sort(b)) for a, b in zip(rows, want, strict=True))
     return sum(len(r) for r in rows)
+
+
+def _atoms(n, extent, seed):
+    """n atoms over a cube of the given extent, a third of them partners of others at about the list radius."""
+    s = systems.argon_random(n, 0.0213, seed)
+    rng = np.random.default_rng(seed)
+    xyz = rng.uniform(0.0, extent, (n, 3))
+    k = n // 3
+    v = rng.normal(size=(k, 3))
+    r = 14.0 * (1.0 + rng.choice([-1.0, 1.0], k) * 10.0 ** rng.uniform(-9, -3, k))
+    xyz[n - k:] = xyz[:k] + v * (r / np.linalg.norm(v, axis=1))[:, None]
+    s.set_coords(xyz)
+    s.pbc_type = "none"
+    return s
+
+
+# 20 list radii are 280 A
+@pytest.mark.parametrize("extent", [5.0, 60.0, 240.0, 300.0, 2e4])
+@pytest.mark.parametrize("offset", [0.0, -1e5])
+@pytest.mark.parametrize("n", [2, 45, 1500])
+def test_rows_without_a_box(n, extent, offset):
+    s = _atoms(n, extent, n)
+    s.set_coords(s.coords() + offset)
+    _compare(s)
+
+
+@pytest.mark.parametrize("n", [8191, 8192])
+def test_rows_without_a_box_at_the_task_size(n):
+    assert _compare(_atoms(n, 90.0, n)) > 100000
 
 
 @pytest.mark.parametrize("kind", ["cubic", "none"])
