@@ -2292,7 +2292,9 @@ int SingleEngine::build_list() {
         CK(launch(k_cell_assign, (n + 255) / 256, 256, d_pq, n, pbc, g, d_cell_of, d_cell_count));
         CK(launch(k_cell_scan, 1, 1024, d_cell_count, ncell, run, d_cell_start, d_cell_fill, d_task_start, d_maxrow));
         CK(launch(k_cell_scatter, (n + 255) / 256, 256, d_cell_of, n, d_cell_start, d_cell_fill, d_cell_atoms));
-        CK(launch(k_cell_sort, ncell, 128, d_cell_start, d_task_start, ncell, run, d_fx, d_pq, g, d_cell_atoms, d_cell_pos, d_home, d_tasks));
+        // a CTA per cell: 128 threads, or 512 where cells hold hundreds of atoms (3,000 in one cell: 82 us an update with
+        // 512 threads, 100 with 128)
+        CK(launch(k_cell_sort, ncell, n / ncell >= 256 ? 512 : 128, d_cell_start, d_task_start, ncell, run, d_fx, d_pq, g, d_cell_atoms, d_cell_pos, d_home, d_tasks));
         const int blocks = std::min((n / run + ncell + ROW_WARPS - 1) / ROW_WARPS, 152 * ROW_CTAS);
 #define MCG_ROWS(A_, P_, I_)                                                                                          \
     CK(launch(k_build_rows<A_, P_, I_>, blocks, 32 * ROW_WARPS, d_pq, d_cell_pos, d_frozen, pbc, g, lp, d_cell_start, \

@@ -1,7 +1,7 @@
 """Verlet rows of the list build's other forms, as sets against the FP64 oracle's: systems without a box (FP32
-coordinates place most pairs, up to an extent of 20 list radii; beyond it the FP64 test takes all) and frozen
-atoms (a flag per home atom and candidate).  Partners are put within 1e-9 to 1e-3 of the list radius, on both
-sides, where FP32 may not decide.
+coordinates place most pairs, up to an extent of 20 list radii; beyond it the FP64 test takes all), frozen atoms
+(a flag per home atom), and cells of hundreds of atoms (512 threads a cell, more than 2,048 unsorted in shared
+memory).  Partners are put within 1e-9 to 1e-3 of the list radius, on both sides, where FP32 may not decide.
 """
 import numpy as np
 import pytest
@@ -68,3 +68,12 @@ def test_rows_with_frozen_atoms(kind, frozen, nmol):
                 "all but one": np.arange(n) != 7, "all": np.ones(n, bool)}[frozen].astype(np.uint8)
     total = _compare(s)
     assert (total == 0) == (frozen == "all")
+
+
+@pytest.mark.parametrize("n", [255, 256, 2047, 2049, 2500])
+@pytest.mark.parametrize("kind", ["cubic", "none"])
+def test_rows_of_crowded_cells(n, kind):
+    s = systems.argon_random(n, 0.0213 * 125, n)       # one cell: the box is at most 10 A, the list radius more than half
+    s.cutoff, s.cuton, s.sig = s.box[0] / 2.1, s.box[0] / 4, s.sig / 5
+    s.pbc_type = kind
+    _compare(s)
