@@ -731,9 +731,11 @@ int GroupPairs::build(cudaStream_t st, const int* rows, const int* lens, int cap
     if (ngroup <= GBM_GROUPS) {
         const int words = (ngroup + 1023) / 1024 * 32;
         const size_t smem = (size_t)GB_WARPS * sizeof(unsigned) * (words + words / 2 + 2 * GH_MAX);
-        static_assert((size_t)GB_WARPS * sizeof(unsigned) * (GBM_GROUPS / 32 * 3 / 2 + 2 * GH_MAX) <= 227 * 1024, "bitmap rows");
-        if (smem > 48 * 1024)
-            GK(cudaFuncSetAttribute(k_group_rows_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the kernel's limit is the process's, not this handle's: always the largest, so that builds of several handles
+        // in several threads do not lower it under each other
+        constexpr size_t most = (size_t)GB_WARPS * sizeof(unsigned) * (GBM_GROUPS / 32 * 3 / 2 + 2 * GH_MAX);
+        static_assert(most > 48 * 1024 && most <= 227 * 1024, "bitmap rows");
+        if (smem > 48 * 1024) GK(cudaFuncSetAttribute(k_group_rows_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         k_group_rows_bitmap<<<blocks, GB_WARPS * 32, smem, st>>>(d_gstart, d_gslot, ngroup, words, rows, lens, cap, d_grow, d_glen,
                                                                  gcap, d_misc);
     } else {
