@@ -1645,7 +1645,10 @@ static int dalloc(T** p, size_t count) {
     *p = nullptr;
     if (count == 0) count = 1;
     cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
-    if (e != cudaSuccess) return fail(MCG_ECUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // reported here, not left for the next call's launches
+        return fail(MCG_ECUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     return MCG_OK;
 }
 
@@ -1943,6 +1946,7 @@ int SingleEngine::set_pair_kernel(int v) {
 // limits keeps the other kernels.
 int SingleEngine::ensure_groups() {
     if (!grp_setup || !grp_dirty) return MCG_OK;
+    if (int rc = need_list()) return rc;
     grp_dirty = false;
     const bool pr = prune_buf > 0.0 && !prune_dirty && d_prn;
     const int grc = grp.build(stream, pr ? d_prn : d_nbr, pr ? d_pnup : d_nup, cap);
@@ -1992,6 +1996,7 @@ bool SingleEngine::uses_pair_variants() const {
 // clusters do not fit the build's shared-memory limits keeps the per-atom list kernels only.
 int SingleEngine::ensure_clusters() {
     if (!clp_dirty) return MCG_OK;
+    if (int rc = need_list()) return rc;
     clp_dirty = false;
     const int crc = clp.build(stream, d_fx, n, hs.L, d_nbr, d_nup, d_nlo, cap);
     launches += clp.build_launches;
@@ -2006,8 +2011,8 @@ int SingleEngine::ensure_clusters() {
 // cluster list built for it); a chosen cluster variant has its list brought up to date.  Runs
 // before the caller takes the partial-sum buffer, which the cluster build may grow.
 int SingleEngine::prepare_pair_kernel() {
-    if (!uses_pair_variants()) return MCG_OK;
-    int rc;
+    int rc = need_list();
+    if (rc || !uses_pair_variants()) return rc;
     if ((rc = ensure_pruned())) return rc;
     if (pair_variant < 0) {
         if ((rc = ensure_clusters())) return rc;
@@ -2030,7 +2035,8 @@ int SingleEngine::prepare_pair_kernel() {
 // between event records, so its device time can be read back without a synchronisation here.
 int SingleEngine::ensure_pruned() {
     if (prune_buf <= 0.0 || !prune_dirty) return MCG_OK;
-    int rc;
+    int rc = need_list();
+    if (rc) return rc;
     if (prn_cap != cap) {   // the pruned rows share the Verlet rows' stride
         if (d_prn) cudaFree(d_prn);
         d_prn = nullptr;
@@ -2213,6 +2219,11 @@ BondedDev SingleEngine::bonded() const {
                      d_dihes, (int)hs.dihes.size(), d_imprs, (int)hs.imprs.size()};
 }
 
+// Rows that a failed build left short (no memory for longer ones) are not read: their counts run past them.
+int SingleEngine::need_list() const {
+    return hs.cut != MCG_CUT_SWITCH || list_ok ? MCG_OK : fail(MCG_ECUDA, "no Verlet list: the last list update failed");
+}
+
 int SingleEngine::build_list() {
     const double rl = hs.rc + hs.dcut;
     Grid g;
@@ -2241,6 +2252,7 @@ int SingleEngine::build_list() {
     const int run = n < 8192 ? 2 : 4;
     int rc;
     if (ncell > ncell_cap) {
+        ncell_cap = 0;             // an allocation that fails leaves them to the next build
         int** const per_cell[] = {&d_cell_count, &d_cell_start, &d_cell_fill, &d_task_start};
         for (int** p : per_cell) {
             if (*p) cudaFree(*p);
@@ -2261,8 +2273,12 @@ int SingleEngine::build_list() {
         double est = g.periodic ? (4.0 / 3.0 * PI * rl * rl * rl) * n / vol : n;
         cap = (int)std::min<double>(n, est * 1.3 + 64);
         cap = (cap + 31) & ~31;
-        if ((rc = dalloc(&d_nbr, (size_t)n * cap))) return rc;
     }
+    if (!d_nbr && (rc = dalloc(&d_nbr, (size_t)n * cap))) {
+        cap = 0;
+        return rc;
+    }
+    list_ok = false;   // until the rows are whole
     ListParams lp{rl * rl, cap, hs.maxExclSpan, {0, 0, 0}, 0.f, 0.f, 0.f, any_frozen};
     {
         // equal box lengths: r^2 stays in the mirrors' own units
@@ -2313,13 +2329,17 @@ int SingleEngine::build_list() {
             clp_dirty = uses_pair_variants();   // the cluster form follows on first use
             prune_dirty = true;                 // and so do the pruned rows
             grp_dirty = grp_setup;              // and the group rows
+            list_ok = true;
             return MCG_OK;
         }
         cudaFree(d_nbr);
         d_nbr = nullptr;
         cap = ((int)(maxrow * 1.1) + 32 + 31) & ~31;
         lp.cap = cap;
-        if ((rc = dalloc(&d_nbr, (size_t)n * cap))) return rc;
+        if ((rc = dalloc(&d_nbr, (size_t)n * cap))) {
+            cap = 0;               // the next build begins at the estimate again
+            return rc;
+        }
     }
     return fail(MCG_ECAPACITY, "Verlet row capacity could not be grown");
 }
@@ -2439,6 +2459,7 @@ int SingleEngine::get_coords(double* x, double* y, double* z) {
 
 int SingleEngine::delta_e(int m, const int* atoms_in, const double* nx, const double* ny, const double* nz, double* de) {
     pending_m = 0;   // a new proposal replaces the pending one, also when it is rejected
+    if (int rc = need_list()) return rc;
     if (m <= 0 || m > MAX_MOVED) return fail(MCG_EINVAL, "moved-set size must be in [1, 1024]");
     // sort the moved set (keeps proposal coordinates paired), reject duplicates
     std::vector<int> ord(m);
@@ -2904,6 +2925,7 @@ int SingleEngine::metropolis_device(std::mt19937& gen, const std::vector<MoveKin
                                     double* etot, int64_t* n_accepted) {
     const int nt = (int)moves.size();
     if (nt < 1 || nt > RP_MAXT) return fail(MCG_ENOTSUP, "device run: 1 to 8 move types");
+    if (int rc = need_list()) return rc;
     ReplayTables T{};
     ReplayState S{};
     std::vector<int> first, ranges;
@@ -3048,6 +3070,7 @@ int SingleEngine::get_pairlist(int* counts, int* entries, int64_t cap_entries, i
         if (total) *total = 0;
         return MCG_OK;
     }
+    if (int rc = need_list()) return rc;
     std::vector<int> up(n);
     CK(cudaMemcpyAsync(up.data(), d_nup, sizeof(int) * n, cudaMemcpyDeviceToHost, stream));
     std::vector<int> rows((size_t)n * cap);

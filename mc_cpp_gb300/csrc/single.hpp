@@ -70,6 +70,7 @@ public:
 
 private:
     int build_list();
+    int need_list() const;                 // MCG_OK, or the status of a system whose last list build failed
     void release();
     AtomsDev atoms() const;
     int launch_nonbonded(double* nbp);     // returns the CTAs launched (partial sums written)
@@ -135,6 +136,7 @@ private:
     uint4* d_cell_pos = nullptr;  // candidates in cell order: fixed-point position, atom index
     int any_frozen = 0;
     int ncell_cap = 0;
+    bool list_ok = false;
     double* d_part = nullptr;
     size_t part_cap = 0;
     unsigned* d_ticket = nullptr;

@@ -77,3 +77,24 @@ def test_rows_of_crowded_cells(n, kind):
     s.cutoff, s.cuton, s.sig = s.box[0] / 2.1, s.box[0] / 4, s.sig / 5
     s.pbc_type = kind
     _compare(s)
+
+
+# rows that would need more memory than any device has: the update fails, what needs rows is refused until an
+# update succeeds, and then everything is as before.  (Two million atoms drawn together to 45,000 partners each
+# would take 400 GB; their 1,400 to a cell stay within a cell's sort.)
+def test_rows_that_do_not_fit_the_device():
+    n = 2_000_000
+    s = systems.argon_random(n, n / 300.0 ** 3, 5)
+    ff = FFieldCUDA(s, "fp64", moves=False)
+    e = ff.getE10()
+    idx, new = np.array([3], np.int32), s.coords()[3:4] + 0.01
+    de = ff.delta_e(idx, new)
+    ff.setCoords(np.random.default_rng(6).uniform(0.0, 80.0, (n, 3)))
+    with pytest.raises(native.McgError, match="cudaMalloc"):
+        ff.askListUpdate(0)
+    for call in (ff.getE10, lambda: ff.delta_e(idx, new), lambda: ff.time_nonbonded(1)):
+        with pytest.raises(native.McgError, match="no Verlet list"):
+            call()
+    ff.setCoords(s.coords())
+    ff.askListUpdate(0)
+    assert np.array_equal(ff.getE10(), e) and ff.delta_e(idx, new) == de
