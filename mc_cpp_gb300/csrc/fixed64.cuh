@@ -20,9 +20,12 @@
 //   2^-49).  Rounding s^6 and s^12 to doubles instead would be an error common to all pairs of two classes.
 // * The switch is v^2 (3 - 2 v) with v = (rc^2 - u) / (rc^2 - ron^2) clamped to [0, 1] (the
 //   reference's polynomial in another variable), to 2^-56 of itself (beside u's own last place).
-// Totals against 113-bit sums, RMS over eight boxes each (FP64 pair terms in brackets): 2,400 water atoms
-// switched, Coulomb 5.3e-16 (9.3e-16), Lennard-Jones 1.1e-16 (2.4e-16); 1,200 in full mode 1.4e-16
-// (3.2e-16) and 1.0e-16 (3.0e-16); 2,000 argon atoms 0.6e-16 (1.0e-16).
+// Totals against 113-bit sums, relative (FP64 pair terms in brackets).  Switched, 12 and 10 A, over 24 boxes of 28.6 to
+// 60 A on both sides of the switch's normalisation, RMS: 2,400 water atoms in cubic boxes Coulomb 4.5e-16 (3.0e-15),
+// Lennard-Jones 2.2e-16 (3.8e-16), orthorhombic 1.1e-15 (3.1e-15) and 0.9e-16 (1.2e-16); 500 to 1,500 argon atoms
+// 1.2e-16 (3.4e-16) and 1.1e-16 (7.4e-16).  Full mode, 60 boxes of 24 to 60 A: water Coulomb (median: some totals nearly
+// cancel) 3.5e-16 (5.3e-16) and 8.3e-16 (1.6e-15), Lennard-Jones RMS 0.9e-16 (1.0e-16) and 0.9e-16 (2.8e-16); argon
+// 1.0e-16 (3.0e-16) and 1.0e-16 (1.9e-16).
 // A pair closer than some 2^-11 of a box length (0.05 A in a box of 100 A; the geometry's emax), where the
 // positions' unit would tell, is left to the caller.
 #pragma once

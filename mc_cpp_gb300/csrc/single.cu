@@ -6,7 +6,7 @@
 //   es14[n]      double2 (eps14, sig14)
 //   fx[n]        uint4 (fx, fy, fz, parameter class)  fixed-point mirror for the mixed kernels
 //   cls_of[n], cls[ncls]  parameter class of each atom and the classes' (q hi, q lo, eps, sig)
-//   x64[n]       ulonglong4 (x, y, z as box fractions in 2^-64, class), FP64 switched periodic systems
+//   x64[n]       ulonglong4 (x, y, z as box fractions in 2^-64, class), FP64 periodic systems
 //   pair64[ncls^2]   the class pairs' parameter products (fixed64.hpp)
 //   esf[n]       float2 (eps, sig)
 //   nbr[n*cap]   int   Verlet rows: partners j > i from the front, j < i from the back
@@ -53,8 +53,9 @@ namespace mcg {
 
 constexpr int NB_BLOCKS = 152 * 4;   // grid of the list-driven kernels: 4 CTAs per SM
 constexpr int NB_THREADS = 256;
-constexpr int BD_BLOCKS = 152 * 4;   // largest grid of the bonded terms: a term per thread up to 155,648 (two CTAs per
-                                     // SM: 116 against 111 us for the mixed energy of 100,002 water atoms; one: 121)
+// largest grid of the bonded terms: a term per thread up to 155,648.  One, two and four CTAs per SM, us of a mixed energy:
+// 100,002 water atoms 122, 115, 111; 36,000 64, 64, 63; 1,800 to 18,000 the same, and so FP64 (568, 568, 569 at 100,002)
+constexpr int BD_BLOCKS = 152 * 4;
 constexpr int MAX_MOVED = 1024;
 constexpr int SORT_MAX = 2048;       // cells larger than this are sorted by one thread
 constexpr int CLS_MAX = 1024;        // parameter classes the mixed pair kernel keeps in shared memory
@@ -273,7 +274,10 @@ __device__ __forceinline__ bool stored_excluded(int lo, int hi, const int* __res
 // the former from 754 to 653 us.  Without a box, where every candidate took the FP64 test: 36,000 water atoms
 // 1756 us, 299 with the FP32 coordinates.)
 constexpr int ROW_WARPS = 4;
-constexpr int ROW_CTAS = 7;    // CTAs of four warps resident per SM at the kernel's 72 registers
+// CTAs of four warps launched per SM: what is resident with two home atoms (72 registers).  With four (96 registers) five
+// are, and two start as others end: whole updates 136 us against 158 with five at 12,288 atoms, 274 against 280 at
+// 36,000, 649 against 645 at 100,002.
+constexpr int ROW_CTAS = 7;
 constexpr int ROW_RING = 128;  // up to 63 pending candidates and 64 new ones
 
 // The pairs the FP32 test does not decide: in the band around the list radius, or close in index (the atom
@@ -650,10 +654,11 @@ __device__ __forceinline__ void pair64_params(const AtomsDev& A, double ileff, i
 // switch factor of exactly 0, and one placed outside ron that lies inside a factor of 1 to 2^-56.
 // The rings are drained at one place in the code, after a chunk of E64_U entries per lane: with the
 // evaluation inlined behind every entry the kernel stalled on instruction fetch (0.69 against 0.61 ms on
-// the 100,002-atom water box).  That box takes 0.53 ms, 69 G pairs/s (4.2 ms with the pair terms in
-// FP64); ncu at 12,288 atoms: FP64 pipe 45%, ALU 45%, the rest latency of the gathers.  Three entries
-// per lane in flight against two: 0.527 and 0.532 ms; five or six CTAs per SM instead of four: 0.520 and
-// 0.513 ms there, but 0.073 against 0.070 ms at 12,288 atoms.
+// the 100,002-atom water box).  That box takes 0.56 ms, 64 G pairs/s (4.2 ms with the pair terms in
+// FP64, 0.53 with the sigmas' powers as doubles); ncu there: issue 60%, ALU 49%, FP64 pipe 42%, the rest
+// latency of the gathers.  Three entries per lane in flight against two: 0.527 and 0.532 ms.  A grid of six
+// CTAs per SM instead of four, whole energies: 59 against 62 us at 6,000 atoms, 132 against 117 at 18,000,
+// 226 against 217 at 36,000, 626 against 568 at 100,002.
 constexpr int E64_U = 3;
 constexpr int E64_RING = 128;   // up to 31 pending pairs and 32 E64_U new ones
 
@@ -1083,8 +1088,9 @@ __global__ void __launch_bounds__(ALL_I, ALLMIX_CTAS) k_energy_all_mix(AtomsDev 
 // FP64 full energy for periodic boxes, on 64-bit integer pair terms (fixed64.cuh): three FP64
 // operations a pair, about 230 cycles of a scheduler's FP64 pipe per warp, beside some 150 integer
 // and FP32 ones.
-// 12,288 atoms (75 M pairs): the whole energy call takes 0.62 ms, 3.78 ms with the pair terms in FP64.
-constexpr int A64_CTAS = 10;   // per SM; 8: 641 against 622 us for a call at 12,288 atoms
+// 12,288 atoms (75 M pairs): the whole energy call takes 0.62 ms, 3.78 ms with the pair terms in FP64 (0.57 with the
+// sigmas' powers as doubles, whose rounding all pairs of two classes share).  ncu: FP64 pipe 62%, ALU 50%, issue 59%.
+constexpr int A64_CTAS = 10;   // per SM; 8, whole calls: 632 against 620 us at 12,288 atoms, 91.7 against 89.3 at 4,096, alike below
 
 template <bool ISO, bool TABLE>
 __global__ void __launch_bounds__(ALL_I, A64_CTAS) k_energy_all64(AtomsDev A, Fix64Geom G, PbcDev pbc, CutDev cut, int n,
@@ -2246,9 +2252,10 @@ int SingleEngine::build_list() {
     for (int k = 0; k < 3; k++) g.csf[k] = (float)(ext[k] / g.nc[k] * (1.0 - 1e-6));
     int ncell = g.nc[0] * g.nc[1] * g.nc[2];
     const bool iso = g.periodic && hs.L[0] == hs.L[1] && hs.L[1] == hs.L[2];
-    // home atoms that share a walk: four share more of it, two leave fewer warps idle in a small system.  A
-    // whole update with two, four and eight, each some 14 us more than now: 50, 58, 59 us (864 argon atoms), 72, 84, 97 (1,800 water
-    // atoms), 170, 159, 174 (12,288), 359, 305, 338 (36,000), 948, 761, 753 (100,002), so the line is at 8,192
+    // home atoms that share a walk: four share more of it, two leave fewer warps idle in a small system.  A whole
+    // update with two and four, us: 33, 37 (864 argon atoms), 42, 39 (4,000 argon), 51, 57 (1,800 water atoms), 83, 86
+    // (4,500), 100, 106 (6,000), 104, 113 (8,193), 158, 120 (9,600), 167, 136 (12,288), 185, 182 (18,000), 751, 649
+    // (100,002); eight were slower up to 36,000.  The line is at 8,192
     const int run = n < 8192 ? 2 : 4;
     int rc;
     if (ncell > ncell_cap) {
