@@ -119,7 +119,8 @@ int mcg_energy(mcg_system* s, double ener[10]);
 int mcg_energy_host(mcg_system* s, const double* x, const double* y, const double* z, double* etot);
 
 /* FField::askListUpdate (src/FField.cpp:222-235): rebuild the Verlet list from the current
- * coordinates with a device cell list.  No-op in full mode. */
+ * coordinates with a device cell list.  No-op in full mode.  When the rows do not fit the device
+ * the status is MCG_ECUDA, and what needs the list is refused with it until an update succeeds. */
 int mcg_update_lists(mcg_system* s);
 
 /* Energy change of moving atoms[0..n) to (nx,ny,nz), nonbonded (current list, same cutoff, switch,
